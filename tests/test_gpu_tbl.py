@@ -100,6 +100,44 @@ def test_quirks_match_oracle(cuda):
     check_same(got, want)
 
 
+@pytest.mark.parametrize("tile_lines", [40, 4000])
+def test_field_forms_match_oracle(cuda, tile_lines):
+    """Every mix of usual and unusual field forms (digits, decimals, signs, blanks, odd dates, bytes next
+    to '|' and above 127, long leading fields, a missing last '|'), at every alignment and around the
+    parse kernel's 63 KB tiles: values, malformed lines and the first one's offset as the oracle's.
+    tile_lines: lines to a tile, few (long trailing fields) or, with runs of empty lines, thousands."""
+    rng = np.random.default_rng(48 + tile_lines)
+    def pick(usual, unusual, n):
+        return [str(rng.choice(usual if rng.random() < 0.9 else unusual)) for _ in range(n)]
+    n = 12_000
+    qty = pick(["1", "50", "7.00", "49.00", "0", "9999.99"], ["12345", "123456.78", "1.5", "+3", "-4.00", "", ".50", "1.", "x", "12a", "0.123"], n)
+    price = pick(["901.00", "104949.50", "99999999.99", "1.00"], ["123", "1.5", "123456789.01", "-5.00", "+7.25", "", "1a.00", "1.0a", "..00"], n)
+    cents = ["0.00", "0.10", "0.09", "9.99"]
+    odd = ["0.1", "10.00", "0", "-0.04", "0,04", "0.0a", "", "0.004"]
+    disc, tax = pick(cents, odd, n), pick(cents, odd, n)
+    rf, ls = pick(["A", "N", "R"], ["", "RR", "~", "{", "}"], n), pick(["F", "O"], ["", "OO", " "], n)
+    date = pick(["1992-01-02", "1998-12-31", "1996-02-29", "2000-02-29", "0001-01-01", "9999-12-31"],
+                ["1900-02-29", "1995-13-01", "1995-00-10", "1995-04-31", "1995-04-00", "0000-01-01", "1995-4-1",
+                 "12345-01-01", "1995/04/01", "1995-0a-01", ""], n)
+    lead = [["1", "155190", "7706", "1"], ["600000000", "20000000", "1000000", "7"], ["", "", "", ""],
+            ["1234567890123", "12345678901", "12345678", "9"], ["a\x80\xfc", "{z}", "\xff", "}"]]
+    lines = []
+    for i in range(n):
+        head = lead[0] if rng.random() < 0.8 else lead[rng.integers(1, len(lead))]
+        end = ["|1996-02-12|TRUCK|text|", "|", "", "|tail"][rng.choice(4, p=[0.9, 0.04, 0.03, 0.03])]
+        line = "|".join(head + [qty[i], price[i], disc[i], tax[i], rf[i], ls[i], date[i]]) + end
+        lines.append(line.encode("latin1") + (b"y" * int(rng.integers(0, 1600)) if tile_lines == 40 else b""))
+        if tile_lines > 1000 and rng.random() < 0.1:
+            lines.extend([b""] * int(rng.integers(1, 3000)))          # empty lines: thousands to a tile
+    text = b"\n".join(lines) + b"\n"
+    want, wrows, wbad, wfirst = O.parse_tbl(text)
+    for offset in [0, 5]:
+        got, rows, st, msg = gpu_parse(text, offset=offset)
+        assert rows == wrows
+        assert st == 1 and f"{wbad} malformed line(s); the first starts at byte {wfirst}" in msg
+        check_same(got, want)
+
+
 def test_malformed_lines_are_reported(cuda):
     lines = q.tbl_format(q.generate_host(44, 0, 5000)).split(b"\n")[:-1]
     lines[10] = b"1|2|3|4|x|1.00|0.01|0.02|R|F|1994-01-01|"

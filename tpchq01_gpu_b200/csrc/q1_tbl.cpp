@@ -93,6 +93,12 @@ struct PinnedMem {
     }
 };
 
+q1_status current_device(DeviceInfo** di) {
+    int dev = 0;
+    Q1_CUDA(cudaGetDevice(&dev));
+    return device_info(dev, di);
+}
+
 // Civil date of a MonetDB day number (inverse of the parser's day_number), years >= 1.
 void civil_from_day(int32_t n, int* y, int* m, int* d) {
     auto first = [](int yy) {
@@ -185,15 +191,16 @@ q1_status q1_tbl_count_device(const char* dev_text, uint64_t bytes, uint64_t* ro
     *rows = 0;
     if (!bytes) return Q1_OK;
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    const uint64_t tiles = tbl_tiles(bytes);
-    DeviceMem lines;
-    q1_status s = lines.alloc_async((tiles + 1) * 8, st);
+    DeviceInfo* di = nullptr;
+    q1_status s = current_device(&di);
     if (s != Q1_OK) return s;
+    DeviceMem lines;
+    if ((s = lines.alloc_async(8, st)) != Q1_OK) return s;
     auto* v = static_cast<unsigned long long*>(lines.p);
-    Q1_CUDA(launch_tbl_count(dev_text, bytes, v, st));
+    Q1_CUDA(launch_tbl_count(dev_text, bytes, v, di->sm_count, st));
     unsigned long long total = 0;
     char last = 0;
-    Q1_CUDA(cudaMemcpyAsync(&total, v + tiles, 8, cudaMemcpyDeviceToHost, st));
+    Q1_CUDA(cudaMemcpyAsync(&total, v, 8, cudaMemcpyDeviceToHost, st));
     Q1_CUDA(cudaMemcpyAsync(&last, dev_text + bytes - 1, 1, cudaMemcpyDeviceToHost, st));
     Q1_CUDA(cudaStreamSynchronize(st));
     *rows = total + (last != '\n' ? 1u : 0u);
@@ -213,31 +220,27 @@ q1_status q1_tbl_parse_device(const char* dev_text, uint64_t bytes, const q1_col
         misaligned(dev_out->discount, 8) || misaligned(dev_out->tax, 8))
         return set_error(Q1_ERR_INVALID_ARGUMENT, "output columns must be aligned to their element size");
     cudaStream_t st = (cudaStream_t)cuda_stream;
-    const uint64_t tiles = tbl_tiles(bytes);
-    DeviceMem scratch;
-    q1_status s = scratch.alloc_async((tiles + 3) * 8, st);
+    DeviceInfo* di = nullptr;
+    q1_status s = current_device(&di);
     if (s != Q1_OK) return s;
-    auto* v = static_cast<unsigned long long*>(scratch.p);
-    unsigned long long* bad = v + tiles + 1;
-    Q1_CUDA(cudaMemsetAsync(bad, 0, 8, st));
-    Q1_CUDA(cudaMemsetAsync(bad + 1, 0xFF, 8, st));
-    Q1_CUDA(launch_tbl_count(dev_text, bytes, v, st));
-    Q1_CUDA(launch_tbl_parse(dev_text, bytes, v, dev_out->shipdate, dev_out->quantity, dev_out->extendedprice,
-                             dev_out->discount, dev_out->tax, dev_out->returnflag, dev_out->linestatus, capacity, bad,
-                             st));
-    unsigned long long host[3] = {0, 0, 0};
-    char last = 0;
-    Q1_CUDA(cudaMemcpyAsync(host, v + tiles, 24, cudaMemcpyDeviceToHost, st));
-    Q1_CUDA(cudaMemcpyAsync(&last, dev_text + bytes - 1, 1, cudaMemcpyDeviceToHost, st));
+    DeviceMem scratch;
+    if ((s = scratch.alloc_async(tbl_scratch_bytes(dev_text, bytes), st)) != Q1_OK) return s;
+    Q1_CUDA(launch_tbl_parse(dev_text, bytes, scratch.p, dev_out->shipdate, dev_out->quantity, dev_out->extendedprice,
+                             dev_out->discount, dev_out->tax, dev_out->returnflag, dev_out->linestatus, capacity,
+                             di->sm_count, st));
+    TblResult r{};
+    Q1_CUDA(cudaMemcpyAsync(&r, scratch.p, sizeof(r), cudaMemcpyDeviceToHost, st));
     Q1_CUDA(cudaStreamSynchronize(st));
-    const uint64_t rows = host[0] + (last != '\n' ? 1u : 0u);
+    if (r.status) return set_error(Q1_ERR_DEVICE_TIMEOUT, "a bounded wait of the text parser expired");
+    const uint64_t rows = r.newlines + (r.last_is_newline ? 0u : 1u);
     *rows_out = rows;
     if (rows > capacity)
         return set_error(Q1_ERR_INVALID_ARGUMENT, "the text holds " + std::to_string(rows) + " rows, the output " +
                                                       std::to_string(capacity));
-    if (host[1])
-        return set_error(Q1_ERR_INVALID_ARGUMENT, std::to_string(host[1]) + " malformed line(s); the first starts at byte " +
-                                                      std::to_string(host[2]));
+    if (r.malformed)
+        return set_error(Q1_ERR_INVALID_ARGUMENT, std::to_string(r.malformed) +
+                                                      " malformed line(s); the first starts at byte " +
+                                                      std::to_string(~r.first_malformed));
     return Q1_OK;
 }
 

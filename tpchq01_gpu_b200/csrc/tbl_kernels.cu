@@ -14,41 +14,69 @@
 // A line that does not match is counted as malformed (its row is written as zeros) and the host
 // reports the count and the first malformed line's byte offset.
 //
-// Kernels (64 KB text tiles, 256 threads, 256 bytes a thread):
-//   tbl_count_kernel  newlines per tile (16-byte loads, byte compares on 32-bit words)
-//   tbl_scan_kernel   exclusive prefix of the tile counts (one CTA)
-//   tbl_parse_kernel  recounts its tile, ranks each thread's newlines with a block scan,
-//                     gathers the line starts into shared memory in text order and parses them
-//                     lane-parallel (row = newlines before the line); thread 0 of tile 0 also
-//                     parses the line at byte 0.
+// Kernels:
+//   tbl_count_kernel  newlines of the whole text (16-byte loads, byte compares on 32-bit words)
+//   tbl_parse_kernel  one pass over the text. One persistent CTA per SM takes 63 KB tiles in ticket
+//                     order and streams them into shared memory with bulk copies (three stages).
+//                     Workers find the next tile's newlines with word compares and rank them by
+//                     ballots, then parse the current tile's lines, a line a lane, word by word from
+//                     shared memory (parse_fast; any other form goes to the byte-wise parse_line).
+//                     A control warp meanwhile sums the newlines before the tile from the counts the
+//                     other CTAs published (decoupled look-back, bounded).
+//
+// What bounds it: instructions, 28 warp instructions a line at half of the issue slots. 6.0 M rows of
+// dbgen text (757 MB, 1.0 GB with the columns, 0.15 ms at the copy bandwidth) take 0.31 ms a call;
+// counting, scanning the counts and parsing byte by byte in three kernels took 1.62 ms (142 warp
+// instructions a line, the text read twice). 10,000 rows: 91 -> 37 us. Measured on the way: tiles of
+// 30 KB with two CTAs an SM 0.36 to 0.59 ms (twice the tiles to order), a look-back step of 256 tiles
+// 0.1 ms more than one of 64, the newline search with 512 bytes a load across the warp 0.39 ms.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "q1_kernels.h"
+#include "q1_ptx.cuh"
 
 namespace q1 {
 
 namespace tbl {
 
-constexpr uint32_t kThreads = 256;
-constexpr uint32_t kPerThread = 256;                 // bytes
-constexpr uint64_t kTile = (uint64_t)kThreads * kPerThread;
+using namespace ptx;
 
-// Newlines in text[a, b) (a 16-byte aligned or b - a < 16 handled bytewise).
-__device__ __forceinline__ uint32_t count_newlines(const char* __restrict__ text, uint64_t a, uint64_t b) {
-    uint32_t n = 0;
-    if (b - a == kPerThread && ((reinterpret_cast<uintptr_t>(text) + a) & 15u) == 0) {
-        const uint4* p = reinterpret_cast<const uint4*>(text + a);
-#pragma unroll 4
-        for (uint32_t k = 0; k < kPerThread / 16; ++k) {
-            const uint4 v = __ldg(p + k);
-            n += __popc(__vcmpeq4(v.x, 0x0A0A0A0Au)) + __popc(__vcmpeq4(v.y, 0x0A0A0A0Au)) +
-                 __popc(__vcmpeq4(v.z, 0x0A0A0A0Au)) + __popc(__vcmpeq4(v.w, 0x0A0A0A0Au));
-        }
-        return n / 8;   // __vcmpeq4 sets all 8 bits of an equal byte
-    }
-    for (uint64_t i = a; i < b; ++i) n += text[i] == '\n' ? 1u : 0u;
-    return n;
+// A CTA is 18 worker warps and one control warp, one CTA per SM (16 workers 0.336 ms, 17 0.324 ms,
+// 18 0.311 ms: as many as three stages leave room for). Text positions are counted from the 16-byte
+// boundary at or before the first byte, so that every tile starts on a boundary. A worker's part of a
+// tile is 3.5 KB: long enough to spread what each tile costs beside the search (barriers, sums),
+// and at 120 to 130 bytes a line just under 32 lines, so that a tile's lines make about one batch of
+// 32 for every worker.
+constexpr uint32_t kWorkers = 18;
+constexpr uint32_t kThreads = (kWorkers + 1) * 32;
+constexpr uint32_t kSubs = 7;                        // 16-byte pieces a lane
+constexpr uint32_t kLaneBytes = kSubs * 16;
+constexpr uint32_t kWords = (kSubs + 1) / 2;         // words of a lane's newline bits
+constexpr uint32_t kWarpBytes = 32 * kLaneBytes;
+constexpr uint32_t kTile = kWorkers * kWarpBytes;
+constexpr uint32_t kAhead = 128;                     // bytes after the tile kept with it: a line's window
+constexpr uint32_t kFront = 16;                      // room before the tile for right-aligned field loads
+constexpr uint32_t kStageBytes = kFront + kTile + kAhead;
+constexpr uint32_t kRing = 3;                        // tiles in flight or in use a CTA
+constexpr uint32_t kWarpList = 96;                   // line starts listed a part (about 28 in dbgen text)
+static_assert(kStageBytes % 16 == 0, "stages stay 16-byte aligned");
+static_assert(kSubs % 2 == 1, "conflict-free loads of a lane's consecutive bytes");
+static_assert(kWarpList >= 64, "two newlines a lane");
+static_assert(kRing == 3, "a tile reloads the stage of the tile before it");
+static_assert(kTile <= 65535, "a tile's newlines fit 16 bits");
+
+// Bit 7 of byte i set iff byte i of w equals the byte repeated in c4 (below 128; exact for every w).
+__device__ __forceinline__ uint32_t equal_bytes(uint32_t w, uint32_t c4) {
+    return ~((((w ^ c4) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w) & 0x80808080u;
+}
+// 16 bits, bit i set iff byte i of v equals the byte. The multiply gathers a word's four flags
+// into its top four bits (no two partial products meet), a funnel shift appends them.
+__device__ __forceinline__ uint32_t match16(const uint4& v, uint32_t c4) {
+    uint32_t m = __funnelshift_l(equal_bytes(v.w, c4) * 0x00204081u, 0u, 4);
+    m = __funnelshift_l(equal_bytes(v.z, c4) * 0x00204081u, m, 4);
+    m = __funnelshift_l(equal_bytes(v.y, c4) * 0x00204081u, m, 4);
+    return __funnelshift_l(equal_bytes(v.x, c4) * 0x00204081u, m, 4);
 }
 
 // Day number of a civil date counted the MonetDB way (days since a year 0, years >= 1 here);
@@ -172,178 +200,510 @@ struct Out {
     char *rf, *ls;
 };
 
-// Parses the line starting at byte s into row `row`; false (row zeroed) if malformed.
-__device__ bool parse_line(const char* __restrict__ text, uint64_t bytes, uint64_t s, uint64_t row, const Out& o) {
+struct Row {
+    int64_t qty, price, disc, tax;
+    int32_t ship;
+    char rf, ls;
+};
+
+// Parses the line starting at byte s of the text, any form; false (row zeroed) if malformed.
+__device__ __noinline__ bool parse_line(const char* __restrict__ text, uint64_t bytes, uint64_t s, Row& r) {
     Cursor c(text, s, bytes);
-    int64_t q = 0, pr = 0, di = 0, tx = 0;
-    char rf = 0, ls = 0;
-    int32_t ship = 0;
+    r = Row{0, 0, 0, 0, 0, 0, 0};
     bool ok = c.skip_field() && c.skip_field() && c.skip_field() && c.skip_field();
-    ok = ok && c.decimal(q) && c.sep() && c.decimal(pr) && c.sep() && c.decimal(di) && c.sep() && c.decimal(tx) &&
-         c.sep();
-    ok = ok && c.chr(rf) && c.sep() && c.chr(ls) && c.sep() && c.date(ship);
-    if (!ok) q = pr = di = tx = 0, rf = ls = 0, ship = 0;
-    o.ship[row] = ship;
-    o.qty[row] = q;
-    o.price[row] = pr;
-    o.disc[row] = di;
-    o.tax[row] = tx;
-    o.rf[row] = rf;
-    o.ls[row] = ls;
+    ok = ok && c.decimal(r.qty) && c.sep() && c.decimal(r.price) && c.sep() && c.decimal(r.disc) && c.sep() &&
+         c.decimal(r.tax) && c.sep();
+    ok = ok && c.chr(r.rf) && c.sep() && c.chr(r.ls) && c.sep() && c.date(r.ship);
+    if (!ok) r = Row{0, 0, 0, 0, 0, 0, 0};
     return ok;
+}
+
+// A line of the usual form: every value but the price fits 32 bits.
+struct FastRow {
+    int64_t price;
+    uint32_t qty, disc, tax;
+    int32_t ship;
+    uint32_t flags;   // return flag, line status << 8
+};
+
+// n words of the byte stream from any offset (at least -16), realigned.
+template <int n>
+__device__ __forceinline__ void load_bytes(const uint8_t* buf, int32_t at, uint32_t out[n]) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(buf + (at & ~3));
+    const uint32_t sh = (uint32_t)(at & 3) * 8;
+    uint32_t lo = w[0];
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+        const uint32_t hi = w[i + 1];
+        out[i] = __funnelshift_r(lo, hi, sh);
+        lo = hi;
+    }
+}
+// The last n (0..4) bytes of a word of four characters; x: digits, 0 in the bytes before them.
+__device__ __forceinline__ uint32_t last_bytes(int32_t n) {
+    return __funnelshift_lc(0u, 0xFFFFFFFFu, n >= 4 ? 0 : 8 * (4 - n));
+}
+// Four digit values, the first character's in byte 0, as a number.
+__device__ __forceinline__ uint32_t four_digits(uint32_t x) {
+    return __dp4a((x * 10u + (x >> 8)) & 0x00FF00FFu, 0x00010064u, 0u);
+}
+// Any byte above 9: bit 7 of a byte of the result (other bits are noise).
+__device__ __forceinline__ uint32_t not_digits(uint32_t x) { return (x + 0x76767676u) | x; }
+
+// Days before each month of a non-leap year | its days << 16 (0: no such month).
+__device__ __forceinline__ uint32_t month_entry(uint32_t m) {
+    if (m < 1 || m > 12) return 0;
+    return (uint32_t)days_before_month((int32_t)m) |
+           (uint32_t)(m == 12 ? 31 : days_before_month((int32_t)m + 1) - days_before_month((int32_t)m)) << 16;
+}
+
+// Parses a line of the form dbgen writes, held in shared memory, a word at a time: four fields, a
+// quantity of up to four digits with two decimals or none, a price of up to eight digits with two
+// decimals (all of them within 49 characters), then the 25 characters "d.dd|d.dd|R|L|yyyy-mm-dd|".
+// p: the line's first byte in buf, next: the next line's; months: month_entry of 0..15. False: not
+// of this form (the caller parses the line with parse_line; every line accepted here gets the
+// values that parse_line gives).
+__device__ __forceinline__ bool parse_fast(const uint8_t* buf, uint32_t p, uint32_t next, const uint32_t* months,
+                                           FastRow& r) {
+    // the '|' of the 49 or more bytes from p, as bits
+    const uint4* w = reinterpret_cast<const uint4*>(buf + (p & ~15u));
+    const uint32_t bar = 0x7C7C7C7Cu;
+    const uint32_t m0 = match16(w[0], bar) | match16(w[1], bar) << 16;
+    const uint32_t m1 = match16(w[2], bar) | match16(w[3], bar) << 16;
+    const uint32_t s = p & 15u;
+    const uint32_t l0 = __funnelshift_r(m0, m1, s), l1 = m1 >> s;
+    uint32_t a = l0 & (l0 - 1u);
+    a &= a - 1u;
+    a &= a - 1u;
+    const uint32_t e4 = (uint32_t)__ffs((int)a) - 1u;             // fourth '|' (there is one if a != 0)
+    const uint32_t n0 = __funnelshift_rc(l0, l1, e4 + 1u);
+    const uint32_t b = n0 & (n0 - 1u);
+    const uint32_t e5 = (uint32_t)__ffs((int)n0) - 1u, e6 = (uint32_t)__ffs((int)b) - 1u;   // from field 5 on
+    const uint32_t c = p + e4 + e6 + 2u;                          // field 7
+    if (!a || !b || c + 25u >= next) return false;
+    // "d.dd|d.dd|R|L|yyyy-mm-dd|"; wrong: not a digit, off: not the character expected
+    uint32_t A[7];
+    load_bytes<7>(buf, (int32_t)c, A);
+    const uint32_t xd = A[0] ^ 0x30302E30u, xt = __byte_perm(A[1], A[2], 0x4321u) ^ 0x30302E30u;
+    uint32_t wrong = not_digits(xd) | not_digits(xt);
+    uint32_t off = (xd | xt) & 0x0000FF00u;
+    r.disc = __dp4a(xd, 0x010A0064u, 0u);
+    r.tax = __dp4a(xt, 0x010A0064u, 0u);
+    off |= ((A[1] ^ 0x7Cu) & 0xFFu) | ((A[2] ^ 0x7C007C00u) & 0xFF00FF00u) | ((A[3] ^ 0x7C00u) & 0xFF00u) |
+           ((A[6] ^ 0x7Cu) & 0xFFu);
+    r.flags = __byte_perm(A[2], A[3], 0x0042u);
+    const bool blank = (r.flags & 0xFFu) == '|' || (r.flags & 0xFF00u) == ('|' << 8);   // an empty flag field
+    const uint32_t xy = __byte_perm(A[3], A[4], 0x5432u) ^ 0x30303030u;
+    const uint32_t xm = __byte_perm(A[4], A[5], 0x5432u) ^ 0x2D30302Du, xx = (A[5] >> 16) ^ 0x3030u;
+    wrong |= not_digits(xy) | not_digits(xm) | not_digits(xx);
+    off |= xm & 0xFF0000FFu;
+    // the day number of yyyy = 100 yh + yl (day_number's steps, the centuries from the digits)
+    const uint32_t yp = xy * 10u + (xy >> 8), yh = yp & 0xFFu, yl = (yp >> 16) & 0xFFu, year = 100u * yh + yl;
+    const uint32_t month = __dp4a(xm, 0x00010A00u, 0u), day = __dp4a(xx, 0x0000010Au, 0u);
+    const uint32_t me = months[month & 15u];
+    const uint32_t leap = ((yl ? yl : yh) & 3u) == 0u ? 1u : 0u, cent = yh - (yl ? 0u : 1u);
+    const uint32_t in_month = (me >> 16) + (month == 2u ? leap : 0u);
+    const bool no_day = day - 1u >= in_month || year == 0u || month > 15u;
+    r.ship = (int32_t)(365u * year + ((year - 1u) >> 2) - cent + (cent >> 2) + (me & 0xFFFFu) +
+                       (month > 2u ? leap : 0u) + day);
+    // price: ".dd|" ends at the '|' before field 7, up to eight digits before it
+    uint32_t D[3];
+    load_bytes<3>(buf, (int32_t)c - 12, D);
+    const int32_t pd = (int32_t)(e6 - e5) - 4;                    // digits before the point
+    const uint32_t x0 = (D[0] ^ 0x30303030u) & last_bytes(pd - 4 < 0 ? 0 : pd - 4);
+    const uint32_t x1 = (D[1] ^ 0x30303030u) & last_bytes(pd < 0 ? 0 : pd);
+    const uint32_t xc = D[2] ^ 0x7C30302Eu;
+    wrong |= not_digits(x0) | not_digits(x1) | not_digits(xc);
+    off |= xc & 0xFF0000FFu;
+    r.price = (int64_t)(four_digits(x0) * 10000u + four_digits(x1)) * 100 + __dp4a(xc, 0x00010A00u, 0u);
+    // quantity: with ".dd" or whole
+    uint32_t Q[2];
+    load_bytes<2>(buf, (int32_t)(p + e4 + e5) - 6, Q);             // the eight bytes up to its '|'
+    const bool point = (Q[1] & 0xFFu) == '.' && e5 >= 4u;
+    const int32_t qd = (int32_t)e5 - (point ? 3 : 0);
+    const uint32_t xq = ((point ? Q[0] : __byte_perm(Q[0], Q[1], 0x6543u)) ^ 0x30303030u) & last_bytes(qd);
+    const uint32_t xf = point ? (Q[1] ^ 0x7C30302Eu) : 0u;
+    wrong |= not_digits(xq) | not_digits(xf);
+    r.qty = four_digits(xq) * 100u + __dp4a(xf, 0x00010A00u, 0u);
+    return ((wrong & 0x80808080u) | off) == 0u && (uint32_t)(pd - 1) < 8u && (uint32_t)(qd - 1) < 4u && !no_day && !blank;
+}
+
+// Published state of a tile: flag in the top two bits, value below.
+constexpr uint64_t kFlagCount = 1ull << 62;    // value: newlines of the tile
+constexpr uint64_t kFlagPrefix = 2ull << 62;   // value: newlines of the tiles up to this one
+constexpr uint64_t kValueMask = (1ull << 62) - 1;
+constexpr uint32_t kStatePad = 64;             // zeroed states before tile 0's (a look-back step's reach)
+
+__device__ __forceinline__ void store_state(unsigned long long* p, uint64_t v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// Newlines before tile k: sums the published counts of the tiles before it, two a lane and 64 a
+// step, down to the nearest published prefix. A step is kept short: the control warp gets one
+// warp's share of the issue slots (eight tiles a lane, 256 a step, took 0.1 ms longer in all).
+// Every tile before k was taken by a running CTA (tickets), so the wait ends; it is bounded all the
+// same. All lanes of one warp call it. state: 16-byte aligned, kStatePad zeroed states before it.
+__device__ __forceinline__ bool look_back(const unsigned long long* state, uint64_t k, uint32_t lane, uint64_t& prefix,
+                                          uint32_t* status) {
+    prefix = 0;
+    const unsigned long long* at = state + 2 * ((int64_t)((k - 1) / 2) - (int64_t)lane);
+    bool skip = lane == 0 && (k & 1u);   // lane 0's second tile is k itself
+    uint64_t t0 = 0;
+    for (uint32_t spin = 0;;) {
+        uint64_t a, b;
+        asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(at) : "memory");
+        if (skip) b = kFlagCount;
+        const uint32_t fa = (uint32_t)(a >> 62), fb = (uint32_t)(b >> 62);
+        const uint32_t pre = __ballot_sync(0xffffffffu, fb == 2 || (fb == 1 && fa == 2));
+        const uint32_t known = __ballot_sync(0xffffffffu, fb == 2 || (fb == 1 && fa != 0));
+        const uint32_t last = pre ? (uint32_t)__ffs((int)pre) - 1u : 31u;
+        if ((~known & (0xFFFFFFFFu >> (31u - last))) == 0u) {
+            const uint64_t sum = (b & kValueMask) + (fb == 2 ? 0ull : a & kValueMask);
+            prefix += __reduce_add_sync(0xffffffffu, (lane < last || !pre) ? (uint32_t)sum : 0u);
+            if (pre) {
+                prefix += __shfl_sync(0xffffffffu, sum, (int)last);
+                return true;
+            }
+            at -= 64;
+            skip = false;
+            continue;
+        }
+        __nanosleep(64);
+        if ((++spin & 63u) == 0) {
+            const uint64_t now = globaltimer();
+            if (!t0) t0 = now;
+            if (__any_sync(0xffffffffu, now - t0 > kWaitLimitNs)) {
+                if (lane == 0) atomicOr(status, kStatusWaitTimeout);
+                return false;
+            }
+        }
+    }
 }
 
 }  // namespace tbl
 
-__global__ void __launch_bounds__(tbl::kThreads) tbl_count_kernel(const char* __restrict__ text, uint64_t bytes,
-                                                                  unsigned long long* __restrict__ tile_lines) {
+// Newlines of the text, added to *total.
+__global__ void __launch_bounds__(256) tbl_count_kernel(const char* __restrict__ text, uint64_t bytes,
+                                                        unsigned long long* __restrict__ total) {
     using namespace tbl;
     __shared__ uint32_t sum;
     if (threadIdx.x == 0) sum = 0;
     __syncthreads();
-    const uint64_t a = blockIdx.x * kTile + (uint64_t)threadIdx.x * kPerThread;
-    const uint64_t b = a + kPerThread < bytes ? a + kPerThread : bytes;
-    uint32_t n = a < bytes ? count_newlines(text, a, b) : 0u;
-    n += __shfl_xor_sync(0xffffffffu, n, 16);
-    n += __shfl_xor_sync(0xffffffffu, n, 8);
-    n += __shfl_xor_sync(0xffffffffu, n, 4);
-    n += __shfl_xor_sync(0xffffffffu, n, 2);
-    n += __shfl_xor_sync(0xffffffffu, n, 1);
-    if ((threadIdx.x & 31u) == 0) atomicAdd(&sum, n);
-    __syncthreads();
-    if (threadIdx.x == 0) tile_lines[blockIdx.x] = sum;
-}
-
-// In-place exclusive prefix over `tiles` counts; element `tiles` receives the total.
-__global__ void __launch_bounds__(1024) tbl_scan_kernel(unsigned long long* v, uint64_t tiles) {
-    __shared__ unsigned long long part[1024];
-    __shared__ unsigned long long carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (uint64_t base = 0; base < tiles; base += 1024) {
-        const uint64_t i = base + threadIdx.x;
-        const unsigned long long x = i < tiles ? v[i] : 0ull;
-        part[threadIdx.x] = x;
-        __syncthreads();
-        for (uint32_t off = 1; off < 1024; off <<= 1) {
-            const unsigned long long y = threadIdx.x >= off ? part[threadIdx.x - off] : 0ull;
-            __syncthreads();
-            part[threadIdx.x] += y;
-            __syncthreads();
+    const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(text) & 15u);
+    const uint4* blk = reinterpret_cast<const uint4*>(text - off);
+    const uint64_t end = off + bytes, pieces = (end + 15) / 16;
+    uint32_t n = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < pieces; i += (uint64_t)gridDim.x * blockDim.x) {
+        if (16 * i >= off && 16 * i + 16 <= end) {
+            const uint4 v = __ldg(blk + i);
+            n += __popc(equal_bytes(v.x, 0x0A0A0A0Au)) + __popc(equal_bytes(v.y, 0x0A0A0A0Au)) +
+                 __popc(equal_bytes(v.z, 0x0A0A0A0Au)) + __popc(equal_bytes(v.w, 0x0A0A0A0Au));
+        } else {
+            for (uint64_t x = 16 * i < off ? off : 16 * i; x < 16 * i + 16 && x < end; ++x)
+                n += text[x - off] == '\n' ? 1u : 0u;
         }
-        if (i < tiles) v[i] = carry + part[threadIdx.x] - x;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry += part[1023];
-        __syncthreads();
     }
-    if (threadIdx.x == 0) v[tiles] = carry;
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31u) == 0 && n) atomicAdd(&sum, n);
+    __syncthreads();
+    if (threadIdx.x == 0 && sum) atomicAdd(total, (unsigned long long)sum);
 }
 
-// Parses the lines that start in this block's tile. The line starts are first gathered into
-// shared memory in text order (each thread's newlines at its block-scan rank), then every thread
-// parses lines tid, tid + 256, ...: the lanes of a warp parse different lines side by side instead
-// of one lane at a time. Tiles with more than kList lines take several rounds.
-__global__ void __launch_bounds__(tbl::kThreads) tbl_parse_kernel(const char* __restrict__ text, uint64_t bytes,
-                                                                  const unsigned long long* __restrict__ tile_first,
-                                                                  tbl::Out o, uint64_t capacity,
-                                                                  unsigned long long* __restrict__ bad) {
+__global__ void __launch_bounds__(tbl::kThreads, 1) tbl_parse_kernel(const char* __restrict__ text, uint64_t bytes,
+                                                                     tbl::Out o, uint64_t capacity, uint64_t tiles,
+                                                                     uint64_t full_tiles,
+                                                                     unsigned long long* __restrict__ state,
+                                                                     TblResult* __restrict__ res) {
     using namespace tbl;
-    constexpr uint32_t kList = 4096;
-    __shared__ uint32_t warp_sum[kThreads / 32];
-    __shared__ uint32_t total;
-    __shared__ uint32_t starts[kList];   // newline offsets within the tile, in text order
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ __align__(8) uint64_t full_bar[kRing];
+    __shared__ __align__(8) uint64_t prefix_bar;
+    __shared__ unsigned long long tile_of[kRing];
+    __shared__ uint32_t starts[kWorkers * kWarpList + 2];       // line starts in the tile, in text order, then the next one
+    __shared__ uint32_t warp_starts[kWorkers][kWarpList];   // the line starts of each worker's part, in order
+    __shared__ uint32_t warp_lines[2][32];       // newlines of each worker's part, by tile parity
+    __shared__ uint64_t prefix_s[2];             // newlines before the tile, by tile parity
+    __shared__ uint32_t months[16];
+    __shared__ uint32_t counted_s;               // workers done counting << 16 | their newlines
+    __shared__ uint32_t failed_s;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint64_t tile = blockIdx.x * kTile;
-    const uint64_t a = tile + (uint64_t)tid * kPerThread;
-    const uint64_t b = a + kPerThread < bytes ? a + kPerThread : bytes;
-    const uint32_t n = a < bytes ? count_newlines(text, a, b) : 0u;
-    // block-wide exclusive prefix of n
-    uint32_t inc = n;
-#pragma unroll
-    for (uint32_t off = 1; off < 32; off <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += y;
-    }
-    if (lane == 31) warp_sum[warp] = inc;
-    __syncthreads();
-    uint32_t before = 0;
-    for (uint32_t w = 0; w < warp; ++w) before += warp_sum[w];
-    before += inc - n;
-    if (tid == kThreads - 1) total = before + n;
-    __syncthreads();
-    const uint32_t T = total;
-    const unsigned long long first = tile_first[blockIdx.x];   // newlines before this tile
-    unsigned long long nbad = 0, first_bad = ~0ull;
-    auto one = [&](uint64_t s, uint64_t row) {
-        if (row >= capacity || !parse_line(text, bytes, s, row, o)) {
-            ++nbad;
-            if (s < first_bad) first_bad = s;
+    const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(text) & 15u);
+    const uint8_t* base = reinterpret_cast<const uint8_t*>(text) - off;   // position 0
+    const uint64_t end = off + bytes;
+    uint32_t* const status = &res->status;
+
+    // bytes of tile k and what is kept after it
+    auto tile_bytes = [&](uint64_t k) -> uint32_t {
+        const uint64_t left = end - k * kTile;
+        return left < kTile + kAhead ? (uint32_t)left : kTile + kAhead;
+    };
+    auto start_load = [&](uint32_t s, uint64_t k) {   // one thread
+        tile_of[s] = k;
+        if (k >= tiles) return;
+        const uint32_t n = tile_bytes(k) & ~15u, bar = smem_addr(&full_bar[s]);
+        if (n) {
+            mbar_arrive_expect_tx(bar, n);
+            bulk_g2s(smem_addr(smem) + s * kStageBytes + kFront, base + k * kTile, n, bar, policy_evict_first());
+        } else {
+            mbar_arrive(bar);
         }
     };
-    if (blockIdx.x == 0 && tid == 0 && bytes > 0) one(0, 0);
-    const bool vec = b - a == kPerThread && ((reinterpret_cast<uintptr_t>(text) + a) & 15u) == 0;
-    for (uint32_t r0 = 0; r0 < T; r0 += kList) {
-        // gather: this thread's newlines whose block rank falls in [r0, r0 + kList)
-        if (n && before + n > r0 && before < r0 + kList) {
-            uint32_t k = before;
-            if (vec) {
-                const uint4* p = reinterpret_cast<const uint4*>(text + a);
-                for (uint32_t q = 0; q < kPerThread / 16; ++q) {
-                    const uint4 v = __ldg(p + q);
-                    const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+    if (tid < 16) months[tid] = month_entry(tid);
+    if (tid < 32) warp_lines[0][tid] = warp_lines[1][tid] = 0;
+    if (tid == 0) {
+        failed_s = counted_s = 0;
+        for (uint32_t s = 0; s < kRing; ++s) mbar_init(smem_addr(&full_bar[s]), 1);
+        mbar_init(smem_addr(&prefix_bar), 1);
+        fence_mbar_init();
+        for (uint32_t s = 1; s < kRing; ++s) tile_of[s] = ~0ull;
+        start_load(0, atomicAdd(&res->ticket, 1ull));
+    }
+    __syncthreads();
+
+    // Newlines of this worker's part of the tile in stage s.
+    auto scan = [&](uint32_t s, uint32_t ph, uint64_t k, uint32_t parity) {
+        uint8_t* const buf = smem + s * kStageBytes + kFront;
+        if (!mbar_wait(smem_addr(&full_bar[s]), ph, status)) failed_s = 1;
+        // a lane takes 112 consecutive bytes (an odd multiple of 16: its loads meet no bank conflict)
+        const uint32_t at0 = warp * kWarpBytes + lane * kLaneBytes;
+        if (k >= full_tiles) {
+            // the last tiles: the bytes after the bulk copy, then zeros
+            const uint32_t n_here = tile_bytes(k), from = n_here & ~15u;
+            if (warp == 0)
+                for (uint32_t i = kTile + lane; i < kTile + kAhead; i += 32)
+                    if (i >= from) buf[i] = i < n_here ? base[k * kTile + i] : 0;
+            for (uint32_t i = at0; i < at0 + kLaneBytes; ++i)
+                if (i >= from) buf[i] = i < n_here ? base[k * kTile + i] : 0;
+        }
+        uint32_t m[kWords];   // bit i: byte at0 + i is a newline
 #pragma unroll
-                    for (uint32_t h = 0; h < 4; ++h) {
-                        uint32_t m = __vcmpeq4(w4[h], 0x0A0A0A0Au) & 0x80808080u;
-                        while (m) {
-                            const uint32_t byte = (uint32_t)(__ffs(m) - 1) >> 3;
-                            m &= m - 1;
-                            if (k >= r0 && k < r0 + kList) starts[k - r0] = (uint32_t)(a - tile) + q * 16 + h * 4 + byte;
-                            ++k;
-                        }
-                    }
+        for (uint32_t j = 0; j < kWords; ++j) {
+            m[j] = match16(*reinterpret_cast<const uint4*>(buf + at0 + j * 32), 0x0A0A0A0Au);
+            if (2 * j + 1 < kSubs)
+                m[j] |= match16(*reinterpret_cast<const uint4*>(buf + at0 + j * 32 + 16), 0x0A0A0A0Au) << 16;
+        }
+        if (k == 0 && at0 < off) m[0] &= 0xFFFFFFFFu << off;   // the bytes before the text
+        uint32_t c = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kWords; ++j) c += __popc(m[j]);
+        const uint32_t one = __ballot_sync(0xffffffffu, c >= 1u), two = __ballot_sync(0xffffffffu, c >= 2u);
+        uint32_t run = __popc(one) + __popc(two);
+        if (!__any_sync(0xffffffffu, c > 2u)) {   // lines of 56 bytes or more: at most two newlines a lane
+            const uint32_t lt = (1u << lane) - 1u;
+            const uint32_t at = __popc(one & lt) + __popc(two & lt);
+            if (c) {
+                uint32_t w = m[kWords - 1], lo = (kWords - 1) * 32;
+#pragma unroll
+                for (int j = (int)kWords - 2; j >= 0; --j) lo = m[j] ? j * 32u : lo, w = m[j] ? m[j] : w;
+                warp_starts[warp][at] = at0 + lo + (uint32_t)__ffs((int)w);
+            }
+            if (c == 2u) {
+                uint32_t w = m[0], hi = 32;
+#pragma unroll
+                for (uint32_t j = 1; j < kWords; ++j) hi = m[j] ? j * 32u + 32u : hi, w = m[j] ? m[j] : w;
+                warp_starts[warp][at + 1u] = at0 + hi - (uint32_t)__clz((int)w);
+            }
+        } else {
+            uint32_t inc = c;
+#pragma unroll 1
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, inc, d);
+                if (lane >= d) inc += u;
+            }
+            run = __shfl_sync(0xffffffffu, inc, 31);
+            uint32_t at = inc - c;
+#pragma unroll
+            for (uint32_t j = 0; j < kWords; ++j)
+#pragma unroll 1
+                for (uint32_t x = m[j]; x; x &= x - 1u, ++at)
+                    if (at < kWarpList) warp_starts[warp][at] = at0 + j * 32 + (uint32_t)__ffs((int)x);
+        }
+        if (lane == 0) {
+            warp_lines[parity][warp] = run;
+            // the last worker publishes the tile's count, long before anyone needs it
+            const uint32_t c = atomicAdd(&counted_s, 1u << 16 | run) + (1u << 16 | run);
+            if (c >> 16 == kWorkers) {
+                counted_s = 0;
+                store_state(state + k, (k == 0 ? kFlagPrefix : kFlagCount) | (c & 0xFFFFu));
+            }
+        }
+    };
+    // The line at byte `at` of the text, of any form, into row i (newlines before it); counted when
+    // malformed or past the capacity.
+    auto put_any = [&](uint64_t i, uint64_t at) {
+        Row row;
+        const bool good = parse_line(text, bytes, at, row);
+        if (i < capacity) {
+            o.ship[i] = row.ship;
+            o.qty[i] = row.qty;
+            o.price[i] = row.price;
+            o.disc[i] = row.disc;
+            o.tax[i] = row.tax;
+            o.rf[i] = row.rf;
+            o.ls[i] = row.ls;
+        }
+        if (i >= capacity || !good) {
+            atomicAdd(&res->malformed, 1ull);
+            atomicMax(&res->first_malformed, ~(unsigned long long)at);
+        }
+    };
+
+    // Tile by tile: the workers list tile i's lines (between two barriers), then find the newlines of
+    // tile i + 1 and parse tile i while the control warp looks back.
+    const bool control = warp == kWorkers;
+    uint32_t s = 0, ph = 0, parity = 0;
+    // Tickets are taken one at a time, as the CTA gets to them, so that the tiles before a tile are
+    // counted earlier than it: three tickets at the start left every CTA waiting for the third tile
+    // of the CTA before it.
+    if (tile_of[0] < tiles) {
+        if (!control) {
+            scan(0, 0, tile_of[0], 0);
+        } else if (lane == 0) {
+            mbar_wait(smem_addr(&full_bar[0]), 0, status);
+            start_load(1, atomicAdd(&res->ticket, 1ull));
+        }
+    }
+    for (;;) {
+        const uint64_t k = tile_of[s];
+        if (k >= tiles) break;
+        unsigned long long ticket = 0;
+        if (control && lane == 0) ticket = atomicAdd(&res->ticket, 1ull);
+        __syncthreads();   // newlines of tile i counted; tile i - 1 done
+        if (failed_s) break;
+        uint8_t* const buf = smem + s * kStageBytes + kFront;
+        const uint32_t wl = warp_lines[parity][lane];
+        const uint32_t newlines = __reduce_add_sync(0xffffffffu, wl);
+        // the text's first line has no newline before it: it comes first in tile 0
+        const uint32_t extra = k == 0 ? 1u : 0u, lines = newlines + extra;
+        const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? wl : 0u) + extra;
+        const bool listed = !__any_sync(0xffffffffu, wl > kWarpList);   // (the same in every warp)
+        if (control) {
+            if (lane == 0) {
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                start_load(s == 0 ? kRing - 1 : s - 1, ticket);   // tile i - 1's stage
+                if (extra) starts[0] = off;
+            }
+            if (listed) {
+                // the end of the tile's last line: the first newline after the tile, if it is near
+                const uint32_t x = lane < kAhead / 16
+                                       ? match16(*reinterpret_cast<const uint4*>(buf + kTile + lane * 16), 0x0A0A0A0Au)
+                                       : 0u;
+                const uint32_t any = __ballot_sync(0xffffffffu, x != 0u);
+                const uint32_t from = any ? (uint32_t)__ffs((int)any) - 1u : 0u;
+                const uint32_t xf = __shfl_sync(0xffffffffu, x, (int)from);
+                if (lane == 0)
+                    starts[lines] = any ? kTile + from * 16 + (uint32_t)__ffs((int)xf) : kTile + kAhead + 1u;
+            }
+        } else if (listed) {
+            const uint32_t n = warp_lines[parity][warp];
+            for (uint32_t j = lane; j < n; j += 32) starts[before + j] = warp_starts[warp][j];
+        }
+        __syncthreads();   // tile i's lines listed
+        uint32_t ns = s + 1, nph = ph;
+        if (ns == kRing) ns = 0, nph ^= 1u;
+        if (control) {
+            uint64_t pre = 0;
+            const bool ok = k == 0 || look_back(state, k, lane, pre, status);
+            if (lane == 0) {
+                if (ok && k) store_state(state + k, kFlagPrefix | (pre + newlines));
+                if (!ok) failed_s = 1;
+                prefix_s[parity] = pre;
+                if (k + 1 == tiles) {
+                    res->newlines = pre + newlines;
+                    res->last_is_newline = buf[tile_bytes(k) - 1] == '\n' ? 1u : 0u;
                 }
-            } else {
-                for (uint64_t i = a; i < b; ++i) {
-                    if (text[i] != '\n') continue;
-                    if (k >= r0 && k < r0 + kList) starts[k - r0] = (uint32_t)(i - tile);
-                    ++k;
+                mbar_arrive(smem_addr(&prefix_bar));
+            }
+        } else {
+            bool known = false;
+            auto prefix = [&]() -> uint64_t {   // the look-back's result
+                if (!known && !mbar_wait(smem_addr(&prefix_bar), parity, status)) failed_s = 1;
+                known = true;
+                return prefix_s[parity] + 1u - extra;
+            };
+            if (!listed) {
+                // very short lines: the worker walks its part, a byte a lane, without a list
+                const uint64_t first = prefix();
+                if (extra && tid == 0) put_any(0, 0);
+                uint64_t i = first + before;
+#pragma unroll 1
+                for (uint32_t j = 0; j < kWarpBytes / 32; ++j) {
+                    const uint32_t p = warp * kWarpBytes + j * 32 + lane;   // a byte a lane
+                    const bool nl = buf[p] == '\n' && k * kTile + p >= off;
+                    const uint32_t b = __ballot_sync(0xffffffffu, nl);
+                    const uint64_t at = k * kTile + p + 1;
+                    if (nl && at < end) put_any(i + __popc(b & ((1u << lane) - 1u)), at - off);
+                    i += __popc(b);
+                }
+            }
+            if (tile_of[ns] < tiles) scan(ns, nph, tile_of[ns], parity ^ 1u);
+            if (listed) {
+                for (uint32_t j = warp * 32 + lane; j - lane < lines; j += kWorkers * 32) {
+                    FastRow row;
+                    bool fast = false;
+                    if (j < lines && k * kTile + starts[j] < end) fast = parse_fast(buf, starts[j], starts[j + 1], months, row);
+                    const uint64_t i = prefix() + j;
+                    fast &= i < capacity;
+                    if (fast) {
+                        o.ship[i] = row.ship;
+                        o.qty[i] = row.qty;
+                        o.price[i] = row.price;
+                        o.disc[i] = row.disc;
+                        o.tax[i] = row.tax;
+                        o.rf[i] = (char)row.flags;
+                        o.ls[i] = (char)(row.flags >> 8);
+                    } else if (j < lines) {
+                        const uint64_t at = k * kTile + starts[j];
+                        if (at < end) put_any(i, at - off);
+                    }
                 }
             }
         }
-        __syncthreads();
-        const uint32_t cnt = T - r0 < kList ? T - r0 : kList;
-        for (uint32_t j = tid; j < cnt; j += kThreads) {
-            const uint64_t i = tile + starts[j];            // a newline; the next line is row first + rank + 1
-            if (i + 1 < bytes) one(i + 1, first + r0 + j + 1);
+        s = ns, ph = nph, parity ^= 1u;
+    }
+    // Never leave with copies in flight (only after a failed wait are there any).
+    if (tid == 0 && failed_s)
+        for (uint32_t i = 0; i < kRing; ++i) {
+            if (tile_of[s] < tiles) mbar_wait(smem_addr(&full_bar[s]), ph, status);
+            if (++s == kRing) s = 0, ph ^= 1u;
         }
-        __syncthreads();
-    }
-    if (nbad) {
-        atomicAdd(&bad[0], nbad);
-        atomicMin(&bad[1], first_bad);
-    }
 }
 
-uint64_t tbl_tiles(uint64_t bytes) { return (bytes + tbl::kTile - 1) / tbl::kTile; }
-
-cudaError_t launch_tbl_count(const char* text, uint64_t bytes, unsigned long long* tile_lines, cudaStream_t stream) {
-    const uint64_t tiles = tbl_tiles(bytes);
-    if (tiles) {
-        tbl_count_kernel<<<(unsigned)tiles, tbl::kThreads, 0, stream>>>(text, bytes, tile_lines);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    tbl_scan_kernel<<<1, 1024, 0, stream>>>(tile_lines, tiles);
+cudaError_t launch_tbl_count(const char* text, uint64_t bytes, unsigned long long* total, int sm_count,
+                             cudaStream_t stream) {
+    cudaError_t e = cudaMemsetAsync(total, 0, 8, stream);
+    if (e != cudaSuccess || !bytes) return e;
+    const uint64_t blocks = (bytes + 31) / 16 / 256 + 1, cap = (uint64_t)sm_count * 16;
+    tbl_count_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, stream>>>(text, bytes, total);
     return cudaGetLastError();
 }
 
-cudaError_t launch_tbl_parse(const char* text, uint64_t bytes, const unsigned long long* tile_first,
-                             int32_t* ship, int64_t* qty, int64_t* price, int64_t* disc, int64_t* tax, char* rf,
-                             char* ls, uint64_t capacity, unsigned long long* bad, cudaStream_t stream) {
-    const uint64_t tiles = tbl_tiles(bytes);
-    if (!tiles) return cudaSuccess;
-    tbl::Out o{ship, qty, price, disc, tax, rf, ls};
-    tbl_parse_kernel<<<(unsigned)tiles, tbl::kThreads, 0, stream>>>(text, bytes, tile_first, o, capacity, bad);
+static uint64_t tbl_tiles(const char* text, uint64_t bytes) {
+    return ((reinterpret_cast<uintptr_t>(text) & 15u) + bytes + tbl::kTile - 1) / tbl::kTile;
+}
+
+uint64_t tbl_scratch_bytes(const char* text, uint64_t bytes) {
+    static_assert(sizeof(TblResult) % 16 == 0, "states start on a 16-byte boundary");
+    return sizeof(TblResult) + 8 * (tbl::kStatePad + ((tbl_tiles(text, bytes) + 1) & ~1ull));
+}
+
+cudaError_t launch_tbl_parse(const char* text, uint64_t bytes, void* scratch, int32_t* ship, int64_t* qty,
+                             int64_t* price, int64_t* disc, int64_t* tax, char* rf, char* ls, uint64_t capacity,
+                             int sm_count, cudaStream_t stream) {
+    using namespace tbl;
+    const uint64_t tiles = tbl_tiles(text, bytes);
+    cudaError_t e = cudaMemsetAsync(scratch, 0, tbl_scratch_bytes(text, bytes), stream);
+    if (e != cudaSuccess || !bytes) return e;
+    const uint32_t dyn = kRing * kStageBytes;
+    if ((e = cudaFuncSetAttribute(tbl_parse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn)) != cudaSuccess)
+        return e;
+    TblResult* res = static_cast<TblResult*>(scratch);
+    Out o{ship, qty, price, disc, tax, rf, ls};
+    const uint64_t end = (reinterpret_cast<uintptr_t>(text) & 15u) + bytes;
+    const uint64_t full_tiles = end < kAhead ? 0 : (end - kAhead) / kTile;   // those with all of their kAhead bytes
+    const uint64_t cap = (uint64_t)sm_count;
+    tbl_parse_kernel<<<(unsigned)(tiles < cap ? tiles : cap), kThreads, dyn, stream>>>(
+        text, bytes, o, capacity, tiles, full_tiles, reinterpret_cast<unsigned long long*>(res + 1) + kStatePad, res);
     return cudaGetLastError();
 }
 
