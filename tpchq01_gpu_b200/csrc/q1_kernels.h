@@ -25,44 +25,36 @@ enum ScanPlacement : int {
     kPlaceGlobal = 4,
 };
 
-// Consumer warps per CTA (plus one producer warp), per input layout and placement, as measured on
-// the 600 M-row table (100 M uncompressed). More warps per SM sub-partition hide more of the decode's
-// issue latency where the registers allow. 12 warps leave 128 registers a thread (13 warps, which the
-// allocator rounds up to 16 warps' worth): the pair layouts' kernels fit (in_registers_per_thread
-// 0.909 -> 0.871 ms; in_registers, shared and global 5-20% faster), and so do the separate-flag
-// layouts' register placements, which keep only four groups' planes in registers (A/O and R/O go
-// to the CTA's shared table: per-thread 1.129 ms with 8 warps and six planes, 1.044 with 10, 0.980
-// with 12; global 1.31 -> 1.22 -> 1.16). Their shared placement runs 10 (3.04 -> 2.71 ms), and so
-// does the uncompressed layout, which needs up to 168 registers (per-thread 0.625 -> 0.600 ms
-// although one register spills; shared 0.670 -> 0.548). local_mem keeps 8 with compressed rows
-// (its per-thread tables run out of L1 with more threads: pair 2.83 -> 3.06 ms), and so does the
-// separate layout's in_registers (3.58 -> 3.65 ms with 10).
+// Consumer warps per CTA (plus one producer warp), per input layout, as measured on the 600 M-row
+// table (100 M uncompressed). More warps per SM sub-partition hide more of the decode's issue latency
+// where the registers allow. 12 warps leave 128 registers a thread (13 warps, which the allocator
+// rounds up to 16 warps' worth): the compressed layouts' kernels fit, the separate-flag ones by
+// keeping only four groups' planes in registers (A/O and R/O go to the CTA's shared table). Pair
+// layout 0.909 -> 0.871 ms, separate flags 1.129 ms with 8 warps and six planes, 1.044 with 10, 0.980
+// with 12. The uncompressed layout runs 10: it needs up to 168 registers (per-thread 0.625 -> 0.600 ms
+// although one register spills; shared 0.670 -> 0.548).
 template <int L, int P>
 inline constexpr uint32_t kConsumerWarps =
-    (L == kLayPair || L == kLayPairFilter) ? (P == kPlaceLocalMem ? 8u : 12u)
-    : (L == kLaySep || L == kLaySepFilter)
-        ? ((P == kPlaceLocalMem || P == kPlaceInRegisters) ? 8u
-                                                           : ((P == kPlaceSharedMemPerThread) ? 10u : 12u))
-        : 10u;
+    L == kLayUncomp || ((L == kLaySep || L == kLaySepFilter) && P == kPlaceInRegisters) ? 10u : 12u;
 // Rows per tile (one bulk copy per column per tile): a multiple of 128, so that every column slice
 // of every tile starts on a 16-byte boundary down to 1-bit columns, and of the consumer threads x
 // the rows of a step, so that a tile's steps divide evenly among the consumer threads.
 template <int L, int P>
 inline constexpr uint32_t kTileRows =
-    (L == kLayUncomp) ? 128u * kConsumerWarps<L, P> : (kConsumerWarps<L, P> == 8u ? 4096u : 384u * kConsumerWarps<L, P>);
-// Shared-memory ring depth.
+    (L == kLayUncomp ? 128u : 384u) * kConsumerWarps<L, P>;
+// Shared-memory ring depth: 3 where the shared placement's tables take the room of the fourth.
 template <int L, int P>
-inline constexpr uint32_t kStages = (P == kPlaceSharedMemPerThread) ? 3u : 4u;
-// Tiles a warp of the global placement write-combines in registers between its atomic adds into
-// the global table (12 or 16 rows per thread of a compressed tile, so 49,152 or 65,536 rows per warp
-// between flushes; a few flushes per warp over 600 M rows). Measured on 600 M rows (8 warps,
-// 4096-row tiles): 1 tile 12.94 ms (same-address L2 atomics serialise: 7.1 M atomic requests per
-// 100 M rows), 4 tiles 4.05 ms, 16 tiles 1.95 ms, 64 tiles 1.22 ms, 128 tiles 1.08 ms. A 64-bit
-// warp sum bounds the rows a thread may buffer (the kernel's static_assert).
-#ifndef Q1_GLOBAL_FLUSH_TILES
-#define Q1_GLOBAL_FLUSH_TILES 128
+inline constexpr uint32_t kStages = (P == kPlaceSharedMemPerThread && L != kLayPair && L != kLayPairFilter) ? 3u : 4u;
+// Tiles a thread sums in registers before its sums go to the table of a placement that keeps it
+// elsewhere (12 rows a thread and tile, 4 of the uncompressed layout: 49,152 rows a warp between
+// two flushes, a few per warp over 600 M rows). The global placement sets it: 600 M rows (8 warps,
+// 4096-row tiles) took 12.94 ms with 1 tile (same-address L2 atomics serialise), 4.05 ms with 4,
+// 1.95 ms with 16, 1.22 ms with 64 and 1.08 ms with 128. A 64-bit warp sum bounds the rows a thread
+// may buffer (the kernel's static_assert).
+#ifndef Q1_COMBINE_TILES
+#define Q1_COMBINE_TILES 128
 #endif
-inline constexpr uint32_t kGlobalFlushTiles = Q1_GLOBAL_FLUSH_TILES;
+inline constexpr uint32_t kCombineTiles = Q1_COMBINE_TILES;
 
 struct ScanParams {
     const uint8_t* col[7];      // column base pointers in tile order; 16-byte aligned

@@ -117,82 +117,25 @@ __host__ __device__ constexpr uint32_t stage_bytes(uint32_t R) {
 //   q  quantity (whole units for compressed, hundredths for uncompressed)
 //   d  discount, a = 100 - d, ab = a * (100 + tax), p = extendedprice
 
-// Aggregates of one group, per thread, in registers.
-template <bool kWideQty>
+// Aggregates of one group, per thread, in registers (reference-typed rows, one at a time).
 struct GroupRegs {
-    uint64_t p, dp, ch;
-    uint64_t qd64;      // packed: sum q (low 32) | sum d (high 32)   [!kWideQty]
-    uint64_t q64;       // sum q                                      [kWideQty]
-    uint32_t qd, d32, cnt;
+    uint64_t p, dp, ch, q;
+    uint32_t d, cnt;
 
     __device__ __forceinline__ void zero() {
-        p = dp = ch = qd64 = q64 = 0;
-        qd = d32 = cnt = 0;
+        p = dp = ch = q = 0;
+        d = cnt = 0;
     }
-    __device__ __forceinline__ void add(bool hit, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t pr) {
+    __device__ __forceinline__ void add(bool hit, uint32_t qty, uint32_t disc, uint32_t a, uint32_t ab, uint32_t pr) {
         const uint32_t pg = hit ? pr : 0u;
-        if (kWideQty) {
-            q64 = mad_wide(hit ? q : 0u, 1u, q64);
-            d32 += hit ? d : 0u;
-        } else {
-            qd += hit ? (q | (d << 16)) : 0u;
-        }
+        q = mad_wide(hit ? qty : 0u, 1u, q);
+        d += hit ? disc : 0u;
         cnt += hit ? 1u : 0u;
         p += pg;
         dp = mad_wide(a, pg, dp);
         ch = mad_wide(ab, pg, ch);
     }
-    // Move the 16-bit packed partials into 64 bits; needed at least every 256 rows.
-    __device__ __forceinline__ void fold() {
-        if (!kWideQty) {
-            qd64 += (uint64_t)(qd & 0xFFFFu) | ((uint64_t)(qd >> 16) << 32);
-            qd = 0;
-        }
-    }
-    // Aggregate values in q1 order (count, qty, price, disc, disc_price, charge); after fold().
-    __device__ __forceinline__ uint64_t value(int agg) const {
-        switch (agg) {
-            case kAggCount: return cnt;
-            case kAggQty: return kWideQty ? q64 : (qd64 & 0xFFFFFFFFull);
-            case kAggBasePrice: return p;
-            case kAggDisc: return kWideQty ? (uint64_t)d32 : (qd64 >> 32);
-            case kAggDiscPrice: return dp;
-            default: return ch;
-        }
-    }
-};
-
-// Code of row r of a quad (0..7 = group code, 7 also = filtered out) for row-wise placements.
-__device__ __forceinline__ uint32_t quad_code(const Quad& x, int r) {
-    const uint32_t b = (x.OH >> (8 * r)) & 0xFFu;
-    return b ? (uint32_t)(__ffs(b) - 1) : 7u;
-}
-
-// Aggregates of one group, per thread, fed a quad at a time. W1 (byte r = 1 iff row r is in the
-// group) drives three byte dot products (count, quantity, discount of 4 rows in one dp4a each);
-// the price products use the FMA pipe: pg = m * p (m in {0,1}), then wide multiply-adds.
-// 32-bit count/quantity/discount partials stay exact: a thread adds at most 2^15 rows per launch
-// (the host caps rows per launch at 2^15 per consumer thread), so quantity <= 255 * 2^15.
-struct GroupQuadRegs {
-    uint64_t p, dp, ch;
-    uint32_t cnt, q, d;
-    __device__ __forceinline__ void zero() {
-        p = dp = ch = 0;
-        cnt = q = d = 0;
-    }
-    __device__ __forceinline__ void add_quad(uint32_t W1, const Quad& x) {
-        cnt = __dp4a(W1, 0x01010101u, cnt);
-        q = __dp4a(W1, x.Q, q);
-        d = __dp4a(W1, x.D, d);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const uint32_t m = __byte_perm(W1, 0u, 0x4440u | (uint32_t)r);
-            const uint32_t pg = m * x.p[r];
-            p += pg;
-            dp = mad_wide(x.a[r], pg, dp);
-            ch = mad_wide(x.ab[r], pg, ch);
-        }
-    }
+    // Aggregate values in q1 order (count, qty, price, disc, disc_price, charge).
     __device__ __forceinline__ uint64_t value(int agg) const {
         switch (agg) {
             case kAggCount: return cnt;
@@ -224,7 +167,7 @@ struct AccPerThread {
     // four other groups' planes take registers (a kernel of 128 registers a thread, 12 warps).
     static constexpr bool kCold = (G == 6) && !kWideQty;
     static constexpr int kPlanes = kWideQty ? 1 : (kCold ? 4 : G);
-    GroupRegs<kWideQty> g[kWideQty ? G : 1];      // row-wise path (uncompressed layout)
+    GroupRegs g[kWideQty ? G : 1];      // row-wise path (uncompressed layout)
     GroupPlanes gq[kPlanes];                      // quad path (compressed layouts)
     unsigned long long* red;                      // the CTA's [G][6][lo, hi] table (cold groups)
     // group of plane slot s: the codes themselves, or with cold groups AF, NF, NO, RF
@@ -299,12 +242,6 @@ struct AccPerThread {
             else add_quad_planes<false>(x);
         }
     }
-    __device__ __forceinline__ void fold() {
-        if constexpr (kWideQty) {
-#pragma unroll
-            for (int i = 0; i < G; ++i) g[i].fold();
-        }
-    }
     // plane slot of group i (not called for cold groups)
     static __device__ __forceinline__ constexpr int slot_of(int i) { return kCold ? (i == 0 ? 0 : i - 1) : i; }
     // The thread's partial of group i (0 for a cold group: its rows are in the CTA table already).
@@ -316,14 +253,11 @@ struct AccPerThread {
         if constexpr (kWideQty) g[i].zero();
         else if (!cold(i)) gq[slot_of(i)].zero();
     }
-    // whether this thread sums the rows of group code c (every thread reads every row it is given)
-    __device__ __forceinline__ bool owns(uint32_t) const { return true; }
     template <class P>
     __device__ __forceinline__ void tile_done(const P&, uint32_t) {}
     template <class P>
     __device__ __forceinline__ void finish(const P&, uint32_t) {}
     __device__ __forceinline__ void flush(CtaRed red, uint32_t lane) {
-        fold();
 #pragma unroll
         for (int i = 0; i < G; ++i) {
             if (cold(i)) continue;
@@ -337,272 +271,252 @@ struct AccPerThread {
     }
 };
 
-// --- in_registers ("warp-lane tables", src/kernels/ht_in_registers.cuh:30-121): the lanes of a
-// warp form floor(32/G) tables of G lanes; lane (table, g) keeps only group g in registers; all
-// G lanes of a table read the same rows (a shared-memory broadcast, so unlike the reference no
-// row is fetched from DRAM more than once) and each adds the rows of its own group.
+// The other placements keep their table elsewhere and write-combine: a thread sums its rows of some
+// tiles in registers (AccPerThread, four rows an instruction), then adds the sums to the table.
+// Adding every quad or row to the table directly made the table the bound: 600 M pair-layout rows
+// took 1.95 ms (in_registers: every lane of a table read all of its rows), 2.13 ms
+// (shared_mem_per_thread) and 3.19 ms (local_mem) against 0.88 ms in registers.
 template <int G, bool kWideQty>
-struct AccWarpLane {
-    GroupRegs<kWideQty> r;
-    GroupQuadRegs rq;
-    uint32_t my;
-    __device__ __forceinline__ void init(uint32_t lane, uint32_t, uint8_t*, unsigned long long*) {
-        r.zero();
-        rq.zero();
-        my = lane % G;
-    }
-    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
-        if constexpr (kWideQty) {
-            r.add(c == my, q, d, a, ab, p);
-        } else {
-            Quad x;
-            x.OH = c == my ? 1u << my : 0u;
-            x.Q = q;
-            x.D = d;
-            x.a[0] = a;
-            x.ab[0] = ab;
-            x.p[0] = p;
-            x.a[1] = x.a[2] = x.a[3] = x.ab[1] = x.ab[2] = x.ab[3] = x.p[1] = x.p[2] = x.p[3] = 0;
-            add_quad(x);
-        }
-    }
-    __device__ __forceinline__ void add_quad(const Quad& x) { rq.add_quad((x.OH >> my) & 0x01010101u, x); }
-    __device__ __forceinline__ void fold() { r.fold(); }
-    // all G lanes of a table read the same rows; the lane of group c sums them
-    __device__ __forceinline__ bool owns(uint32_t c) const { return c == my; }
-    template <class P>
-    __device__ __forceinline__ void tile_done(const P&, uint32_t) {}
-    template <class P>
-    __device__ __forceinline__ void finish(const P&, uint32_t) {}
-    __device__ __forceinline__ void flush(CtaRed red, uint32_t lane) {
-        fold();
-        if (lane < (32u / G) * G) {
-#pragma unroll
-            for (int a = 0; a < kNumAggs; ++a) red.add((int)my, a, kWideQty ? r.value(a) : rq.value(a), 0);
-        }
-    }
-};
-
-// Sums of the rows of one group in a quad (W1: byte r is 1 iff row r is in the group): the packed
-// word count | quantity << 16 | discount << 39 (a thread adds at most 2^15 rows per launch, so
-// count < 2^16, quantity <= 255 * 2^15 < 2^23, discount <= 100 * 2^15 < 2^22) and price,
-// (100 - d) price and (100 - d)(100 + t) price.
-struct QuadGroupSums {
-    uint64_t w0, p, dp, ch;
-};
-__device__ __forceinline__ QuadGroupSums quad_group_sums(uint32_t W1, const Quad& x) {
-    QuadGroupSums s{0, 0, 0, 0};
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const uint32_t pg = __byte_perm(W1, 0u, 0x4440u | (uint32_t)r) * x.p[r];
-        s.p += pg;
-        s.dp = mad_wide(x.a[r], pg, s.dp);
-        s.ch = mad_wide(x.ab[r], pg, s.ch);
-    }
-    s.w0 = (uint64_t)__popc(W1) | ((uint64_t)__dp4a(W1, x.Q, 0u) << 16) | ((uint64_t)__dp4a(W1, x.D, 0u) << 39);
-    return s;
-}
-
-// --- local_mem (src/kernels/ht_in_local_mem.cuh:11-74): per-thread tables indexed by the row's
-// group, which places them in (L1-cached) local memory. A group's entry is four 64-bit words
-// (five for reference-typed columns, whose quantity needs a word of its own): the count, quantity
-// and discount share one word (see quad_group_sums), then price, (100 - d) price and
-// (100 - d)(100 + t) price. Compressed quads are added group by group, every lane of the warp at
-// the same group at a time: the group's four rows are summed in registers and its entry is
-// read and written once, by accesses that coalesce across the warp (a row-by-row update at each
-// row's own group scatters the warp's accesses over the table: 2.8 sectors per row each way,
-// L1-bound). Reference-typed rows come one at a time and update their group's entry.
-template <int G, bool kWideQty>
-struct AccLocal {
-    static constexpr int kWords = kWideQty ? 5 : 4;
-    static constexpr int kQtyShift = 16, kDiscShift = kWideQty ? 16 : 39;
-    uint64_t t[G][kWords];   // [0] count | quantity << 16 | discount << 39 (or count | discount << 16), [1] p,
-                             // [2] (100-d) p, [3] (100-d)(100+t) p, [4] quantity (reference-typed columns)
-    __device__ __forceinline__ void init(uint32_t, uint32_t, uint8_t*, unsigned long long*) {
-        for (int i = 0; i < G; ++i)
-            for (int j = 0; j < kWords; ++j) t[i][j] = 0;
-    }
-    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
-        if (c < (uint32_t)G) {
-            if constexpr (kWideQty) {
-                t[c][0] += 1ull | ((uint64_t)d << kDiscShift);
-                t[c][4] += q;
-            } else {
-                t[c][0] += 1ull | ((uint64_t)q << kQtyShift) | ((uint64_t)d << kDiscShift);
-            }
-            t[c][1] += p;
-            t[c][2] = mad_wide(a, p, t[c][2]);
-            t[c][3] = mad_wide(ab, p, t[c][3]);
-        }
-    }
-    __device__ __forceinline__ void add_quad(const Quad& x) {
-        // not unrolled, so that the table stays in local memory, indexed by the loop's group
-#pragma unroll 1
-        for (int g = 0; g < G; ++g) {
-            const uint32_t W1 = (x.OH >> g) & 0x01010101u;
-            if (W1) {
-                const QuadGroupSums q = quad_group_sums(W1, x);
-                t[g][0] += q.w0;
-                t[g][1] += q.p;
-                t[g][2] += q.dp;
-                t[g][3] += q.ch;
-            }
-        }
-    }
-    __device__ __forceinline__ void fold() {}
-    __device__ __forceinline__ bool owns(uint32_t) const { return true; }
-    template <class P>
-    __device__ __forceinline__ void tile_done(const P&, uint32_t) {}
-    template <class P>
-    __device__ __forceinline__ void finish(const P&, uint32_t) {}
-    __device__ __forceinline__ void flush(CtaRed red, uint32_t lane) {
-#pragma unroll
-        for (int i = 0; i < G; ++i) {
-            const uint64_t w0 = t[i][0];
-            const uint64_t qty = kWideQty ? t[i][kWords - 1] : (w0 >> kQtyShift) & ((1ull << 23) - 1);
-            const uint64_t vals[kNumAggs] = {w0 & 0xFFFFull, qty, t[i][1], w0 >> kDiscShift, t[i][2], t[i][3]};
-#pragma unroll
-            for (int a = 0; a < kNumAggs; ++a) {
-                uint64_t lo = vals[a], hi = 0;
-                warp_sum_u128(lo, hi);
-                if (lane == 0) red.add(i, a, lo, hi);
-            }
-        }
-    }
-};
-
-// --- shared_mem_per_thread (src/kernels/ht_in_shared_mem_per_thread.cuh:23-118): per-thread
-// tables in shared memory, laid out [word][group][thread] so a warp's accesses are bank-conflict
-// free. A group's entry holds the same words as the local_mem table, and compressed quads are
-// added group by group in the same way: every lane at the same group, one read-modify-write per
-// word and group.
-template <int G, bool kWideQty>
-struct AccSharedPerThread {
-    static constexpr int kWords = kWideQty ? 5 : 4;
-    static constexpr int kDiscShift = kWideQty ? 16 : 39;
-    uint64_t* tab;       // kWords * G * T entries: [w0, p, dp, ch, (quantity)][group][thread]
-    uint32_t tid, nthreads;
-    __device__ __forceinline__ void init(uint32_t, uint32_t consumer_tid, uint8_t* scratch, unsigned long long*) {
-        tid = consumer_tid;
-        nthreads = blockDim.x - 32;
-        tab = reinterpret_cast<uint64_t*>(scratch);
-        for (int i = 0; i < kWords * G; ++i) tab[i * nthreads + tid] = 0;
-    }
-    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
-        if (c < (uint32_t)G) {
-            const uint32_t base = c * nthreads + tid;
-            const uint32_t stride = G * nthreads;
-            if constexpr (kWideQty) {
-                tab[base] += 1ull | ((uint64_t)d << kDiscShift);
-                tab[base + 4 * stride] += q;
-            } else {
-                tab[base] += 1ull | ((uint64_t)q << 16) | ((uint64_t)d << kDiscShift);
-            }
-            tab[base + stride] += p;
-            tab[base + 2 * stride] = mad_wide(a, p, tab[base + 2 * stride]);
-            tab[base + 3 * stride] = mad_wide(ab, p, tab[base + 3 * stride]);
-        }
-    }
-    __device__ __forceinline__ void add_quad(const Quad& x) {
-        const uint32_t stride = G * nthreads;
-#pragma unroll 1
-        for (int g = 0; g < G; ++g) {
-            const uint32_t W1 = (x.OH >> g) & 0x01010101u;
-            if (W1) {
-                const QuadGroupSums q = quad_group_sums(W1, x);
-                const uint32_t base = g * nthreads + tid;
-                tab[base] += q.w0;
-                tab[base + stride] += q.p;
-                tab[base + 2 * stride] += q.dp;
-                tab[base + 3 * stride] += q.ch;
-            }
-        }
-    }
-    __device__ __forceinline__ void fold() {}
-    // whether this thread sums the rows of group code c (every thread reads every row it is given)
-    __device__ __forceinline__ bool owns(uint32_t) const { return true; }
-    template <class P>
-    __device__ __forceinline__ void tile_done(const P&, uint32_t) {}
-    template <class P>
-    __device__ __forceinline__ void finish(const P&, uint32_t) {}
-    __device__ __forceinline__ void flush(CtaRed red, uint32_t lane) {
-        const uint32_t stride = G * nthreads;
-#pragma unroll
-        for (int i = 0; i < G; ++i) {
-            const uint32_t base = i * nthreads + tid;
-            const uint64_t w0 = tab[base];
-            const uint64_t qty = kWideQty ? tab[base + 4 * stride] : (w0 >> 16) & ((1ull << 23) - 1);
-            const uint64_t vals[kNumAggs] = {w0 & 0xFFFFull, qty, tab[base + stride], w0 >> kDiscShift,
-                                             tab[base + 2 * stride], tab[base + 3 * stride]};
-#pragma unroll
-            for (int a = 0; a < kNumAggs; ++a) {
-                uint64_t lo = vals[a], hi = 0;
-                warp_sum_u128(lo, hi);
-                if (lane == 0) red.add(i, a, lo, hi);
-            }
-        }
-    }
-};
-
-// --- global (src/kernels/ht_in_global_mem.hpp:11-52): no thread- or block-private table; the
-// aggregates live only in the global output, updated by atomics all through the scan. The
-// reference issues 6 atomics per row; here each warp write-combines its rows of
-// kGlobalFlushTiles tiles in a register buffer, then issues one 128-bit atomic add per
-// (group, aggregate) straight into the global table and empties the buffer.
-template <int G, bool kWideQty>
-struct AccGlobal {
-    // A warp's flush of one sum is a 64-bit warp reduction; the kernel bounds the rows a lane
-    // buffers between flushes so that it cannot wrap.
-    static_assert(kGlobalFlushTiles >= 1, "flush cadence");
+struct AccCombining {
     AccPerThread<G, kWideQty> buf;
-    uint32_t tiles;
-    __device__ __forceinline__ void init(uint32_t a, uint32_t b, uint8_t* s, unsigned long long* r) {
-        buf.init(a, b, s, r);
+    uint32_t tiles;   // in buf
+    __device__ __forceinline__ void init_buffer(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
+        buf.init(lane, ctid, scratch, red);
         tiles = 0;
     }
     __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
         buf.add(c, q, d, a, ab, p);
     }
     __device__ __forceinline__ void add_quad(const Quad& x) { buf.add_quad(x); }
-    __device__ __forceinline__ void fold() { buf.fold(); }
-    __device__ __forceinline__ bool owns(uint32_t) const { return true; }
-    // Called by all lanes after each tile (warp-uniform count).
+    // Whether the buffer goes to the table now; called by all lanes after each tile.
+    __device__ __forceinline__ bool due() {
+        if (++tiles < kCombineTiles) return false;
+        tiles = 0;
+        return true;
+    }
+};
+
+// --- in_registers ("warp-lane tables", src/kernels/ht_in_registers.cuh:30-121): lane g of a warp
+// holds group g's sums in registers; the warp's buffers meet there through warp reductions. (In
+// the reference all lanes of a table read the same rows, each keeping those of its group.)
+template <int G, bool kWideQty>
+struct AccWarpLane : AccCombining<G, kWideQty> {
+    // lane g: group g. A launch gives a warp at most 2^20 rows: the charge sum takes 128 bits
+    // (2^47.2 a row), the others 64.
+    uint64_t t[kNumAggs], ch_hi;
+    __device__ __forceinline__ void init(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
+        this->init_buffer(lane, ctid, scratch, red);
+#pragma unroll
+        for (int a = 0; a < kNumAggs; ++a) t[a] = 0;
+        ch_hi = 0;
+    }
+    __device__ __forceinline__ void to_table(uint32_t lane) {
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+#pragma unroll
+            for (int a = 0; a < kNumAggs; ++a) {
+                const uint64_t v = warp_sum_u64(this->buf.value(i, a));
+                if (lane == (uint32_t)i) {
+                    t[a] += v;
+                    if (a == kAggCharge) ch_hi += t[a] < v ? 1u : 0u;
+                }
+            }
+            this->buf.zero_group(i);
+        }
+    }
+    template <class P>
+    __device__ __forceinline__ void tile_done(const P&, uint32_t lane) {
+        if (this->due()) to_table(lane);
+    }
+    template <class P>
+    __device__ __forceinline__ void finish(const P&, uint32_t lane) { to_table(lane); }
+    __device__ __forceinline__ void flush(CtaRed red, uint32_t lane) {
+        if (lane < (uint32_t)G) {
+#pragma unroll
+            for (int a = 0; a < kNumAggs; ++a) red.add((int)lane, a, t[a], a == kAggCharge ? ch_hi : 0);
+        }
+    }
+};
+
+// A group's entry in the per-thread tables below: count, quantity and discount in one word (a thread
+// adds at most 2^15 rows per launch, so count < 2^16, quantity <= 255 * 2^15 < 2^23, discount
+// <= 100 * 2^15 < 2^22), then price, (100 - d) price and (100 - d)(100 + t) price. Reference-typed
+// rows' quantity takes a word of its own.
+template <bool kWideQty>
+struct Entry {
+    static constexpr int kWords = kWideQty ? 5 : 4;
+    static constexpr int kQtyShift = 16, kDiscShift = kWideQty ? 16 : 39;
+    // word w of a group's sums
+    template <class Buf>
+    static __device__ __forceinline__ uint64_t word(const Buf& b, int i, int w) {
+        switch (w) {
+            case 0:
+                return b.value(i, kAggCount) | (kWideQty ? 0ull : b.value(i, kAggQty) << kQtyShift) |
+                       (b.value(i, kAggDisc) << kDiscShift);
+            case 1: return b.value(i, kAggBasePrice);
+            case 2: return b.value(i, kAggDiscPrice);
+            case 3: return b.value(i, kAggCharge);
+            default: return b.value(i, kAggQty);
+        }
+    }
+    // aggregate a of the words w
+    static __device__ __forceinline__ uint64_t value(const uint64_t w[kWords], int a) {
+        switch (a) {
+            case kAggCount: return w[0] & 0xFFFFull;
+            case kAggQty: return kWideQty ? w[kWords - 1] : (w[0] >> kQtyShift) & ((1ull << 23) - 1);
+            case kAggBasePrice: return w[1];
+            case kAggDisc: return w[0] >> kDiscShift;
+            case kAggDiscPrice: return w[2];
+            default: return w[3];
+        }
+    }
+    // The warp's sum of group i's entries into the CTA's table.
+    static __device__ __forceinline__ void reduce(const uint64_t w[kWords], int i, CtaRed red, uint32_t lane) {
+#pragma unroll
+        for (int a = 0; a < kNumAggs; ++a) {
+            uint64_t lo = value(w, a), hi = 0;
+            warp_sum_u128(lo, hi);
+            if (lane == 0) red.add(i, a, lo, hi);
+        }
+    }
+};
+
+// --- local_mem (src/kernels/ht_in_local_mem.cuh:11-74): per-thread tables in (L1-cached) local
+// memory.
+template <int G, bool kWideQty>
+struct AccLocal : AccCombining<G, kWideQty> {
+    using E = Entry<kWideQty>;
+    volatile uint64_t t[G][E::kWords];   // (volatile: not in registers)
+    __device__ __forceinline__ void init(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
+        this->init_buffer(lane, ctid, scratch, red);
+        for (int i = 0; i < G; ++i)
+            for (int j = 0; j < E::kWords; ++j) t[i][j] = 0;
+    }
+    __device__ __forceinline__ void to_table() {
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            if (this->buf.cold(i)) continue;
+#pragma unroll
+            for (int j = 0; j < E::kWords; ++j) t[i][j] = t[i][j] + E::word(this->buf, i, j);
+            this->buf.zero_group(i);
+        }
+    }
+    template <class P>
+    __device__ __forceinline__ void tile_done(const P&, uint32_t) {
+        if (this->due()) to_table();
+    }
+    template <class P>
+    __device__ __forceinline__ void finish(const P&, uint32_t) { to_table(); }
+    __device__ __forceinline__ void flush(CtaRed red, uint32_t lane) {
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            if (this->buf.cold(i)) continue;
+            uint64_t w[E::kWords];
+#pragma unroll
+            for (int j = 0; j < E::kWords; ++j) w[j] = t[i][j];
+            E::reduce(w, i, red, lane);
+        }
+    }
+};
+
+// --- shared_mem_per_thread (src/kernels/ht_in_shared_mem_per_thread.cuh:23-118): per-thread
+// tables in shared memory, laid out [word][group][thread] so a warp's accesses are bank-conflict
+// free. Reference-typed rows update their group's entry row by row: six groups' 64-bit sums in
+// registers cost more than the table (100 M rows 0.599 ms against 0.548 ms).
+template <int G, bool kWideQty, uint32_t kThreads>
+struct AccSharedPerThread : AccCombining<G, kWideQty> {
+    using E = Entry<kWideQty>;
+    uint64_t* tab;       // this thread's column of [w0, p, dp, ch, (quantity)][group][thread]
+    __device__ __forceinline__ void init(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
+        this->init_buffer(lane, ctid, scratch, red);
+        tab = reinterpret_cast<uint64_t*>(scratch) + ctid;
+#pragma unroll
+        for (int i = 0; i < E::kWords * G; ++i) tab[i * kThreads] = 0;
+    }
+    __device__ __forceinline__ uint64_t& entry(uint32_t i, uint32_t j) { return tab[(j * G + i) * kThreads]; }
+    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
+        if constexpr (kWideQty) {
+            if (c < (uint32_t)G) {
+                entry(c, 0) += 1ull | ((uint64_t)d << E::kDiscShift);
+                entry(c, 4) += q;
+                entry(c, 1) += p;
+                entry(c, 2) = mad_wide(a, p, entry(c, 2));
+                entry(c, 3) = mad_wide(ab, p, entry(c, 3));
+            }
+        } else {
+            this->buf.add(c, q, d, a, ab, p);
+        }
+    }
+    __device__ __forceinline__ void to_table() {
+        if constexpr (!kWideQty) {
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                if (this->buf.cold(i)) continue;
+#pragma unroll
+                for (int j = 0; j < E::kWords; ++j) entry(i, j) += E::word(this->buf, i, j);
+                this->buf.zero_group(i);
+            }
+        }
+    }
+    template <class P>
+    __device__ __forceinline__ void tile_done(const P&, uint32_t) {
+        if (this->due()) to_table();
+    }
+    template <class P>
+    __device__ __forceinline__ void finish(const P&, uint32_t) { to_table(); }
+    __device__ __forceinline__ void flush(CtaRed red, uint32_t lane) {
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            if (this->buf.cold(i)) continue;
+            uint64_t w[E::kWords];
+#pragma unroll
+            for (int j = 0; j < E::kWords; ++j) w[j] = entry(i, j);
+            E::reduce(w, i, red, lane);
+        }
+    }
+};
+
+// --- global (src/kernels/ht_in_global_mem.hpp:11-52): no thread- or block-private table; the
+// aggregates live only in the global output, updated by atomics all through the scan. The
+// reference issues 6 atomics per row; here each warp issues one 128-bit atomic add per (group,
+// aggregate) for its buffered rows straight into the global table.
+template <int G, bool kWideQty>
+struct AccGlobal : AccCombining<G, kWideQty> {
+    __device__ __forceinline__ void init(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
+        this->init_buffer(lane, ctid, scratch, red);
+    }
     template <class P>
     __device__ __forceinline__ void tile_done(const P& prm, uint32_t lane) {
-        buf.fold();
-        if (++tiles < kGlobalFlushTiles) return;
-        to_global(prm, lane);
+        if (this->due()) to_global(prm, lane);
     }
     template <class P>
-    __device__ __forceinline__ void finish(const P& prm, uint32_t lane) {
-        buf.fold();
-        if (tiles) to_global(prm, lane);
-    }
+    __device__ __forceinline__ void finish(const P&, uint32_t) {}
     template <class P>
     __device__ __forceinline__ void to_global(const P& prm, uint32_t lane) {
-        tiles = 0;
 #pragma unroll
         for (int i = 0; i < G; ++i) {
             const int grp = G == 4 ? prm.pair_group[i] : i;
 #pragma unroll
             for (int a = 0; a < kNumAggs; ++a) {
-                uint64_t v = warp_sum_u64(buf.value(i, a));
+                uint64_t v = warp_sum_u64(this->buf.value(i, a));
                 if (a == kAggQty) v *= prm.qty_scale;
                 if (lane == (uint32_t)((i * kNumAggs + a) & 31)) atomic_add_u128(prm.out + 2 * (grp * kNumAggs + a), v, 0);
             }
-            buf.zero_group(i);
+            this->buf.zero_group(i);
         }
     }
-    __device__ __forceinline__ void flush(CtaRed, uint32_t) {}
+    // What is left at the end goes through the CTA's reduction, one atomic per CTA and sum instead of
+    // one per warp (60 M rows: 0.118 -> 0.107 ms).
+    __device__ __forceinline__ void flush(CtaRed red, uint32_t lane) { this->buf.flush(red, lane); }
 };
 
-template <int P, int G, bool W>
+template <int P, int G, bool W, uint32_t T>
 struct AccSel;
-template <int G, bool W> struct AccSel<kPlaceInRegisters, G, W> { using T = AccWarpLane<G, W>; };
-template <int G, bool W> struct AccSel<kPlaceInRegistersPerThread, G, W> { using T = AccPerThread<G, W>; };
-template <int G, bool W> struct AccSel<kPlaceLocalMem, G, W> { using T = AccLocal<G, W>; };
-template <int G, bool W> struct AccSel<kPlaceSharedMemPerThread, G, W> { using T = AccSharedPerThread<G, W>; };
-template <int G, bool W> struct AccSel<kPlaceGlobal, G, W> { using T = AccGlobal<G, W>; };
+template <int G, bool W, uint32_t T> struct AccSel<kPlaceInRegisters, G, W, T> { using A = AccWarpLane<G, W>; };
+template <int G, bool W, uint32_t T> struct AccSel<kPlaceInRegistersPerThread, G, W, T> { using A = AccPerThread<G, W>; };
+template <int G, bool W, uint32_t T> struct AccSel<kPlaceLocalMem, G, W, T> { using A = AccLocal<G, W>; };
+template <int G, bool W, uint32_t T> struct AccSel<kPlaceSharedMemPerThread, G, W, T> { using A = AccSharedPerThread<G, W, T>; };
+template <int G, bool W, uint32_t T> struct AccSel<kPlaceGlobal, G, W, T> { using A = AccGlobal<G, W>; };
 
 // ---------------------------------------------------------------------------------------------
 // Row decoding
@@ -656,8 +570,7 @@ __device__ __forceinline__ void process_step(const ScanParams& prm, uint32_t bas
         const uint4 P = lds_v4(base + col_offset<L>(4, R) + 16 * j);
         const uint32_t RF = lds_u16(base + col_offset<L>(5, R) + 2 * j);
         const uint32_t LS = lds_u16(base + col_offset<L>(6, R) + 2 * j);
-        // Both rows in the fast domain (always, in TPC-H data): the placement's tables only. A
-        // per-thread branch, not a warp vote: the warp-lane placement's lanes may diverge here.
+        // Both rows in the fast domain (always, in TPC-H data): the placement's tables only.
         const bool fast = ((Q.y | Q.w | D.y | D.w | X.y | X.w | P.y | P.w) == 0u) & (D.x <= 100u) & (D.z <= 100u) &
                           (X.x <= 255u) & (X.z <= 255u);
         if (fast) {
@@ -685,7 +598,7 @@ __device__ __forceinline__ void process_step(const ScanParams& prm, uint32_t bas
                 const bool wide =
                     ((r ? (Q.w | D.w | X.w | P.w) : (Q.y | D.y | X.y | P.y)) != 0u) | (d > 100u) | (t > 255u);
                 const bool pass = ship <= cut;
-                if (wide && pass && acc.owns(code))
+                if (wide && pass)
                     wide_row(prm, code, (int64_t)((uint64_t)(r ? Q.w : Q.y) << 32 | q),
                              (int64_t)((uint64_t)(r ? D.w : D.y) << 32 | d),
                              (int64_t)((uint64_t)(r ? X.w : X.y) << 32 | t),
@@ -743,7 +656,7 @@ __device__ __forceinline__ void process_row_global(const ScanParams& prm, uint64
         const uint32_t ls = (uint8_t)__ldg(reinterpret_cast<const char*>(prm.col[6]) + i);
         const bool wide = ((q | p) >> 32) != 0 || d > 100u || t > 255u;
         const bool pass = ship <= prm.cutoff;
-        if (wide && pass && acc.owns(code_of_chars(rf, ls)))
+        if (wide && pass)
             wide_row(prm, code_of_chars(rf, ls), (int64_t)q, (int64_t)d, (int64_t)t, (int64_t)p);
         const uint32_t c = (pass && !wide) ? code_of_chars(rf, ls) : 7u;
         const uint32_t a = 100u - (uint32_t)d;
@@ -845,25 +758,18 @@ q1_scan_kernel(const __grid_constant__ ScanParams prm) {
         }
     } else {
         // ----------------------------- consumer warps -----------------------------------
-        using Acc = typename AccSel<P, G, T::kWideQty>::T;
+        using Acc = typename AccSel<P, G, T::kWideQty, W * 32>::A;
         const uint32_t ctid = threadIdx.x;  // 0 .. 32W-1
         Acc acc;
         acc.init(lane, ctid, smem + S * kStage, red);
         uint32_t bad = 0;
         constexpr uint32_t kSteps = R / T::kRowsPerStep;  // steps per tile
-        // Rows one consumer thread adds per tile, and how often the 16-bit packed partials
-        // (quantity <= 255 per row) must be folded into 64 bits: at most every 257 rows.
-        constexpr uint32_t kTablesPerWarp = 32u / G;
-        constexpr uint32_t kRowsPerThreadTile =
-            (P == kPlaceInRegisters) ? (kSteps + W * kTablesPerWarp - 1) / (W * kTablesPerWarp) * T::kRowsPerStep
-                                     : kSteps / (W * 32) * T::kRowsPerStep;
-        constexpr uint32_t kFoldEvery = (257u / kRowsPerThreadTile) > 0 ? (257u / kRowsPerThreadTile) : 1u;
-        static_assert(kRowsPerThreadTile <= 257u, "tile too large for the packed partials");
+        // Rows one consumer thread adds per tile.
+        constexpr uint32_t kRowsPerThreadTile = kSteps / (W * 32) * T::kRowsPerStep;
         static_assert(kSteps % (W * 32) == 0, "steps must divide evenly among consumer threads");
-        // The global placement's warp flush is a 64-bit sum of 32 lanes' buffered rows: at most
-        // 2048 rows a lane of charges below 100 (2^32 - 1) 355 < 2^47.2 stays below 2^64.
-        static_assert(P != kPlaceGlobal || kRowsPerThreadTile * kGlobalFlushTiles <= 2048u,
-                      "global flush sums must stay below 2^64");
+        // The in_registers and global placements sum a warp's buffers in 64 bits: at most 2048 rows
+        // a lane of charges below 100 (2^32 - 1) 355 < 2^47.2 stays below 2^64.
+        static_assert(kRowsPerThreadTile * kCombineTiles <= 2048u, "warp sums must stay below 2^64");
         bool ok = true;
         uint32_t k = 0;
         for (uint64_t t = blockIdx.x; t < num_tiles; t += gridDim.x, ++k) {
@@ -875,35 +781,17 @@ q1_scan_kernel(const __grid_constant__ ScanParams prm) {
                 break;
             }
             const uint32_t base = ring + s * kStage;
-            if constexpr (P == kPlaceInRegisters) {
-                const uint32_t tbl = lane / G;
-                if (tbl < kTablesPerWarp) {
-                    for (uint32_t j = warp * kTablesPerWarp + tbl; j < kSteps; j += W * kTablesPerWarp)
-                        process_step<L, R>(prm, base, j, prm.cutoff, lut, acc, bad);
-                }
-            } else {
 #pragma unroll
-                for (uint32_t it = 0; it < kSteps / (W * 32); ++it)
-                    process_step<L, R>(prm, base, ctid + it * (W * 32), prm.cutoff, lut, acc, bad);
-            }
+            for (uint32_t it = 0; it < kSteps / (W * 32); ++it)
+                process_step<L, R>(prm, base, ctid + it * (W * 32), prm.cutoff, lut, acc, bad);
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_addr(&empty_bar[s]));
             acc.tile_done(prm, lane);
-            if ((k + 1) % kFoldEvery == 0) acc.fold();
         }
-        acc.fold();
         // Tail rows [num_tiles * R, rows): handled by the CTA next in the round robin.
         if (ok && blockIdx.x == (uint32_t)(num_tiles % gridDim.x)) {
             const uint64_t first = num_tiles * R;
-            if constexpr (P == kPlaceInRegisters) {
-                const uint32_t tbl = lane / G;
-                if (tbl < kTablesPerWarp) {
-                    for (uint64_t i = first + warp * kTablesPerWarp + tbl; i < prm.rows; i += W * kTablesPerWarp)
-                        process_row_global<L>(prm, i, acc, bad);
-                }
-            } else {
-                for (uint64_t i = first + ctid; i < prm.rows; i += W * 32) process_row_global<L>(prm, i, acc, bad);
-            }
+            for (uint64_t i = first + ctid; i < prm.rows; i += W * 32) process_row_global<L>(prm, i, acc, bad);
             acc.tile_done(prm, lane);
         }
         acc.finish(prm, lane);
@@ -961,8 +849,9 @@ static cudaError_t launch_one(const ScanParams& prm, int sm_count, int max_block
     constexpr uint32_t S = kStages<L, P>;
     constexpr uint32_t W = kConsumerWarps<L, P>;
     constexpr int G = LayoutTraits<L>::kCodes;
-    uint32_t dyn = S * stage_bytes<L>(R);
-    if (P == kPlaceSharedMemPerThread) dyn += (uint32_t)(8 * (L == kLayUncomp ? 5 : 4) * G * W * 32);
+    constexpr uint32_t dyn =
+        S * stage_bytes<L>(R) + (P == kPlaceSharedMemPerThread ? 8u * Entry<L == kLayUncomp>::kWords * G * W * 32u : 0u);
+    static_assert(dyn + 2048 <= 227 * 1024, "ring and tables beside the static shared memory");
     cudaError_t e = cudaFuncSetAttribute(q1_scan_kernel<L, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = scan_grid_blocks(L, P, prm.rows, sm_count, max_blocks);
@@ -1024,11 +913,8 @@ Geometry geometry(int layout, int placement) {
 }  // namespace
 
 uint64_t scan_max_rows_per_launch(int layout, int placement, uint32_t grid) {
-    // accumulating lanes per CTA: every consumer thread, or the lanes of one warp-lane table
-    const uint64_t codes = (layout == kLayPair || layout == kLayPairFilter) ? 4 : 6;
     const Geometry g = geometry(layout, placement);
-    const uint64_t lanes = placement == kPlaceInRegisters ? g.warps * (32 / codes) : g.warps * 32ull;
-    uint64_t n = (uint64_t)grid * lanes * 32768ull;
+    uint64_t n = (uint64_t)grid * g.warps * 32ull * 32768ull;   // every consumer thread sums its own rows
     if (n > (1ull << 31)) n = 1ull << 31;
     return n / g.tile_rows * g.tile_rows;
 }
