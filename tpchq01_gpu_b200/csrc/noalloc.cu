@@ -12,9 +12,9 @@
 // In the placements with per-thread or per-lane tables (in_registers, in_registers_per_thread,
 // local_mem, shared_mem_per_thread) the scan kernel writes its CTA's partial sums into its record
 // instead of one 128-bit atomic per (group, aggregate) into the caller's table, and a one-block
-// reduction kernel adds the records into the caller's table. The global placement keeps no CTA
-// partials: its warps add every tile's sums straight into the caller's table, as they do under
-// q1_launch_compressed, so its records stay zero and the reduction adds nothing.
+// reduction kernel adds the records into the caller's table. The global placement's warps add their
+// sums of full buffers straight into the caller's table, as they do under q1_launch_compressed; its
+// records hold what was left in the buffers at the end.
 // Limit: at most kNoAllocMaxCtas CTAs per launch (the library uses one per SM, 148 on a B200).
 //
 // The array is shared by every call and keeps the last call's contents: each call clears the
