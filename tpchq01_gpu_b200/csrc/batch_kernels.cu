@@ -114,7 +114,9 @@ __device__ __forceinline__ bool consume_engine(const BatchParams& prm, uint32_t 
     };
     auto add = [&](const ka::KeyQuad& x) {
         if constexpr (E == kEngRegisters) {
-            regs.add(x, c.num_groups, c.acc, bad);
+            regs.add(x, c.num_groups, bad, [&](uint32_t key, uint32_t q, uint32_t d, uint32_t t, uint32_t p) {
+                ka::scratch_row(c.acc, key, q, d, t, p);
+            });
         } else if constexpr (E == kEngCube3) {
             ka::table_quad(cube3, x, c.num_groups, c.hot, c.acc, bad);
         } else if constexpr (E == kEngCube) {

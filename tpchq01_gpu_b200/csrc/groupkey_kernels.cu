@@ -25,7 +25,11 @@
 // Accumulators live in scratch memory (per launch, zeroed first): per group 8 x u64 (see
 // q1_keyagg.cuh); a finalize kernel folds them into the caller's int128 table [group][6] with
 // 128-bit atomics (so, like the reference kernels, results accumulate into a caller-zeroed
-// buffer). Launches are capped at 2^31 rows so every u64 scratch sum stays exact.
+// buffer). Launches are capped at 2^31 rows so every u64 scratch sum stays exact. The register
+// placement needs neither: its warps leave records in shared memory and each CTA adds its sums to the
+// caller's table, one 128-bit atomic per (group, aggregate). (Every warp reducing into the scratch
+// made 1,184 same-address atomics per word: 4 groups, 1.0 M rows with the zeroed output 35 us, 8 groups
+// 47 us.)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -98,10 +102,10 @@ struct GroupKeyParams {
     uint32_t num_groups;
     uint32_t table;                 // gk::TableKind
     uint32_t stages;                // ring stages
-    unsigned long long* acc;        // scratch: num_groups x 8 u64, zeroed
+    unsigned long long* acc;        // scratch: num_groups x 8 u64, zeroed (shared and global placements)
+    unsigned long long* out;        // [num_groups][6][lo, hi] (register placement)
     uint32_t* status;
-    const uint32_t* mode;           // when set, the kernel runs only if *mode == mode_want
-    uint32_t mode_want;
+    const uint32_t* mode;           // when set, the path chosen on the device (GroupKeyMode)
 };
 
 // P: placement; NG: plane groups of in_registers_per_thread (4 or 8); kWide: 12 consumer warps
@@ -120,7 +124,17 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
     __shared__ __align__(8) uint64_t full_bar[kMaxStages];
     __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
     __shared__ __align__(8) uint64_t cons_bar;
-    if (prm.mode && *prm.mode != prm.mode_want) return;   // the other path of a chosen pair runs
+    // the register placement's warp records, and the rows its planes do not take (128-bit sums)
+    constexpr uint32_t kRegValues = P == kPlaceInRegistersPerThread ? NG * kNumAggs : 1;
+    __shared__ uint64_t warp_rec[P == kPlaceInRegistersPerThread ? W : 1][kRegValues];
+    __shared__ __align__(16) unsigned long long wide[2 * kRegValues];
+    // a path chosen on the device: this kernel (its table, or the global one) unless partitioned
+    uint32_t table = prm.table;
+    if (P == kPlaceSharedMemPerThread && prm.mode) {
+        const uint32_t mode = *prm.mode;
+        if (mode == kModePartitioned) return;
+        if (mode == kModeGlobalPath) table = kTableNone;
+    }
     const uint32_t S = prm.stages;
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -132,9 +146,9 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
     ka::SlotTable slots;
     const uint32_t hot = G < kWideSlots ? G : kWideSlots;
     if (P == kPlaceSharedMemPerThread) {
-        if (prm.table == kTableCube3) cube3.bind(smem + S * kStage, G);
-        else if (prm.table == kTableCube) cube.bind(smem + S * kStage, G);
-        else slots.bind(smem + S * kStage, hot);
+        if (table == kTableCube3) cube3.bind(smem + S * kStage, G);
+        else if (table == kTableCube) cube.bind(smem + S * kStage, G);
+        else if (table == kTableSlots) slots.bind(smem + S * kStage, hot);
     }
 
     if (threadIdx.x == 0) {
@@ -146,10 +160,12 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
         fence_mbar_init();
     }
     if (P == kPlaceSharedMemPerThread) {
-        if (prm.table == kTableCube3) cube3.zero(threadIdx.x, blockDim.x);
-        else if (prm.table == kTableCube) cube.zero(threadIdx.x, blockDim.x);
-        else slots.zero(threadIdx.x, blockDim.x);
+        if (table == kTableCube3) cube3.zero(threadIdx.x, blockDim.x);
+        else if (table == kTableCube) cube.zero(threadIdx.x, blockDim.x);
+        else if (table == kTableSlots) slots.zero(threadIdx.x, blockDim.x);
     }
+    if (P == kPlaceInRegistersPerThread)
+        for (uint32_t i = threadIdx.x; i < 2 * kRegValues; i += blockDim.x) wide[i] = 0;
     __syncthreads();
 
     if (warp == W) {
@@ -182,33 +198,47 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
         uint32_t tiles_since = 0;
         uint64_t rows_since = 0;
 
+        // every passing row of a quad straight into the global accumulators
+        auto add_global = [&](const ka::KeyQuad& x) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (!((x.PM >> (8 * r)) & 1u)) continue;
+                const uint32_t key = x.k[r];
+                if (key >= G) {
+                    bad = 1u;
+                    continue;
+                }
+                ka::scratch_row(prm.acc, key, (x.Q >> (8 * r)) & 0xFFu, (x.D >> (8 * r)) & 0xFFu,
+                                (x.X >> (8 * r)) & 0xFFu, x.p[r]);
+            }
+        };
         // one decoded quad into the placement's engine
         auto add_quad = [&](const ka::KeyQuad& x) {
             if constexpr (P == kPlaceInRegistersPerThread) {
-                regs.add(x, G, prm.acc, bad);
+                regs.add(x, G, bad, [&](uint32_t key, uint32_t q, uint32_t d, uint32_t t, uint32_t p) {
+                    unsigned long long* v = wide + 2 * (key * kNumAggs);
+                    const uint32_t a = 100u - d;
+                    atomic_add_u128_shared(v + 2 * kAggCount, 1, 0);
+                    atomic_add_u128_shared(v + 2 * kAggQty, q, 0);
+                    atomic_add_u128_shared(v + 2 * kAggBasePrice, p, 0);
+                    atomic_add_u128_shared(v + 2 * kAggDisc, d, 0);
+                    atomic_add_u128_shared(v + 2 * kAggDiscPrice, (uint64_t)a * p, 0);
+                    atomic_add_u128_shared(v + 2 * kAggCharge, (uint64_t)(a * (100u + t)) * p, 0);
+                });
             } else if constexpr (P == kPlaceSharedMemPerThread) {
-                if (prm.table == kTableCube3) ka::table_quad(cube3, x, G, G, prm.acc, bad);
-                else if (prm.table == kTableCube) ka::table_quad(cube, x, G, G, prm.acc, bad);
-                else ka::table_quad(slots, x, G, hot, prm.acc, bad);
+                if (table == kTableCube3) ka::table_quad(cube3, x, G, G, prm.acc, bad);
+                else if (table == kTableCube) ka::table_quad(cube, x, G, G, prm.acc, bad);
+                else if (table == kTableSlots) ka::table_quad(slots, x, G, hot, prm.acc, bad);
+                else add_global(x);
             } else {
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    if (!((x.PM >> (8 * r)) & 1u)) continue;
-                    const uint32_t key = x.k[r];
-                    if (key >= G) {
-                        bad = 1u;
-                        continue;
-                    }
-                    ka::scratch_row(prm.acc, key, (x.Q >> (8 * r)) & 0xFFu, (x.D >> (8 * r)) & 0xFFu,
-                                    (x.X >> (8 * r)) & 0xFFu, x.p[r]);
-                }
+                add_global(x);
             }
         };
         auto table_flush = [&]() {
             cb.sync(lane, prm.status);
-            if (prm.table == kTableCube3) cube3.flush(prm.acc, G, ctid, W * 32);
-            else if (prm.table == kTableCube) cube.flush(prm.acc, G, ctid, W * 32);
-            else slots.flush(prm.acc, ctid, W * 32);
+            if (table == kTableCube3) cube3.flush(prm.acc, G, ctid, W * 32);
+            else if (table == kTableCube) cube.flush(prm.acc, G, ctid, W * 32);
+            else if (table == kTableSlots) slots.flush(prm.acc, ctid, W * 32);
             cb.sync(lane, prm.status);
         };
 
@@ -221,7 +251,14 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
                 break;
             }
             if (P == kPlaceInRegistersPerThread && tiles_since >= ka::kPlaneFlushTiles) {
-                regs.flush(prm.acc, G, lane);
+#pragma unroll
+                for (int i = 0; i < NG; ++i)
+#pragma unroll
+                    for (int a = 0; a < kNumAggs; ++a) {
+                        const uint64_t v = regs.warp_total(i, a) * (a == kAggQty ? 100u : 1u);
+                        if (lane == 0 && (uint32_t)i < G) atomic_add_u128(prm.out + 2 * (i * kNumAggs + a), v, 0);
+                    }
+                regs.zero();
                 tiles_since = 0;
             }
             if (P == kPlaceSharedMemPerThread && rows_since + R > ka::kTableFlushRows) {
@@ -251,13 +288,32 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
             }
         }
         if (bad && prm.status) atomicOr(prm.status, kStatusDomain);
-        if (P == kPlaceInRegistersPerThread) regs.flush(prm.acc, G, lane);
+        if constexpr (P == kPlaceInRegistersPerThread) {
+#pragma unroll
+            for (int i = 0; i < NG; ++i)
+#pragma unroll
+                for (int a = 0; a < kNumAggs; ++a) {
+                    const uint64_t v = regs.warp_total(i, a);
+                    if (lane == 0) warp_rec[warp][i * kNumAggs + a] = v;
+                }
+        }
     }
     __syncthreads();
+    if constexpr (P == kPlaceInRegistersPerThread) {
+        // the CTA's sums (below 2^64 over its warps) and the rows kept out of the planes
+        if (threadIdx.x < G * kNumAggs) {
+            uint64_t lo = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < W; ++w) lo += warp_rec[w][threadIdx.x];
+            unsigned __int128 v = ((unsigned __int128)wide[2 * threadIdx.x + 1] << 64 | wide[2 * threadIdx.x]) + lo;
+            if (threadIdx.x % kNumAggs == kAggQty) v *= 100u;
+            atomic_add_u128(prm.out + 2 * threadIdx.x, (uint64_t)v, (uint64_t)(v >> 64));
+        }
+    }
     if (P == kPlaceSharedMemPerThread) {
-        if (prm.table == kTableCube3) cube3.flush(prm.acc, G, threadIdx.x, blockDim.x);
-        else if (prm.table == kTableCube) cube.flush(prm.acc, G, threadIdx.x, blockDim.x);
-        else slots.flush(prm.acc, threadIdx.x, blockDim.x);
+        if (table == kTableCube3) cube3.flush(prm.acc, G, threadIdx.x, blockDim.x);
+        else if (table == kTableCube) cube.flush(prm.acc, G, threadIdx.x, blockDim.x);
+        else if (table == kTableSlots) slots.flush(prm.acc, threadIdx.x, blockDim.x);
     }
 }
 
@@ -318,11 +374,13 @@ static bool chosen_on_device(int placement, uint32_t num_groups) {
 // + 0.3 p; partitioned 1.7 + 4.3 c + 5.65 (p - c), the hot rows costing more there because skewed
 // keys contend for the same ring counters and slots. The single pass wins when
 // 21.35 c - 5.35 p < -0.5: skewed keys with many passing rows.
-__global__ void __launch_bounds__(256) q1_groupkey_choose(const uint16_t* __restrict__ ship,
-                                                          const uint32_t* __restrict__ keys, uint64_t rows,
-                                                          int32_t cutoff, uint32_t hot, uint32_t allow_part,
-                                                          uint32_t force, uint32_t* mode) {
-    constexpr uint32_t K = 8192, kList = 512;
+// All loads of a thread's eight samples are in flight together: one block of 256 threads taking them
+// one after another was 31 us, two thirds of a launch on 100,000 rows.
+__global__ void __launch_bounds__(1024) q1_groupkey_choose(const uint16_t* __restrict__ ship,
+                                                           const uint32_t* __restrict__ keys, uint64_t rows,
+                                                           int32_t cutoff, uint32_t hot, uint32_t allow_part,
+                                                           uint32_t force, uint32_t* mode) {
+    constexpr uint32_t K = 8192, kPer = K / 1024, kList = 512;
     if (force) {
         if (threadIdx.x == 0) *mode = force;
         return;
@@ -330,27 +388,39 @@ __global__ void __launch_bounds__(256) q1_groupkey_choose(const uint16_t* __rest
     __shared__ uint32_t cnt[4];       // passing, cold, listed, largest key multiplicity
     __shared__ uint32_t list[kList];  // keys of the sampled passing rows
     if (threadIdx.x < 4) cnt[threadIdx.x] = 0;
+    uint32_t day[kPer], key[kPer];
+#pragma unroll
+    for (uint32_t e = 0; e < kPer; ++e) {
+        const uint64_t i = (uint64_t)(e * 1024 + threadIdx.x) * rows / K;
+        day[e] = __ldg(ship + i);
+        key[e] = __ldg(keys + i);
+    }
     __syncthreads();
     uint32_t pass = 0, cold = 0;
-    for (uint32_t j = threadIdx.x; j < K; j += blockDim.x) {
-        const uint64_t i = (uint64_t)j * rows / K;
-        if ((int32_t)ship[i] <= cutoff) {
-            const uint32_t key = keys[i];
-            ++pass;
-            cold += key >= hot ? 1u : 0u;
-            const uint32_t at = atomicAdd(&cnt[2], 1u);
-            if (at < kList) list[at] = key;
-        }
+#pragma unroll
+    for (uint32_t e = 0; e < kPer; ++e) {
+        const bool in = (int32_t)day[e] <= cutoff;
+        pass += in ? 1u : 0u;
+        cold += in && key[e] >= hot ? 1u : 0u;
     }
-    atomicAdd(&cnt[0], pass);
-    atomicAdd(&cnt[1], cold);
+    pass = __reduce_add_sync(0xffffffffu, pass);
+    cold = __reduce_add_sync(0xffffffffu, cold);
+    if ((threadIdx.x & 31u) == 0) {
+        atomicAdd(&cnt[0], pass);
+        atomicAdd(&cnt[1], cold);
+    }
     __syncthreads();
-    const uint32_t P = cnt[0], C = cnt[1], L = cnt[2] < kList ? cnt[2] : kList;
-    const bool few = (uint64_t)P * 50 < K && cnt[2] <= kList;
+    const uint32_t P = cnt[0], C = cnt[1];
+    const bool few = (uint64_t)P * 50 < K;   // fewer than 164: they fit the list
+    static_assert(K / 50 < kList, "the few passing rows' keys fit the list");
     if (few) {
-        for (uint32_t e = threadIdx.x; e < L; e += blockDim.x) {
+#pragma unroll
+        for (uint32_t e = 0; e < kPer; ++e)
+            if ((int32_t)day[e] <= cutoff) list[atomicAdd(&cnt[2], 1u)] = key[e];
+        __syncthreads();
+        for (uint32_t e = threadIdx.x; e < P; e += blockDim.x) {
             uint32_t m = 0;
-            for (uint32_t x = 0; x < L; ++x) m += list[x] == list[e] ? 1u : 0u;
+            for (uint32_t x = 0; x < P; ++x) m += list[x] == list[e] ? 1u : 0u;
             atomicMax(&cnt[3], m);
         }
     }
@@ -370,7 +440,8 @@ __global__ void __launch_bounds__(256) q1_groupkey_choose(const uint16_t* __rest
 cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_t rows, int32_t cutoff_rel,
                             uint32_t num_groups, unsigned long long* scratch, unsigned long long* out,
                             uint32_t* status, int sm_count, int max_blocks, cudaStream_t stream) {
-    cudaError_t e = cudaMemsetAsync(scratch, 0, acc_bytes(num_groups), stream);
+    const bool direct = placement == kPlaceInRegistersPerThread;   // no scratch: straight into `out`
+    cudaError_t e = direct ? cudaSuccess : cudaMemsetAsync(scratch, 0, acc_bytes(num_groups), stream);
     if (e != cudaSuccess) return e;
     uint8_t* workspace = reinterpret_cast<uint8_t*>(scratch) + ((acc_bytes(num_groups) + 255) & ~255ull);
     const bool choose = chosen_on_device(placement, num_groups);
@@ -395,20 +466,14 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
         prm.table = gk::table_kind(placement, num_groups);
         prm.stages = gk::ring_stages(prm.table, num_groups);
         prm.acc = scratch;
+        prm.out = out;
         prm.status = status;
         if (mode) {
-            q1_groupkey_choose<<<1, 256, 0, stream>>>(reinterpret_cast<const uint16_t*>(prm.col[0]),
+            q1_groupkey_choose<<<1, 1024, 0, stream>>>(reinterpret_cast<const uint16_t*>(prm.col[0]),
                                                       reinterpret_cast<const uint32_t*>(prm.col[5]), n, cutoff_rel,
                                                       gk::kWideSlots, part ? 1u : 0u, force, mode);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
             prm.mode = mode;
-            prm.mode_want = kModeSinglePass;
-            // the global path of the choice (returns at once unless chosen)
-            GroupKeyParams g = prm;
-            g.table = gk::kTableNone;
-            g.stages = gk::kMaxStages;
-            g.mode_want = kModeGlobalPath;
-            if ((e = launch_gk<kPlaceGlobal, 4>(g, sm_count, max_blocks, stream)) != cudaSuccess) return e;
         }
         switch (placement) {
             case kPlaceInRegistersPerThread: {
@@ -434,6 +499,7 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
                                      max_blocks, stream);
             if (e != cudaSuccess) return e;
         }
+        if (direct) continue;
         // fold after every 2^31-row launch so the scratch sums stay exact
         q1_groupkey_finalize<<<(num_groups + 255) / 256, 256, 0, stream>>>(scratch, num_groups, out);
         e = cudaGetLastError();

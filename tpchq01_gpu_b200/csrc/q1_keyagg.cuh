@@ -211,17 +211,17 @@ __device__ __forceinline__ KeyQuad load_row(const uint8_t* const col[6], uint64_
 // ---------------------------------------------------------------------------------------------
 template <int NG>
 struct PlaneRegs {
-    // Three price byte planes a group: a passing row with a price >= 2^24 (none in TPC-H data) is
-    // added, exactly, straight into the scratch behind one warp vote, so that eight groups' planes
-    // fit in registers (the fourth plane took 32 more a thread and made the 8-group kernel spill).
+    // Three price byte planes a group: a passing row with a price >= 2^24 (none in TPC-H data) goes
+    // to `slow` behind one warp vote, so that eight groups' planes fit in registers (the fourth plane
+    // took 32 more a thread and made the 8-group kernel spill).
     GroupPlanesT<3> g[NG];
     __device__ __forceinline__ void zero() {
 #pragma unroll
         for (int i = 0; i < NG; ++i) g[i].zero();
     }
-    // Every lane of the warp calls it (warp vote).
-    __device__ __forceinline__ void add(const KeyQuad& kq, uint32_t num_groups, unsigned long long* acc,
-                                        uint32_t& bad) {
+    // Every lane of the warp calls it (warp vote). slow(key, quantity, discount, tax, price): one row.
+    template <class Slow>
+    __device__ __forceinline__ void add(const KeyQuad& kq, uint32_t num_groups, uint32_t& bad, Slow&& slow) {
         uint32_t OH = 0;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -241,14 +241,22 @@ struct PlaneRegs {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 if (((x.P[3] >> (8 * r)) & 0xFFu) && ((x.OH >> (8 * r)) & 0xFFu)) {
-                    scratch_row(acc, kq.k[r], (kq.Q >> (8 * r)) & 0xFFu, (kq.D >> (8 * r)) & 0xFFu,
-                                (kq.X >> (8 * r)) & 0xFFu, kq.p[r]);
+                    slow(kq.k[r], (kq.Q >> (8 * r)) & 0xFFu, (kq.D >> (8 * r)) & 0xFFu, (kq.X >> (8 * r)) & 0xFFu,
+                         kq.p[r]);
                     x.OH &= ~(0xFFu << (8 * r));
                 }
             }
         }
 #pragma unroll
         for (int i = 0; i < NG; ++i) g[i].template add_quad<false>(x.OH, (uint32_t)i, x);
+    }
+    // Warp sum of aggregate a of group i (kAgg*; quantity in whole units): at most 2^15 rows a thread and
+    // prices below 2^24, so price < 2^39, disc_price < 2^46 and charge < 2^54.2 a thread, < 2^60 a warp.
+    __device__ __forceinline__ uint64_t warp_total(int i, int a) const {
+        const uint64_t v = g[i].value(a);
+        return a == kAggCount || a == kAggQty || a == kAggDisc ? warp_sum<27>(v).lo
+               : a == kAggCharge                               ? warp_sum<63>(v).lo
+                                                               : warp_sum<54>(v).lo;
     }
     // Warp sums of the per-thread partials into the scratch; every lane of the warp calls it.
     __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t num_groups, uint32_t lane) {
