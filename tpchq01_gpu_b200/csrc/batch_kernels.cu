@@ -108,7 +108,7 @@ __device__ __forceinline__ bool consume_engine(const BatchParams& prm, uint32_t 
             cb.sync(lane, prm.status);
             if constexpr (E == kEngCube3) cube3.flush(c.acc, c.num_groups, ctid, W * 32);
             else if constexpr (E == kEngCube) cube.flush(c.acc, c.num_groups, ctid, W * 32);
-            else slots.flush(c.acc, ctid, W * 32);
+            else slots.flush(c.acc, c.hot, ctid, W * 32);
             cb.sync(lane, prm.status);
         }
     };

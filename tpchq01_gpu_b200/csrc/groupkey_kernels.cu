@@ -100,7 +100,6 @@ struct GroupKeyParams {
     uint64_t rows;
     int32_t cutoff;                 // cutoff_day - 727563
     uint32_t num_groups;
-    uint32_t table;                 // gk::TableKind
     uint32_t stages;                // ring stages
     unsigned long long* acc;        // scratch: num_groups x 8 u64, zeroed (shared and global placements)
     unsigned long long* out;        // [num_groups][6][lo, hi] (register placement)
@@ -109,8 +108,15 @@ struct GroupKeyParams {
 };
 
 // P: placement; NG: plane groups of in_registers_per_thread (4 or 8); kWide: 12 consumer warps
-// over 3072-row tiles for four groups' planes.
-template <int P, int NG, bool kWide = false>
+// over 3072-row tiles for four groups' planes; kTab: table engine of shared_mem_per_thread. (Each engine
+// its own kernel: one kernel with all of them behind a launch parameter ran 64 groups, 100 M rows, in
+// 255 us instead of 240 once the global path was a fourth alternative.)
+template <uint32_t kTab>
+struct TableOf { using T = ka::SlotTable; };
+template <> struct TableOf<gk::kTableCube> { using T = ka::CubeTableT<true>; };
+template <> struct TableOf<gk::kTableCube3> { using T = ka::Cube3Table; };
+
+template <int P, int NG, bool kWide = false, uint32_t kTab = gk::kTableNone>
 __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32, 1)
     q1_groupkey_kernel(const __grid_constant__ GroupKeyParams prm) {
     using namespace gk;
@@ -128,12 +134,13 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
     constexpr uint32_t kRegValues = P == kPlaceInRegistersPerThread ? NG * kNumAggs : 1;
     __shared__ uint64_t warp_rec[P == kPlaceInRegistersPerThread ? W : 1][kRegValues];
     __shared__ __align__(16) unsigned long long wide[2 * kRegValues];
-    // a path chosen on the device: this kernel (its table, or the global one) unless partitioned
-    uint32_t table = prm.table;
-    if (P == kPlaceSharedMemPerThread && prm.mode) {
+    // a path chosen on the device: this kernel (its table, or no table: the global path) unless partitioned
+    constexpr bool kChosen = kTab == kTableCube || kTab == kTableSlots;
+    bool no_table = false;
+    if (kChosen && prm.mode) {
         const uint32_t mode = *prm.mode;
         if (mode == kModePartitioned) return;
-        if (mode == kModeGlobalPath) table = kTableNone;
+        no_table = mode == kModeGlobalPath;
     }
     const uint32_t S = prm.stages;
 
@@ -141,15 +148,9 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
     const uint64_t num_tiles = prm.rows / R;
     const uint32_t ring = smem_addr(smem);
     const uint32_t G = prm.num_groups;
-    ka::Cube3Table cube3;
-    ka::CubeTableT<true> cube;
-    ka::SlotTable slots;
-    const uint32_t hot = G < kWideSlots ? G : kWideSlots;
-    if (P == kPlaceSharedMemPerThread) {
-        if (table == kTableCube3) cube3.bind(smem + S * kStage, G);
-        else if (table == kTableCube) cube.bind(smem + S * kStage, G);
-        else if (table == kTableSlots) slots.bind(smem + S * kStage, hot);
-    }
+    const uint32_t hot = kTab == kTableSlots && G > kWideSlots ? kWideSlots : G;   // keys the table takes
+    typename TableOf<kTab>::T tab;
+    if (kTab != kTableNone) tab.bind(smem + S * kStage, hot);
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < S; ++s) {
@@ -159,11 +160,7 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
         mbar_init(smem_addr(&cons_bar), W);
         fence_mbar_init();
     }
-    if (P == kPlaceSharedMemPerThread) {
-        if (table == kTableCube3) cube3.zero(threadIdx.x, blockDim.x);
-        else if (table == kTableCube) cube.zero(threadIdx.x, blockDim.x);
-        else if (table == kTableSlots) slots.zero(threadIdx.x, blockDim.x);
-    }
+    if (kTab != kTableNone && !no_table) tab.zero(threadIdx.x, blockDim.x);
     if (P == kPlaceInRegistersPerThread)
         for (uint32_t i = threadIdx.x; i < 2 * kRegValues; i += blockDim.x) wide[i] = 0;
     __syncthreads();
@@ -225,68 +222,68 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
                     atomic_add_u128_shared(v + 2 * kAggDiscPrice, (uint64_t)a * p, 0);
                     atomic_add_u128_shared(v + 2 * kAggCharge, (uint64_t)(a * (100u + t)) * p, 0);
                 });
-            } else if constexpr (P == kPlaceSharedMemPerThread) {
-                if (table == kTableCube3) ka::table_quad(cube3, x, G, G, prm.acc, bad);
-                else if (table == kTableCube) ka::table_quad(cube, x, G, G, prm.acc, bad);
-                else if (table == kTableSlots) ka::table_quad(slots, x, G, hot, prm.acc, bad);
-                else add_global(x);
+            } else if constexpr (kTab != kTableNone) {
+                ka::table_quad(tab, x, G, hot, prm.acc, bad);
             } else {
                 add_global(x);
             }
         };
         auto table_flush = [&]() {
             cb.sync(lane, prm.status);
-            if (table == kTableCube3) cube3.flush(prm.acc, G, ctid, W * 32);
-            else if (table == kTableCube) cube.flush(prm.acc, G, ctid, W * 32);
-            else if (table == kTableSlots) slots.flush(prm.acc, ctid, W * 32);
+            tab.flush(prm.acc, hot, ctid, W * 32);
             cb.sync(lane, prm.status);
         };
 
-        bool ok = true;
-        uint32_t s = 0, ph = 0;   // stage and phase of the current tile
-        for (uint64_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-            const bool landed = mbar_wait(smem_addr(&full_bar[s]), ph, prm.status);
-            if (!__all_sync(0xffffffffu, landed)) {
-                ok = false;
-                break;
-            }
-            if (P == kPlaceInRegistersPerThread && tiles_since >= ka::kPlaneFlushTiles) {
+        // all of this CTA's rows through `add`
+        auto add_rows = [&](auto&& add, bool flushes) {
+            bool ok = true;
+            uint32_t s = 0, ph = 0;   // stage and phase of the current tile
+            for (uint64_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+                const bool landed = mbar_wait(smem_addr(&full_bar[s]), ph, prm.status);
+                if (!__all_sync(0xffffffffu, landed)) {
+                    ok = false;
+                    break;
+                }
+                if (P == kPlaceInRegistersPerThread && tiles_since >= ka::kPlaneFlushTiles) {
 #pragma unroll
-                for (int i = 0; i < NG; ++i)
+                    for (int i = 0; i < NG; ++i)
 #pragma unroll
-                    for (int a = 0; a < kNumAggs; ++a) {
-                        const uint64_t v = regs.warp_total(i, a) * (a == kAggQty ? 100u : 1u);
-                        if (lane == 0 && (uint32_t)i < G) atomic_add_u128(prm.out + 2 * (i * kNumAggs + a), v, 0);
-                    }
-                regs.zero();
-                tiles_since = 0;
-            }
-            if (P == kPlaceSharedMemPerThread && rows_since + R > ka::kTableFlushRows) {
-                table_flush();
-                rows_since = 0;
-            }
-            ++tiles_since;
-            rows_since += R;
-            const uint32_t base = ring + s * kStage;
+                        for (int a = 0; a < kNumAggs; ++a) {
+                            const uint64_t v = regs.warp_total(i, a) * (a == kAggQty ? 100u : 1u);
+                            if (lane == 0 && (uint32_t)i < G) atomic_add_u128(prm.out + 2 * (i * kNumAggs + a), v, 0);
+                        }
+                    regs.zero();
+                    tiles_since = 0;
+                }
+                if (flushes && rows_since + R > ka::kTableFlushRows) {
+                    table_flush();
+                    rows_since = 0;
+                }
+                ++tiles_since;
+                rows_since += R;
+                const uint32_t base = ring + s * kStage;
 #pragma unroll
-            for (uint32_t it = 0; it < kSteps / (W * 32); ++it)
-                add_quad(ka::load_quad<R>(base, ctid + it * (W * 32), prm.cutoff, bad));
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_addr(&empty_bar[s]));
-            if (++s == S) {
-                s = 0;
-                ph ^= 1u;
+                for (uint32_t it = 0; it < kSteps / (W * 32); ++it)
+                    add(ka::load_quad<R>(base, ctid + it * (W * 32), prm.cutoff, bad));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_addr(&empty_bar[s]));
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
-        }
-        // the rows after the last full tile, by one CTA straight from global memory
-        if (ok && blockIdx.x == (uint32_t)(num_tiles % gridDim.x) && num_tiles * R < prm.rows) {
-            if (P == kPlaceSharedMemPerThread && rows_since + R > ka::kTableFlushRows) table_flush();
-            // every lane runs every round (the table engines vote across the warp)
-            for (uint64_t i0 = num_tiles * R; i0 < prm.rows; i0 += W * 32) {
-                const uint64_t i = i0 + ctid;
-                add_quad(i < prm.rows ? ka::load_row(prm.col, i, prm.cutoff, bad) : ka::empty_quad());
+            // the rows after the last full tile, by one CTA straight from global memory
+            if (ok && blockIdx.x == (uint32_t)(num_tiles % gridDim.x) && num_tiles * R < prm.rows) {
+                if (flushes && rows_since + R > ka::kTableFlushRows) table_flush();
+                // every lane runs every round (the table engines vote across the warp)
+                for (uint64_t i0 = num_tiles * R; i0 < prm.rows; i0 += W * 32) {
+                    const uint64_t i = i0 + ctid;
+                    add(i < prm.rows ? ka::load_row(prm.col, i, prm.cutoff, bad) : ka::empty_quad());
+                }
             }
-        }
+        };
+        if (kChosen && no_table) add_rows(add_global, false);
+        else add_rows(add_quad, kTab != kTableNone);
         if (bad && prm.status) atomicOr(prm.status, kStatusDomain);
         if constexpr (P == kPlaceInRegistersPerThread) {
 #pragma unroll
@@ -310,11 +307,10 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
             atomic_add_u128(prm.out + 2 * threadIdx.x, (uint64_t)v, (uint64_t)(v >> 64));
         }
     }
-    if (P == kPlaceSharedMemPerThread) {
-        if (table == kTableCube3) cube3.flush(prm.acc, G, threadIdx.x, blockDim.x);
-        else if (table == kTableCube) cube.flush(prm.acc, G, threadIdx.x, blockDim.x);
-        else if (table == kTableSlots) slots.flush(prm.acc, threadIdx.x, blockDim.x);
-    }
+    // CTAs start at different groups, so that they do not all add to the same words at once (6.0 M rows,
+    // 4096 groups 91 -> 81 us, 1000 groups 62.5 -> 59 us)
+    if (kTab != kTableNone && !no_table)
+        tab.flush(prm.acc, hot, threadIdx.x, blockDim.x, (uint32_t)((uint64_t)blockIdx.x * hot / gridDim.x));
 }
 
 // acc (num_groups x 8 u64) -> out[group][6] int128 (+=), quantity scaled to hundredths.
@@ -336,12 +332,12 @@ __global__ void __launch_bounds__(256) q1_groupkey_finalize(const unsigned long 
     atomic_add_u128(o + 2 * kAggCharge, (uint64_t)ch, (uint64_t)(ch >> 64));
 }
 
-template <int P, int NG, bool kWide = false>
+template <int P, int NG, bool kWide = false, uint32_t kTab = gk::kTableNone>
 static cudaError_t launch_gk(const GroupKeyParams& prm, int sm_count, int max_blocks, cudaStream_t st) {
     using namespace gk;
     constexpr uint32_t R = tile_rows<P, NG, kWide>();
-    const uint32_t dyn = prm.stages * stage_bytes<P, NG, kWide>() + table_bytes(prm.table, prm.num_groups);
-    cudaError_t e = cudaFuncSetAttribute(q1_groupkey_kernel<P, NG, kWide>,
+    const uint32_t dyn = prm.stages * stage_bytes<P, NG, kWide>() + table_bytes(kTab, prm.num_groups);
+    cudaError_t e = cudaFuncSetAttribute(q1_groupkey_kernel<P, NG, kWide, kTab>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
     const uint64_t tiles = prm.rows / R;
@@ -349,7 +345,7 @@ static cudaError_t launch_gk(const GroupKeyParams& prm, int sm_count, int max_bl
     uint64_t cap = (uint64_t)sm_count;
     if (max_blocks > 0 && (uint64_t)max_blocks < cap) cap = (uint64_t)max_blocks;
     if (blocks > cap) blocks = cap;
-    q1_groupkey_kernel<P, NG, kWide><<<(unsigned)blocks, (consumer_warps<P, NG, kWide>() + 1) * 32, dyn, st>>>(prm);
+    q1_groupkey_kernel<P, NG, kWide, kTab><<<(unsigned)blocks, (consumer_warps<P, NG, kWide>() + 1) * 32, dyn, st>>>(prm);
     return cudaGetLastError();
 }
 
@@ -463,8 +459,8 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
         prm.rows = n;
         prm.cutoff = cutoff_rel;
         prm.num_groups = num_groups;
-        prm.table = gk::table_kind(placement, num_groups);
-        prm.stages = gk::ring_stages(prm.table, num_groups);
+        const uint32_t table = gk::table_kind(placement, num_groups);
+        prm.stages = gk::ring_stages(table, num_groups);
         prm.acc = scratch;
         prm.out = out;
         prm.status = status;
@@ -489,7 +485,13 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
                                    : launch_gk<kPlaceInRegistersPerThread, 4>(prm, sm_count, max_blocks, stream);
                 break;
             }
-            case kPlaceSharedMemPerThread: e = launch_gk<kPlaceSharedMemPerThread, 4>(prm, sm_count, max_blocks, stream); break;
+            case kPlaceSharedMemPerThread:
+                e = table == gk::kTableCube3
+                        ? launch_gk<kPlaceSharedMemPerThread, 4, false, gk::kTableCube3>(prm, sm_count, max_blocks, stream)
+                    : table == gk::kTableCube
+                        ? launch_gk<kPlaceSharedMemPerThread, 4, false, gk::kTableCube>(prm, sm_count, max_blocks, stream)
+                        : launch_gk<kPlaceSharedMemPerThread, 4, false, gk::kTableSlots>(prm, sm_count, max_blocks, stream);
+                break;
             case kPlaceGlobal: e = launch_gk<kPlaceGlobal, 4>(prm, sm_count, max_blocks, stream); break;
             default: return cudaErrorInvalidValue;
         }

@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(gp::kP2Warps * 32, 1) q1_gk_partagg_kernel(con
         if (s0.p != cur || rows_since + s0.n * kChunk > ka::kTableFlushRows) {
             if (cur != kNoPart) {
                 __syncthreads();
-                slots.flush(prm.acc + 8ull * cur * kWidth, tid, T);
+                slots.flush(prm.acc + 8ull * cur * kWidth, kWidth, tid, T);
                 __syncthreads();
             }
             cur = s0.p;
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(gp::kP2Warps * 32, 1) q1_gk_partagg_kernel(con
         }
     }
     __syncthreads();
-    if (cur != kNoPart) slots.flush(prm.acc + 8ull * cur * kWidth, tid, T);
+    if (cur != kNoPart) slots.flush(prm.acc + 8ull * cur * kWidth, kWidth, tid, T);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -357,9 +357,12 @@ struct CubeTableT {
             }
         }
     }
-    // Cells -> per-group sums -> scratch; the caller synchronises the consumers around it.
-    __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t num_groups, uint32_t tid, uint32_t nthreads) {
-        for (uint32_t g = tid; g < num_groups; g += nthreads) {
+    // Cells -> per-group sums -> scratch, from group `first` on (and round to it); the caller
+    // synchronises the consumers around it.
+    __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t num_groups, uint32_t tid, uint32_t nthreads,
+                                          uint32_t first = 0) {
+        for (uint32_t i = tid; i < num_groups; i += nthreads) {
+            const uint32_t g = i + first < num_groups ? i + first : i + first - num_groups;
             uint64_t q = 0, pw = 0, aw = 0, tw = 0;
             if constexpr (kSharedCarries) {
                 q = gw[g], pw = gw[groups + g], aw = gw[2 * groups + g], tw = gw[3 * groups + g];
@@ -440,9 +443,12 @@ struct Cube3Table {
                 if (op[r] > ~p[r]) atomicAdd(w + 3 * cells + c[r], 1u);
         }
     }
-    // Cells -> per-group sums -> scratch; the caller synchronises the consumers around it.
-    __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t num_groups, uint32_t tid, uint32_t nthreads) {
-        for (uint32_t g = tid; g < num_groups; g += nthreads) {
+    // Cells -> per-group sums -> scratch, from group `first` on (and round to it); the caller
+    // synchronises the consumers around it.
+    __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t num_groups, uint32_t tid, uint32_t nthreads,
+                                          uint32_t first = 0) {
+        for (uint32_t i = tid; i < num_groups; i += nthreads) {
+            const uint32_t g = i + first < num_groups ? i + first : i + first - num_groups;
             uint64_t cnt = 0, q = 0, dsum = 0, P = 0;
             unsigned __int128 DP = 0, CH = 0;
             for (uint32_t d = 0; d < kCubeDisc; ++d) {
@@ -531,9 +537,11 @@ struct SlotTable {
             }
         }
     }
-    __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t tid, uint32_t nthreads) {
+    __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t, uint32_t tid, uint32_t nthreads,
+                                          uint32_t first = 0) {
         const uint32_t S = slots;
-        for (uint32_t s = tid; s < S; s += nthreads) {
+        for (uint32_t i = tid; i < S; i += nthreads) {
+            const uint32_t s = i + first < S ? i + first : i + first - S;
             const uint64_t cnt = w[s];
             if (cnt) {
                 const uint64_t P = ((uint64_t)w[4 * S + s] << 32) | w[3 * S + s];
