@@ -207,3 +207,25 @@ def test_zipf_cdf_matches_restatement():
     ref = gen_np.zipf_cdf(65536)
     assert cdf[-1] == 0xFFFFFFFF and np.all(np.diff(cdf.astype(np.int64)) >= 0)
     assert np.max(np.abs(cdf.astype(np.int64) - ref.astype(np.int64))) <= 1
+
+
+@pytest.mark.parametrize("num_groups", [4, 8, 64, 300, 1000, 2048, 4096])
+@pytest.mark.parametrize("blocks", [0, 1, 2])
+def test_groupkey_tile_and_team_edges(table, num_groups, blocks):
+    """Row counts around the tiles of the table engines' teams (1024, 1536 and 3072 rows) and of the
+    register planes (2048, 3072), down to one row, in the default grid and in one and two CTAs, with rows
+    outside the tables' fast domain; also with so few passing rows that the path choice above 256
+    groups takes the global path."""
+    comp, _, _ = table
+    wide = widen(comp, 91, 0.02)
+    c, keep = device_cols(wide)
+    keys, _ = keys_for(num_groups, "uniform")
+    placement = "in_registers_per_thread" if num_groups <= 8 else "shared_mem_per_thread"
+    for rows in [1, 1023, 1025, 1537, 2049, 3071, 3073, 3 * 1024 + 1, 2 * 3072 + 1023, 6 * 3072 + 5, 100_003]:
+        for cutoff in [729999, 727600]:
+            part = {k: v[:rows] for k, v in wide.items() if isinstance(v, np.ndarray) and k in
+                    ["shipdate", "discount", "extendedprice", "tax", "quantity"]}
+            got = run_gpu(c, keys[:rows], num_groups, placement, cutoff, blocks)
+            want, flag = O.q1_groupkey(part, keys[:rows], num_groups, cutoff)
+            assert flag == 0
+            assert np.array_equal(got, want), (rows, cutoff)

@@ -47,24 +47,33 @@ using namespace ptx;
 
 namespace gk {
 
-constexpr uint32_t kMaxStages = 4;    // ring stages (3 when the table needs the room)
+constexpr uint32_t kMaxStages = 10;   // ring stages
 constexpr uint32_t kWideSlots = 4096; // slot-table keys of the single-pass kernel
 constexpr uint32_t kChooseAbove = 256; // the shared placement's path is chosen on the device above
 constexpr uint32_t kMaxDynSmem = 227 * 1024;
-// Consumer warps: 16 for the shared-table and global placements, whose atomics need many warps in
-// flight to hide their latency; 8 for the register planes, or 12 for four groups' planes on a large
-// table (kWide: their 127 registers a thread fit the 128 that 13 warps leave, and a third warp per
-// scheduler hides more of the planes' issue latency: 600 M rows 1.49 -> 1.24 ms, 80% -> 96% of HBM).
+// Consumer warps. Register planes: 8, or 12 for four groups' planes on a large table (kWide: their 110
+// registers a thread fit the 128 that 13 warps leave, and a third warp per scheduler hides more of the
+// planes' issue latency: 600 M rows 1.49 -> 1.24 ms). Global placement: 16. Shared tables: 24, whose
+// atomics need many warps in flight to hide their latency (64 groups, 100 M rows: 237 us with 16, 199
+// with 24).
 template <int P, int NG, bool kWide>
 __host__ __device__ constexpr uint32_t consumer_warps() {
-    return P == kPlaceInRegistersPerThread ? ((NG <= 4 && kWide) ? 12u : 8u) : 16u;
+    return P == kPlaceInRegistersPerThread ? ((NG <= 4 && kWide) ? 12u : 8u)
+                                           : (P == kPlaceSharedMemPerThread ? 24u : 16u);
 }
-// Rows per tile: 2048, or 3072 with 12 warps, so that every consumer thread takes two quads of a
-// tile (at most 8 rows, which the planes' flush cadence assumes).
-template <int P, int NG, bool kWide>
-__host__ __device__ constexpr uint32_t tile_rows() { return consumer_warps<P, NG, kWide>() == 12u ? 3072u : ka::R; }
-template <int P, int NG, bool kWide>
-__host__ __device__ constexpr uint32_t stage_bytes() { return ka::TileLayout<tile_rows<P, NG, kWide>()>::kStageBytes; }
+// Rows per tile: two quads of a tile for every consumer thread of the register planes (at most 8
+// rows, which their flush cadence assumes), one for the others. The shared tables' consumers may
+// form teams that take the tiles in turn, each with a producer warp of its own (one producer feeding
+// three teams' small tiles was the bound: 283 us): the tiles are smaller, so that the ring beside a large
+// table still holds several.
+template <int P, int NG, bool kWide, uint32_t kTeams>
+__host__ __device__ constexpr uint32_t tile_rows() {
+    return consumer_warps<P, NG, kWide>() / kTeams * 128u * (P == kPlaceInRegistersPerThread ? 2u : 1u);
+}
+template <int P, int NG, bool kWide, uint32_t kTeams>
+__host__ __device__ constexpr uint32_t stage_bytes() {
+    return ka::TileLayout<tile_rows<P, NG, kWide, kTeams>()>::kStageBytes;
+}
 
 // Table engine of the shared_mem_per_thread placement.
 enum TableKind : uint32_t { kTableNone = 0, kTableCube = 1, kTableSlots = 2, kTableCube3 = 3 };
@@ -83,15 +92,26 @@ __host__ __device__ constexpr uint32_t table_bytes(uint32_t kind, uint32_t num_g
                                                                                                  : kWideSlots)
                                                                             : 0u));
 }
-// (tables live only beside 2048-row stages; the register planes' 3072-row stages take 4 x 39 KB)
-__host__ __device__ constexpr uint32_t ring_stages(uint32_t kind, uint32_t num_groups) {
-    return kMaxStages * ka::kStageBytes + table_bytes(kind, num_groups) <= kMaxDynSmem ? kMaxStages : kMaxStages - 1;
+// As many stages as fit beside the table (static shared memory: less than 4 KB), at most 4 of those
+// of 2048 rows and more, the same number for each team.
+template <int P, int NG, bool kWide, uint32_t kTeams>
+__host__ constexpr uint32_t ring_stages(uint32_t kind, uint32_t num_groups) {
+    const uint32_t fit = (kMaxDynSmem - 4096 - table_bytes(kind, num_groups)) / stage_bytes<P, NG, kWide, kTeams>();
+    const uint32_t most = kTeams == 1 ? 4u : kMaxStages;
+    return (fit < most ? fit : most) / kTeams * kTeams;
 }
-static_assert(kMaxStages * ka::TileLayout<3072>::kStageBytes + 512 <= kMaxDynSmem, "register-plane ring");
-// the largest tables fit beside a 3-stage ring, with room left for the static shared memory
-static_assert((kMaxStages - 1) * ka::kStageBytes + ka::cube_bytes(ka::kCubeMaxGroups) + 512 <= kMaxDynSmem,
-              "1024-group cells");
-static_assert((kMaxStages - 1) * ka::kStageBytes + ka::slot_bytes(kWideSlots) + 512 <= kMaxDynSmem, "slot table");
+// Teams of the shared tables. One while three stages of its 3072-row tiles fit beside the table, then
+// three (100 M rows, 600 groups: 238 us with one team, 244 with two or three; 1000 groups: 303, 280 and
+// 273; 2500 groups: 326, 337, 337; 4096 groups, 60 M rows: 279, 270, 270). The (group, discount, tax)
+// cells have two throughout (64 groups: 203, 199, 199).
+constexpr uint32_t kSmallTeams = 3;
+static uint32_t table_teams(uint32_t kind, uint32_t num_groups) {
+    if (kind == kTableCube3) return 2;
+    return ring_stages<kPlaceSharedMemPerThread, 4, false, 1>(kind, num_groups) >= 3 ? 1 : kSmallTeams;
+}
+static_assert(ring_stages<kPlaceSharedMemPerThread, 4, false, kSmallTeams>(kTableCube, ka::kCubeMaxGroups) >= kSmallTeams &&
+                  ring_stages<kPlaceSharedMemPerThread, 4, false, kSmallTeams>(kTableSlots, kWideSlots) >= kSmallTeams,
+              "a stage for every team beside the largest tables");
 
 }  // namespace gk
 
@@ -116,16 +136,17 @@ struct TableOf { using T = ka::SlotTable; };
 template <> struct TableOf<gk::kTableCube> { using T = ka::CubeTableT<true>; };
 template <> struct TableOf<gk::kTableCube3> { using T = ka::Cube3Table; };
 
-template <int P, int NG, bool kWide = false, uint32_t kTab = gk::kTableNone>
-__global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32, 1)
+template <int P, int NG, bool kWide = false, uint32_t kTab = gk::kTableNone, uint32_t kTeams = 1>
+__global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + kTeams) * 32, 1)
     q1_groupkey_kernel(const __grid_constant__ GroupKeyParams prm) {
     using namespace gk;
     constexpr uint32_t W = consumer_warps<P, NG, kWide>();
-    constexpr uint32_t R = tile_rows<P, NG, kWide>();
-    constexpr uint32_t kStage = stage_bytes<P, NG, kWide>();
+    constexpr uint32_t R = tile_rows<P, NG, kWide, kTeams>();
+    constexpr uint32_t kStage = stage_bytes<P, NG, kWide, kTeams>();
     constexpr uint32_t kSteps = R / 4;   // 4 rows per consumer step
-    static_assert(kSteps % (W * 32) == 0 && kSteps / (W * 32) * 4 <= 8, "two quads per consumer thread at most");
-    static_assert(P == kPlaceInRegistersPerThread || R == ka::R, "tables beside 2048-row stages only");
+    constexpr uint32_t WT = W / kTeams;   // warps of a team
+    static_assert(W % kTeams == 0 && kSteps % (WT * 32) == 0 && kSteps / (WT * 32) * 4 <= 8,
+                  "two quads per consumer thread at most");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full_bar[kMaxStages];
     __shared__ __align__(8) uint64_t empty_bar[kMaxStages];
@@ -155,7 +176,7 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < S; ++s) {
             mbar_init(smem_addr(&full_bar[s]), 1);
-            mbar_init(smem_addr(&empty_bar[s]), W);
+            mbar_init(smem_addr(&empty_bar[s]), WT);
         }
         mbar_init(smem_addr(&cons_bar), W);
         fence_mbar_init();
@@ -165,12 +186,15 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
         for (uint32_t i = threadIdx.x; i < 2 * kRegValues; i += blockDim.x) wide[i] = 0;
     __syncthreads();
 
-    if (warp == W) {
+    if (warp >= W) {
+        // a producer warp per team: its tiles, into every kTeams-th stage
         if (lane == 0) {
             const uint64_t pol = policy_evict_first();
-            // stage s and phase ph of tile k, stepped rather than divided (S is a launch parameter)
-            uint32_t k = 0, s = 0, ph = 0;
-            for (uint64_t t = blockIdx.x; t < num_tiles; t += gridDim.x, ++k) {
+            // stage s and phase ph of the tile, stepped rather than divided (S is a launch parameter)
+            uint32_t s = warp - W, ph = 0;
+            const uint64_t step = (uint64_t)kTeams * gridDim.x;
+            uint64_t t = blockIdx.x + (uint64_t)(warp - W) * gridDim.x;
+            for (; t < num_tiles; t += step) {
                 if (!mbar_wait(smem_addr(&empty_bar[s]), ph ^ 1u, prm.status)) break;
                 const uint32_t fb = smem_addr(&full_bar[s]);
                 mbar_arrive_expect_tx(fb, kStage);
@@ -179,12 +203,21 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
                     bulk_g2s(ring + s * kStage + ka::TileLayout<R>::col_off(c),
                              prm.col[c] + t * (uint64_t)ka::TileLayout<R>::col_bytes(c),
                              ka::TileLayout<R>::col_bytes(c), fb, pol);
-                if (++s == S) {
-                    s = 0;
+                s += kTeams;
+                if (s >= S) {
+                    s -= S;
                     ph ^= 1u;
                 }
             }
-            for (uint32_t i = (k > S ? k - S : 0u); i < k; ++i) mbar_wait(smem_addr(&full_bar[i % S]), (i / S) & 1u, prm.status);
+            // Never leave with copies in flight: wait for the last tiles issued to land.
+            for (uint32_t i = 0; i < S; i += kTeams) {
+                mbar_wait(smem_addr(&full_bar[s]), ph ^ 1u, prm.status);
+                s += kTeams;
+                if (s >= S) {
+                    s -= S;
+                    ph ^= 1u;
+                }
+            }
         }
     } else {
         const uint32_t ctid = threadIdx.x;
@@ -237,13 +270,10 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
         // all of this CTA's rows through `add`
         auto add_rows = [&](auto&& add, bool flushes) {
             bool ok = true;
-            uint32_t s = 0, ph = 0;   // stage and phase of the current tile
-            for (uint64_t t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-                const bool landed = mbar_wait(smem_addr(&full_bar[s]), ph, prm.status);
-                if (!__all_sync(0xffffffffu, landed)) {
-                    ok = false;
-                    break;
-                }
+            uint32_t s = warp / WT, ph = 0;   // stage and phase of the team's tile
+            // a round is a tile for every team (the last one's may be past the end: the flushes below
+            // are barriers of all consumer warps)
+            for (uint64_t t0 = blockIdx.x; t0 < num_tiles; t0 += (uint64_t)kTeams * gridDim.x) {
                 if (P == kPlaceInRegistersPerThread && tiles_since >= ka::kPlaneFlushTiles) {
 #pragma unroll
                     for (int i = 0; i < NG; ++i)
@@ -255,26 +285,33 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + 1) * 32,
                     regs.zero();
                     tiles_since = 0;
                 }
-                if (flushes && rows_since + R > ka::kTableFlushRows) {
+                if (flushes && rows_since + kTeams * R > ka::kTableFlushRows) {
                     table_flush();
                     rows_since = 0;
                 }
                 ++tiles_since;
-                rows_since += R;
+                rows_since += kTeams * R;
+                if (t0 + (uint64_t)(warp / WT) * gridDim.x >= num_tiles) continue;
+                const bool landed = mbar_wait(smem_addr(&full_bar[s]), ph, prm.status);
+                if (!__all_sync(0xffffffffu, landed)) {
+                    ok = false;
+                    break;
+                }
                 const uint32_t base = ring + s * kStage;
 #pragma unroll
-                for (uint32_t it = 0; it < kSteps / (W * 32); ++it)
-                    add(ka::load_quad<R>(base, ctid + it * (W * 32), prm.cutoff, bad));
+                for (uint32_t it = 0; it < kSteps / (WT * 32); ++it)
+                    add(ka::load_quad<R>(base, ctid % (WT * 32) + it * (WT * 32), prm.cutoff, bad));
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_addr(&empty_bar[s]));
-                if (++s == S) {
-                    s = 0;
+                s += kTeams;
+                if (s >= S) {
+                    s -= S;
                     ph ^= 1u;
                 }
             }
             // the rows after the last full tile, by one CTA straight from global memory
             if (ok && blockIdx.x == (uint32_t)(num_tiles % gridDim.x) && num_tiles * R < prm.rows) {
-                if (flushes && rows_since + R > ka::kTableFlushRows) table_flush();
+                if (flushes && rows_since + kTeams * R > ka::kTableFlushRows) table_flush();
                 // every lane runs every round (the table engines vote across the warp)
                 for (uint64_t i0 = num_tiles * R; i0 < prm.rows; i0 += W * 32) {
                     const uint64_t i = i0 + ctid;
@@ -332,12 +369,13 @@ __global__ void __launch_bounds__(256) q1_groupkey_finalize(const unsigned long 
     atomic_add_u128(o + 2 * kAggCharge, (uint64_t)ch, (uint64_t)(ch >> 64));
 }
 
-template <int P, int NG, bool kWide = false, uint32_t kTab = gk::kTableNone>
-static cudaError_t launch_gk(const GroupKeyParams& prm, int sm_count, int max_blocks, cudaStream_t st) {
+template <int P, int NG, bool kWide = false, uint32_t kTab = gk::kTableNone, uint32_t kTeams = 1>
+static cudaError_t launch_gk(GroupKeyParams prm, int sm_count, int max_blocks, cudaStream_t st) {
     using namespace gk;
-    constexpr uint32_t R = tile_rows<P, NG, kWide>();
-    const uint32_t dyn = prm.stages * stage_bytes<P, NG, kWide>() + table_bytes(kTab, prm.num_groups);
-    cudaError_t e = cudaFuncSetAttribute(q1_groupkey_kernel<P, NG, kWide, kTab>,
+    constexpr uint32_t R = tile_rows<P, NG, kWide, kTeams>();
+    prm.stages = ring_stages<P, NG, kWide, kTeams>(kTab, prm.num_groups);
+    const uint32_t dyn = prm.stages * stage_bytes<P, NG, kWide, kTeams>() + table_bytes(kTab, prm.num_groups);
+    cudaError_t e = cudaFuncSetAttribute(q1_groupkey_kernel<P, NG, kWide, kTab, kTeams>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
     const uint64_t tiles = prm.rows / R;
@@ -345,8 +383,20 @@ static cudaError_t launch_gk(const GroupKeyParams& prm, int sm_count, int max_bl
     uint64_t cap = (uint64_t)sm_count;
     if (max_blocks > 0 && (uint64_t)max_blocks < cap) cap = (uint64_t)max_blocks;
     if (blocks > cap) blocks = cap;
-    q1_groupkey_kernel<P, NG, kWide, kTab><<<(unsigned)blocks, (consumer_warps<P, NG, kWide>() + 1) * 32, dyn, st>>>(prm);
+    q1_groupkey_kernel<P, NG, kWide, kTab, kTeams><<<(unsigned)blocks, (consumer_warps<P, NG, kWide>() + kTeams) * 32, dyn, st>>>(prm);
     return cudaGetLastError();
+}
+
+static cudaError_t launch_table(uint32_t table, uint32_t teams, const GroupKeyParams& prm, int sm_count, int max_blocks,
+                                cudaStream_t st) {
+    constexpr int P = kPlaceSharedMemPerThread;
+    using namespace gk;
+    if (table == kTableCube3) return launch_gk<P, 4, false, kTableCube3, 2>(prm, sm_count, max_blocks, st);
+    if (table == kTableCube)
+        return teams == 1 ? launch_gk<P, 4, false, kTableCube, 1>(prm, sm_count, max_blocks, st)
+                          : launch_gk<P, 4, false, kTableCube, kSmallTeams>(prm, sm_count, max_blocks, st);
+    return teams == 1 ? launch_gk<P, 4, false, kTableSlots, 1>(prm, sm_count, max_blocks, st)
+                      : launch_gk<P, 4, false, kTableSlots, kSmallTeams>(prm, sm_count, max_blocks, st);
 }
 
 static uint64_t acc_bytes(uint32_t num_groups) { return 64ull * num_groups; }
@@ -460,7 +510,6 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
         prm.cutoff = cutoff_rel;
         prm.num_groups = num_groups;
         const uint32_t table = gk::table_kind(placement, num_groups);
-        prm.stages = gk::ring_stages(table, num_groups);
         prm.acc = scratch;
         prm.out = out;
         prm.status = status;
@@ -479,18 +528,14 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
                 // 10^4..5*10^7 rows: 10.72 ms with 2048-row tiles throughout, 11.56 ms with the wide
                 // ones from 2 tiles per CTA, 10.78 ms from 32).
                 const uint64_t grid = (max_blocks > 0 && max_blocks < sm_count) ? (uint64_t)max_blocks : (uint64_t)sm_count;
-                const bool wide = n >= 32 * grid * gk::tile_rows<kPlaceInRegistersPerThread, 4, true>();
+                const bool wide = n >= 32 * grid * gk::tile_rows<kPlaceInRegistersPerThread, 4, true, 1>();
                 e = num_groups > 4 ? launch_gk<kPlaceInRegistersPerThread, 8>(prm, sm_count, max_blocks, stream)
                     : wide         ? launch_gk<kPlaceInRegistersPerThread, 4, true>(prm, sm_count, max_blocks, stream)
                                    : launch_gk<kPlaceInRegistersPerThread, 4>(prm, sm_count, max_blocks, stream);
                 break;
             }
             case kPlaceSharedMemPerThread:
-                e = table == gk::kTableCube3
-                        ? launch_gk<kPlaceSharedMemPerThread, 4, false, gk::kTableCube3>(prm, sm_count, max_blocks, stream)
-                    : table == gk::kTableCube
-                        ? launch_gk<kPlaceSharedMemPerThread, 4, false, gk::kTableCube>(prm, sm_count, max_blocks, stream)
-                        : launch_gk<kPlaceSharedMemPerThread, 4, false, gk::kTableSlots>(prm, sm_count, max_blocks, stream);
+                e = launch_table(table, gk::table_teams(table, num_groups), prm, sm_count, max_blocks, stream);
                 break;
             case kPlaceGlobal: e = launch_gk<kPlaceGlobal, 4>(prm, sm_count, max_blocks, stream); break;
             default: return cudaErrorInvalidValue;
