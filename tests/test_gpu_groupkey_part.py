@@ -147,3 +147,28 @@ def test_crosses_segment_boundary(cuda, path):
             res.append(o.cpu().numpy().view(np.uint64).reshape(G, 6, 2))
         assert np.array_equal(res[0], res[1])
         assert int(res[0][:, 0, 0].sum()) == passing and not res[0][:, 0, 1].any()
+
+
+@pytest.mark.parametrize("num_groups", [64, 1000, 4096, 65536])
+@pytest.mark.parametrize("blocks", [0, 1, 3])
+def test_one_key_many_rows(table, monkeypatch, num_groups, blocks):
+    """Most rows of one key, one discount and the largest quantity: one partition takes every record of a
+    tile (several chunks a round), and one cell's count and quantity pass 65,536 and 2^16 many times
+    over (the carries of a packed word). The other keys' rows fall on partial chunks of 1 to 257
+    records."""
+    comp, _, _ = table
+    comp = {k: (v.copy() if isinstance(v, np.ndarray) else v) for k, v in comp.items()}
+    n = len(comp["shipdate"])
+    hot = num_groups - 1
+    keys = np.full(n, hot, dtype=np.uint32)
+    at = 1000
+    for j, run in enumerate([1, 31, 32, 33, 255, 256, 257, 1500]):
+        keys[at:at + run] = j * 7 % num_groups
+        at += 20_011
+    rest = keys == hot
+    comp["quantity"][rest] = 255
+    comp["discount"][rest] = 5
+    c, keep = device_cols(comp)
+    for forced in ["single", "partitioned"] if num_groups > 4096 else ["single"]:
+        monkeypatch.setenv("Q1_GROUPKEY_PATH", forced)
+        check(comp, keys, num_groups, 730089, run_gpu(c, keys, num_groups, "shared_mem_per_thread", 730089, blocks))

@@ -415,11 +415,11 @@ static bool chosen_on_device(int placement, uint32_t num_groups) {
 //   kModeSinglePass   the group-key kernel: keys < 4096 in a shared slot table, passing rows of
 //                     larger ("cold") keys straight into the global accumulators;
 //   kModePartitioned  (more than 4096 groups) the two-pass radix partition (groupkey_part.cu).
-// Between the last two, a cost model fitted to both paths on a B200 (ms per 600 M rows; c =
-// fraction of the rows that pass with a cold key, p = fraction that pass): single pass 2.2 + 20 c
-// + 0.3 p; partitioned 1.7 + 4.3 c + 5.65 (p - c), the hot rows costing more there because skewed
-// keys contend for the same ring counters and slots. The single pass wins when
-// 21.35 c - 5.35 p < -0.5: skewed keys with many passing rows.
+// Between the last two, a cost model fitted to both paths on a B200 (ms per 200 M rows; c = fraction of
+// the rows that pass with a cold key, p = fraction that pass): single pass 0.73 + 3.5 c + 0.35 p (Zipf
+// keys over 5,000 to 65,536 groups 1.08, 1.49, 1.90 at full pass; uniform ones, all cold, 6.1 to 6.8),
+// partitioned 0.56 + 0.75 p and 8 us for its three kernels (1.26 and 1.35 uniform and Zipf at full
+// pass, 0.65 at 7%). The single pass wins when (0.17 + 3.5 c - 0.4 p) x rows < 1.5 M.
 // All loads of a thread's eight samples are in flight together: one block of 256 threads taking them
 // one after another was 31 us, two thirds of a launch on 100,000 rows.
 __global__ void __launch_bounds__(1024) q1_groupkey_choose(const uint16_t* __restrict__ ship,
@@ -477,8 +477,8 @@ __global__ void __launch_bounds__(1024) q1_groupkey_choose(const uint16_t* __res
         } else if (!allow_part) {
             *mode = kModeSinglePass;
         } else {
-            const int64_t score = 2135ll * C - 535ll * P;   // 100 x (21.35 c - 5.35 p) x K
-            *mode = score < -50ll * K ? kModeSinglePass : kModePartitioned;
+            const int64_t score = 170ll * K + 3500ll * C - 400ll * P;   // 1000 x (0.17 + 3.5 c - 0.4 p) x K
+            *mode = score * (int64_t)rows < 1500000000ll * K ? kModeSinglePass : kModePartitioned;
         }
     }
 }
