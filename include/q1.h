@@ -409,7 +409,7 @@ typedef struct q1_batch_opts {
 
 typedef struct q1_batch_desc {
     uint32_t instances, items, chunk_tiles, tile_rows, grid, uses_graph, tuned_classes;
-    uint32_t mode_count[3];       /* instances per placement: registers, shared table, global  */
+    uint32_t mode_count[3];       /* instances per placement: 0 (unused), shared table, global */
     uint64_t total_rows, total_groups;
 } q1_batch_desc;
 
@@ -422,7 +422,8 @@ q1_status q1_batch_create(const q1_batch_instance* instances, uint32_t n, const 
 /* One execution of every instance (asynchronous; q1_sync_check reports device errors). */
 q1_status q1_batch_run(q1_batch* b, void* cuda_stream);
 q1_status q1_batch_describe(q1_batch* b, q1_batch_desc* out);
-/* Placement chosen for instance i: 0 registers (num_groups <= 4), 1 shared table, 2 global. */
+/* Placement chosen for instance i: 1 shared table, 2 global (0, registers, is no longer chosen: the
+ * table is the faster one for up to four groups too). */
 q1_status q1_batch_instance_mode(q1_batch* b, uint32_t i, int32_t* mode);
 q1_status q1_batch_destroy(q1_batch* b);
 

@@ -164,3 +164,25 @@ def test_batch_equals_plain_launches(data):
                                               ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(stream)))
         _lib.check(q.lib().q1_sync_check(ctypes.c_void_p(stream)))
         assert np.array_equal(read(out, g), want[i])
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("shared", [False, True])
+def test_batch_tables_are_stored_or_summed(cuda, shared, offset):
+    """Each run overwrites what the tables held (empty groups too); instances that share a table sum in it. Tables
+    start at any 8-byte boundary."""
+    inst = [i for i in make_instances(seed=91, n=24) if i[2] in (4, 64, 1024)]
+    arr, outs, keep = to_device(inst)
+    table = {}
+    for i, w in enumerate(oracle_tables(inst)):
+        g = inst[i][2]
+        t = g if shared else i   # a table per group count, or per instance
+        table.setdefault(t, [outs[i].fill_(-7), 0])
+        table[t][1] = table[t][1] + q.decode_aggregates(w, g)
+        arr[i].aggregates = table[t][0].data_ptr() + 8 * offset
+    stream = torch.cuda.current_stream().cuda_stream
+    run_batch(arr, len(inst), _lib.BatchOpts(1, 0, 0, 0, None), stream)
+    for t, (out, total) in table.items():
+        g = t if shared else inst[t][2]
+        got = q.decode_aggregates(out.cpu().numpy().view(np.uint64)[offset : offset + g * 12], g)
+        assert np.array_equal(got, total), (t, g)

@@ -11,16 +11,18 @@
 //
 // Per CTA: one producer warp claims items, and for every tile of the item writes the stage's
 // metadata (instance, first row, row count) and streams the six column slices with
-// cp.async.bulk into a shared-memory ring of 4 stages (3 in the table kernel, whose table takes
-// the room of the fourth; a partial last tile is read by the consumers
-// straight from global memory instead). Eight consumer warps aggregate every tile; when the
+// cp.async.bulk into a shared-memory ring of 3 stages (a partial last tile is read by the consumers
+// straight from global memory instead). Sixteen consumer warps aggregate every tile; when the
 // instance changes they flush their accumulators into the instance's scratch (red.global.add),
 // according to the instance's placement mode:
-//   kModeRegisters  num_groups <= 4: per-thread dp4a byte planes (ka::PlaneRegs<4>)
 //   kModeShared     num_groups <= 64: shared (group, discount, tax) cells (ka::Cube3Table);
 //                   <= 1024: shared (group, discount) cells (ka::CubeTable); more groups:
 //                   shared slots for keys < 2048 (ka::SlotTable), the rest spilled
 //   kModeGlobal     every passing row reduces straight into the scratch accumulators
+// Instances of up to four groups take the cells as well. (Byte planes in registers for them measured
+// slower in every mix: in a kernel of their own, beside the tables' on a share of the SMs, 64 instances
+// of 10^4 to 10^7 rows 330 us instead of 293, 128 of up to 5 * 10^7 rows 2123 instead of 2022, one of
+// 10^8 rows and 4 groups 299 instead of 277; in this kernel they spill.)
 // (engines in q1_keyagg.cuh). Scratch per instance: num_groups x 8 u64, folded into the
 // caller's int128 table by batch_finalize.
 // All waits are bounded (q1_ptx.cuh); on expiry the kernel records a status bit and leaves.
@@ -39,13 +41,9 @@ using namespace ptx;
 namespace bk {
 
 constexpr uint32_t R = ka::R;   // 2048 rows per tile
-// ring stages: 4 in the register-planes kernel, 3 in the table kernel
-template <bool kRegs>
-__host__ __device__ constexpr uint32_t stages() { return kRegs ? 4u : 3u; }
-// consumer warps: 8 in the register-planes kernel (128 registers a thread), 16 in the table
-// kernel, whose shared-memory atomics need more warps in flight
-template <bool kRegs>
-__host__ __device__ constexpr uint32_t consumer_warps() { return kRegs ? 8u : 16u; }
+constexpr uint32_t kRing = 3;            // stages
+// 16 consumer warps: the shared-memory atomics need many in flight.
+constexpr uint32_t kWarps = 16;
 constexpr uint32_t kStage = ka::kStageBytes;
 constexpr uint32_t kSteps = R / 4;
 constexpr uint32_t kKindFull = 0, kKindPartial = 1, kKindEnd = 2;
@@ -53,8 +51,8 @@ constexpr uint32_t kKindFull = 0, kKindPartial = 1, kKindEnd = 2;
 constexpr uint32_t cmax(uint32_t a, uint32_t b) { return a > b ? a : b; }
 constexpr uint32_t kTableBytes =
     cmax(ka::cube3_bytes(ka::kCube3MaxGroups), cmax(ka::cube_bytes(ka::kCubeMaxGroups), ka::slot_bytes(ka::kSlots)));
-// the table kernel's ring and table, with room left for its static shared memory (< 1 KB)
-static_assert(3 * kStage + kTableBytes + 512 <= 227 * 1024, "table kernel shared memory");
+// ring and table, with room left for the static shared memory (< 1 KB)
+static_assert(kRing * kStage + kTableBytes + 512 <= 227 * 1024, "table kernel shared memory");
 
 struct __align__(16) StageMeta {
     uint32_t instance;
@@ -88,23 +86,17 @@ __device__ __forceinline__ bool consume_engine(const BatchParams& prm, uint32_t 
                                                uint64_t* empty_bar, const StageMeta* meta, uint32_t& k,
                                                ka::ConsumerBarrier& cb, uint32_t& bad) {
     const uint32_t lane = threadIdx.x & 31u, ctid = threadIdx.x;
-    ka::PlaneRegs<4> regs;
     ka::Cube3Table cube3;
     ka::CubeTableT<false> cube;
     ka::SlotTable slots;
-    if constexpr (E == kEngRegisters) regs.zero();
     Current c{nullptr, nullptr, 0xFFFFFFFFu, 0, 0, 0};
-    uint32_t tiles_since = 0;
     uint64_t rows_since = 0;
     bool ok = true;
 
     auto flush = [&]() {
-        tiles_since = 0;
         rows_since = 0;
         if (c.id == 0xFFFFFFFFu) return;
-        if constexpr (E == kEngRegisters) {
-            regs.flush(c.acc, c.num_groups, lane);
-        } else if constexpr (E != kEngGlobal) {
+        if constexpr (E != kEngGlobal) {
             cb.sync(lane, prm.status);
             if constexpr (E == kEngCube3) cube3.flush(c.acc, c.num_groups, ctid, W * 32);
             else if constexpr (E == kEngCube) cube.flush(c.acc, c.num_groups, ctid, W * 32);
@@ -113,11 +105,7 @@ __device__ __forceinline__ bool consume_engine(const BatchParams& prm, uint32_t 
         }
     };
     auto add = [&](const ka::KeyQuad& x) {
-        if constexpr (E == kEngRegisters) {
-            regs.add(x, c.num_groups, bad, [&](uint32_t key, uint32_t q, uint32_t d, uint32_t t, uint32_t p) {
-                ka::scratch_row(c.acc, key, q, d, t, p);
-            });
-        } else if constexpr (E == kEngCube3) {
+        if constexpr (E == kEngCube3) {
             ka::table_quad(cube3, x, c.num_groups, c.hot, c.acc, bad);
         } else if constexpr (E == kEngCube) {
             ka::table_quad(cube, x, c.num_groups, c.hot, c.acc, bad);
@@ -165,11 +153,9 @@ __device__ __forceinline__ bool consume_engine(const BatchParams& prm, uint32_t 
             if constexpr (E == kEngCube3) cube3.bind(tab, c.num_groups);
             if constexpr (E == kEngCube) cube.bind(tab, c.num_groups);
             if constexpr (E == kEngSlots) slots.bind(tab, c.hot);
-        } else if ((E == kEngRegisters && tiles_since >= ka::kPlaneFlushTiles) ||
-                   (E != kEngRegisters && E != kEngGlobal && rows_since + m.rows > ka::kTableFlushRows)) {
+        } else if (E != kEngGlobal && rows_since + m.rows > ka::kTableFlushRows) {
             flush();
         }
-        ++tiles_since;
         rows_since += m.rows;
         if (m.kind == kKindFull) {
             const uint32_t base = ring + s * kStage;
@@ -194,28 +180,20 @@ __device__ __forceinline__ bool consume_engine(const BatchParams& prm, uint32_t 
     return ok;
 }
 
-// Engine queue processed at step `step` of a CTA, and the engine code that processes it. The
-// register-planes kernel has one step (queue 0). The table kernel starts at its role's queue
-// among 1..4 (grid ranges role_end), visits the others in turn, then helps with queue 0 through
-// the (group, discount, tax) cells, which hold any instance of <= 4 groups.
-template <bool kRegs>
+// Engine queue processed at step `step` of a CTA: it starts at its role's queue (grid ranges
+// role_end) and visits the others in turn.
 __device__ __forceinline__ uint32_t queue_at(const BatchParams& prm, uint32_t step) {
-    if (kRegs) return kEngRegisters;
-    uint32_t e0 = 1;
+    uint32_t e0 = 0;
     while (e0 + 1 < kEngines && blockIdx.x >= prm.role_end[e0]) ++e0;
-    return step < kEngines - 1 ? 1u + (e0 - 1u + step) % (kEngines - 1u) : (uint32_t)kEngRegisters;
+    return (e0 + step) % kEngines;
 }
-template <bool kRegs>
-__host__ __device__ constexpr uint32_t steps() { return kRegs ? 1u : kEngines; }
 
 }  // namespace bk
 
-template <bool kRegs>
-__global__ void __launch_bounds__((bk::consumer_warps<kRegs>() + 1) * 32, 1)
+__global__ void __launch_bounds__((bk::kWarps + 1) * 32, 1)
     q1_batch_kernel(const __grid_constant__ BatchParams prm) {
     using namespace bk;
-    constexpr uint32_t W = consumer_warps<kRegs>();
-    constexpr uint32_t S = stages<kRegs>();
+    constexpr uint32_t W = kWarps, S = kRing;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full_bar[S];
     __shared__ __align__(8) uint64_t empty_bar[S];
@@ -224,7 +202,7 @@ __global__ void __launch_bounds__((bk::consumer_warps<kRegs>() + 1) * 32, 1)
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t ring = smem_addr(smem);
-    uint8_t* const tab = smem + S * kStage;   // shared table (table kernel), all zero between instances
+    uint8_t* const tab = smem + S * kStage;   // shared table, all zero between instances
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < S; ++s) {
@@ -234,8 +212,7 @@ __global__ void __launch_bounds__((bk::consumer_warps<kRegs>() + 1) * 32, 1)
         mbar_init(smem_addr(&consumers_bar), W);
         fence_mbar_init();
     }
-    if (!kRegs)
-        for (uint32_t i = threadIdx.x; i < kTableBytes / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(tab)[i] = 0;
+    for (uint32_t i = threadIdx.x; i < kTableBytes / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(tab)[i] = 0;
     __syncthreads();
 
     if (warp == W) {
@@ -246,8 +223,8 @@ __global__ void __launch_bounds__((bk::consumer_warps<kRegs>() + 1) * 32, 1)
             const uint64_t pol = policy_evict_first();
             uint32_t k = 0;
             bool ok = true;
-            for (uint32_t step = 0; step < steps<kRegs>() && ok; ++step) {
-                const uint32_t e = queue_at<kRegs>(prm, step);
+            for (uint32_t step = 0; step < kEngines && ok; ++step) {
+                const uint32_t e = queue_at(prm, step);
                 const uint32_t count = prm.item_begin[e + 1] - prm.item_begin[e];
                 for (;;) {
                     const uint32_t idx = count ? atomicAdd(prm.cursor + e, 1u) : count;
@@ -298,20 +275,14 @@ __global__ void __launch_bounds__((bk::consumer_warps<kRegs>() + 1) * 32, 1)
         // The same queue order; each engine's loop keeps only its own accumulators live.
         ka::ConsumerBarrier cb{smem_addr(&consumers_bar), 0};
         uint32_t bad = 0, k = 0;
-        for (uint32_t step = 0; step < steps<kRegs>(); ++step) {
-            const uint32_t e = queue_at<kRegs>(prm, step);
+        for (uint32_t step = 0; step < kEngines; ++step) {
+            const uint32_t e = queue_at(prm, step);
             bool ok;
-            if constexpr (kRegs) {
-                ok = consume_engine<kEngRegisters, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad);
-            } else {
-                switch (e) {
-                    case kEngCube: ok = consume_engine<kEngCube, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad); break;
-                    case kEngSlots: ok = consume_engine<kEngSlots, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad); break;
-                    case kEngGlobal: ok = consume_engine<kEngGlobal, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad); break;
-                    default:   // queues 1 and 0
-                        ok = consume_engine<kEngCube3, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad);
-                        break;
-                }
+            switch (e) {
+                case kEngCube3: ok = consume_engine<kEngCube3, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad); break;
+                case kEngCube: ok = consume_engine<kEngCube, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad); break;
+                case kEngSlots: ok = consume_engine<kEngSlots, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad); break;
+                default: ok = consume_engine<kEngGlobal, W, S>(prm, ring, tab, full_bar, empty_bar, meta, k, cb, bad); break;
             }
             if (!ok) break;
         }
@@ -321,7 +292,9 @@ __global__ void __launch_bounds__((bk::consumer_warps<kRegs>() + 1) * 32, 1)
 }
 
 
-// scratch of every instance -> its int128 table (+=); one thread per (instance, group).
+// scratch of every instance -> its int128 table, added to it or (overwrite) stored, empty groups
+// too, so that the tables need no zeroing first; one thread per (instance, group).
+template <bool kOverwrite>
 __global__ void __launch_bounds__(256) q1_batch_finalize(const BatchInstanceDev* __restrict__ inst,
                                                          const uint64_t* __restrict__ group_base, uint32_t ninst,
                                                          uint64_t total_groups) {
@@ -335,84 +308,41 @@ __global__ void __launch_bounds__(256) q1_batch_finalize(const BatchInstanceDev*
     const BatchInstanceDev& in = inst[lo];
     const uint32_t g = (uint32_t)(t - group_base[lo]);
     const unsigned long long* a = in.acc + 8ull * g;
-    if (!a[0]) return;
     unsigned long long* o = in.out + 12ull * g;
-    atomic_add_u128(o + 2 * kAggCount, a[0], 0);
-    const unsigned __int128 q = (unsigned __int128)a[1] * 100u;
-    atomic_add_u128(o + 2 * kAggQty, (uint64_t)q, (uint64_t)(q >> 64));
-    atomic_add_u128(o + 2 * kAggBasePrice, a[3], 0);
-    atomic_add_u128(o + 2 * kAggDisc, a[2], 0);
-    const unsigned __int128 dp = (unsigned __int128)a[4] + ((unsigned __int128)a[5] << 32);
-    atomic_add_u128(o + 2 * kAggDiscPrice, (uint64_t)dp, (uint64_t)(dp >> 64));
-    const unsigned __int128 ch = (unsigned __int128)a[6] + ((unsigned __int128)a[7] << 32);
-    atomic_add_u128(o + 2 * kAggCharge, (uint64_t)ch, (uint64_t)(ch >> 64));
+    if (!kOverwrite && !a[0]) return;
+    auto put = [&](int agg, unsigned __int128 v) {
+        if (kOverwrite) {   // 8-byte stores: the tables need no more alignment than the 64-bit atomics do
+            o[2 * agg] = (uint64_t)v;
+            o[2 * agg + 1] = (uint64_t)(v >> 64);
+        } else {
+            atomic_add_u128(o + 2 * agg, (uint64_t)v, (uint64_t)(v >> 64));
+        }
+    };
+    put(kAggCount, a[0]);
+    put(kAggQty, (unsigned __int128)a[1] * 100u);
+    put(kAggBasePrice, a[3]);
+    put(kAggDisc, a[2]);
+    put(kAggDiscPrice, (unsigned __int128)a[4] + ((unsigned __int128)a[5] << 32));
+    put(kAggCharge, (unsigned __int128)a[6] + ((unsigned __int128)a[7] << 32));
 }
 
-// Zero every instance's int128 result table; one thread per (instance, group).
-__global__ void __launch_bounds__(256) q1_batch_zero_outputs(const BatchInstanceDev* __restrict__ inst,
-                                                             const uint64_t* __restrict__ group_base, uint32_t ninst,
-                                                             uint64_t total_groups) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total_groups) return;
-    uint32_t lo = 0, hi = ninst;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (group_base[mid] <= t) lo = mid; else hi = mid;
-    }
-    unsigned long long* o = inst[lo].out + 12ull * (t - group_base[lo]);
-#pragma unroll
-    for (int i = 0; i < 12; ++i) o[i] = 0;
+uint32_t batch_smem_bytes() { return bk::kRing * bk::kStage + bk::kTableBytes; }
+
+cudaError_t batch_prepare_launch() {
+    return cudaFuncSetAttribute(q1_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)batch_smem_bytes());
 }
 
-cudaError_t launch_batch_zero_outputs(const BatchInstanceDev* inst, const uint64_t* group_base, uint32_t ninst,
-                                      uint64_t total_groups, cudaStream_t stream) {
-    if (!total_groups) return cudaSuccess;
-    q1_batch_zero_outputs<<<(unsigned)((total_groups + 255) / 256), 256, 0, stream>>>(inst, group_base, ninst,
-                                                                                    total_groups);
+cudaError_t launch_batch(const BatchParams& prm, cudaStream_t stream) {
+    q1_batch_kernel<<<prm.grid, (bk::kWarps + 1) * 32, batch_smem_bytes(), stream>>>(prm);
     return cudaGetLastError();
 }
 
-uint32_t batch_smem_bytes() { return bk::stages<false>() * bk::kStage + bk::kTableBytes; }
-// The register-planes kernel needs only the ring; asking for more than half the SM's shared
-// memory keeps it at one CTA per SM, like the table kernel.
-static uint32_t batch_regs_smem_bytes() { return 120u * 1024u; }
-
-cudaError_t batch_prepare_launch() {
-    cudaError_t e = cudaFuncSetAttribute(q1_batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)batch_smem_bytes());
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(q1_batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)batch_regs_smem_bytes());
-}
-
-cudaError_t launch_batch(const BatchParams& prm, uint32_t grid_regs, uint32_t grid_tables, cudaStream_t stream,
-                         cudaStream_t aux, cudaEvent_t fork, cudaEvent_t join) {
-    cudaError_t e = cudaSuccess;
-    const bool both = grid_regs && grid_tables;
-    if (both) {
-        if ((e = cudaEventRecord(fork, stream)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(aux, fork, 0)) != cudaSuccess) return e;
-    }
-    if (grid_regs) {
-        q1_batch_kernel<true><<<grid_regs, (bk::consumer_warps<true>() + 1) * 32, batch_regs_smem_bytes(),
-                                both ? aux : stream>>>(prm);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    if (grid_tables) {
-        q1_batch_kernel<false><<<grid_tables, (bk::consumer_warps<false>() + 1) * 32, batch_smem_bytes(), stream>>>(prm);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    if (both) {
-        if ((e = cudaEventRecord(join, aux)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-}
-
 cudaError_t launch_batch_finalize(const BatchInstanceDev* inst, const uint64_t* group_base, uint32_t ninst,
-                                  uint64_t total_groups, cudaStream_t stream) {
+                                  uint64_t total_groups, bool overwrite, cudaStream_t stream) {
     if (!total_groups) return cudaSuccess;
-    q1_batch_finalize<<<(unsigned)((total_groups + 255) / 256), 256, 0, stream>>>(inst, group_base, ninst, total_groups);
+    const unsigned grid = (unsigned)((total_groups + 255) / 256);
+    if (overwrite) q1_batch_finalize<true><<<grid, 256, 0, stream>>>(inst, group_base, ninst, total_groups);
+    else q1_batch_finalize<false><<<grid, 256, 0, stream>>>(inst, group_base, ninst, total_groups);
     return cudaGetLastError();
 }
 

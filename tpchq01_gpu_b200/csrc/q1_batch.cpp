@@ -1,14 +1,14 @@
 // Batched aggregation host runtime: instance descriptors, the device work queue, the autotuner
 // and CUDA-graph capture of one batch execution.
 //
-// One execution = [zero the instances' result tables] + zero the scratch + reset the queue
-// cursor + the persistent batch kernel + the finalize kernel, captured once into a CUDA graph and
+// One execution = zero the scratch + reset the queue cursor + the persistent batch kernels + the
+// finalize kernel (which stores or adds the result tables), captured once into a CUDA graph and
 // replayed by every q1_batch_run.
 //
 // Autotuner: an instance's class is (floor(log2 rows), num_groups, selectivity decile), the
 // selectivity being measured on a strided sample of its ship dates. For every class the tuner
 // times the batch kernel on the class's largest instance alone under each applicable placement
-// (registers when num_groups <= 4, shared table, global) and keeps the fastest; the work-item
+// (shared table, global) and keeps the fastest; the work-item
 // size (tiles per item) is then chosen by timing the whole batch with a few candidates. Results
 // are cached in a text file ("mode <log2rows> <groups> <decile> <mode>", "chunk <signature>
 // <tiles>") so later batches with the same classes skip the measurements.
@@ -70,7 +70,8 @@ void load_cache(const std::string& path) {
         if (kind == "mode") {
             int lr, dec;
             uint32_t g, m;
-            if (f >> lr >> g >> dec >> m) modes[ClassKey(lr, g, dec)] = m;
+            // (a file's 0, the register placement it once had, is the shared table)
+            if (f >> lr >> g >> dec >> m) modes[ClassKey(lr, g, dec)] = m == kModeGlobal ? kModeGlobal : kModeShared;
         } else if (kind == "chunk") {
             std::string sig;
             uint32_t t;
@@ -85,7 +86,7 @@ void load_cache(const std::string& path) {
 void save_cache(const std::string& path) {
     if (path.empty()) return;
     std::ofstream f(path, std::ios::trunc);
-    f << "# q1 batch autotuner cache: mode <log2rows> <groups> <selectivity decile> <0 registers|1 shared|2 global>;"
+    f << "# q1 batch autotuner cache: mode <log2rows> <groups> <selectivity decile> <1 shared|2 global>;"
          " chunk <signature> <tiles per work item>\n";
     for (auto& kv : g_mode_cache[path])
         f << "mode " << std::get<0>(kv.first) << ' ' << std::get<1>(kv.first) << ' ' << std::get<2>(kv.first) << ' '
@@ -96,7 +97,6 @@ void save_cache(const std::string& path) {
 }  // namespace
 
 uint32_t q1::batch_engine(uint32_t mode, uint32_t num_groups) {
-    if (mode == kModeRegisters && num_groups <= 4) return kEngRegisters;
     if (mode == kModeGlobal) return kEngGlobal;
     if (num_groups <= 64) return kEngCube3;     // ka::kCube3MaxGroups
     if (num_groups <= 1024) return kEngCube;    // ka::kCubeMaxGroups
@@ -106,23 +106,47 @@ uint32_t q1::batch_engine(uint32_t mode, uint32_t num_groups) {
 namespace {
 
 // Relative cost of a row per engine (time per row of the group-key kernel on a B200 at 100% pass,
-// uniform keys, register planes = 1: 4 groups 1.57 ms per 600 M rows, 64 groups 1.87 ms, 1024
-// groups 2.26 ms, 4096 groups 2.79 ms): used only to split the grid.
-constexpr double kEngineCost[kEngines] = {1.0, 1.19, 1.44, 1.78, 10.0};
+// uniform keys, 64 groups = 1: 1.87 ms per 600 M rows, 1024 groups 2.26 ms, 4096 groups 2.79 ms): used
+// only to split the grid.
+constexpr double kEngineCost[kEngines] = {1.0, 1.21, 1.50, 8.4};
 
-void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, int only, std::vector<BatchItem>& items,
-                uint32_t begin[kEngines + 1]) {
-    std::vector<BatchItem> per[kEngines];
+// Work items: every instance in pieces of `chunk` tiles or, with chunk 0, of falling size: an engine's
+// largest instances first, each piece three quarters of an equal share of the tiles its engine's CTAs still
+// have to do, down to 16 tiles (a CTA's share, if that is less). Every change of instance costs a CTA a
+// flush of its table (5 us for 64 groups' cells), so most of the work is in few large pieces, and the
+// small ones at the end even out the CTAs. 64 instances of 10^4 to 10^7 rows with 5, 64 and 1024 groups:
+// 291 us, 321 in pieces of one size; 64 of 1024 groups: 324 and 391.
+void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32_t grid, int only,
+                std::vector<BatchItem>& items, uint32_t begin[kEngines + 1]) {
+    std::vector<uint32_t> of[kEngines];   // instances by engine, the largest first
+    uint64_t tiles[kEngines] = {};
+    auto tiles_of = [&](uint32_t i) { return (inst[i].rows + kBatchTileRows - 1) / kBatchTileRows; };
+    double total = 0;
     for (uint32_t i = 0; i < n; ++i) {
         if (only >= 0 && i != (uint32_t)only) continue;
         const uint32_t e = batch_engine(inst[i].mode, inst[i].num_groups);
-        const uint64_t tiles = (inst[i].rows + kBatchTileRows - 1) / kBatchTileRows;
-        for (uint64_t t = 0; t < tiles; t += chunk) {
-            BatchItem it{};
-            it.instance = i;
-            it.first_tile = (uint32_t)t;
-            it.num_tiles = (uint32_t)std::min<uint64_t>(chunk, tiles - t);
-            per[e].push_back(it);
+        of[e].push_back(i);
+        tiles[e] += tiles_of(i);
+        total += (double)tiles_of(i) * kEngineCost[e];
+    }
+    std::vector<BatchItem> per[kEngines];
+    for (uint32_t e = 0; e < kEngines; ++e) {
+        std::stable_sort(of[e].begin(), of[e].end(), [&](uint32_t a, uint32_t c) { return inst[a].rows > inst[c].rows; });
+        const double ctas = std::max(1.0, grid * (double)tiles[e] * kEngineCost[e] / std::max(1.0, total));
+        const uint64_t least = std::max<uint64_t>(2, std::min<uint64_t>(16, (uint64_t)(tiles[e] / ctas)));
+        uint64_t left = tiles[e];
+        for (uint32_t i : of[e]) {
+            const uint64_t all = tiles_of(i);
+            for (uint64_t t = 0; t < all;) {
+                const uint64_t most = chunk ? chunk : std::max(least, (uint64_t)((double)left / (1.33 * ctas)));
+                BatchItem it{};
+                it.instance = i;
+                it.first_tile = (uint32_t)t;
+                it.num_tiles = (uint32_t)std::min(most, all - t);
+                per[e].push_back(it);
+                t += it.num_tiles;
+                left -= it.num_tiles;
+            }
         }
     }
     items.clear();
@@ -136,49 +160,29 @@ void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, int on
     begin[kEngines] = (uint32_t)items.size();
 }
 
-// Splits `grid` CTAs: the register-planes kernel gets its cost share (a little under, since the
-// table kernel also drains queue 0 once its own queues are empty), the table kernel the rest,
-// divided among queues 1..4 by cost.
+// At most `grid` CTAs, no more than items, and which queue each starts with: the engines' shares of the
+// estimated cost (a CTA whose queue is empty goes on to the next one).
 void plan_roles(const std::vector<BatchItem>& items, const uint32_t begin[kEngines + 1], uint32_t grid,
                 BatchParams& prm) {
-    double cost[kEngines] = {0, 0, 0, 0, 0}, total = 0, tables = 0;
+    double cost[kEngines] = {}, total = 0;
     for (uint32_t e = 0; e < kEngines; ++e) {
         for (uint32_t j = begin[e]; j < begin[e + 1]; ++j) cost[e] += (double)items[j].num_tiles * kEngineCost[e];
         total += cost[e];
-        if (e) tables += cost[e];
     }
-    uint32_t regs = 0;
-    if (cost[0] > 0) {
-        regs = tables > 0 ? (uint32_t)(0.9 * grid * cost[0] / total) : grid;
-        regs = std::max<uint32_t>(1, std::min<uint32_t>(regs, grid - (tables > 0 ? 1 : 0)));
-        regs = std::min<uint32_t>(regs, begin[1] - begin[0]);
+    prm.grid = std::min<uint32_t>(grid, begin[kEngines]);
+    double before = 0;
+    for (uint32_t e = 0; e < kEngines; ++e) {
+        before += cost[e];
+        prm.role_end[e] = total > 0 ? (uint32_t)(prm.grid * before / total + 0.5) : prm.grid;
     }
-    const uint32_t tgrid = tables > 0 ? std::max<uint32_t>(1, std::min<uint32_t>(grid - regs, begin[kEngines] - begin[1]))
-                                      : 0;
-    prm.grid_regs = regs;
-    prm.grid_tables = tgrid;
-    // queue shares of the table kernel
-    uint32_t share[kEngines] = {0, 0, 0, 0, 0}, used = 0, big = 1;
-    for (uint32_t e = 1; e < kEngines; ++e) {
-        if (cost[e] <= 0) continue;
-        share[e] = std::max<uint32_t>(1, (uint32_t)(tgrid * cost[e] / (tables > 0 ? tables : 1)));
-        used += share[e];
-        if (share[e] > share[big]) big = e;
-    }
-    if (tgrid) {
-        if (used > tgrid) share[big] -= std::min(share[big] - 1, used - tgrid);
-        else share[big] += tgrid - used;
-    }
-    prm.role_end[0] = 0;
-    uint32_t acc = 0;
-    for (uint32_t e = 1; e < kEngines; ++e) prm.role_end[e] = (acc += share[e]);
+    prm.role_end[kEngines - 1] = prm.grid;
 }
 
 }  // namespace
 
 void q1::batch_plan(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32_t grid, std::vector<BatchItem>& items,
                     BatchParams& prm) {
-    plan_items(inst, n, std::max<uint32_t>(1, chunk), -1, items, prm.item_begin);
+    plan_items(inst, n, chunk, grid, -1, items, prm.item_begin);
     plan_roles(items, prm.item_begin, grid, prm);
 }
 
@@ -198,17 +202,13 @@ struct q1_batch {
     uint32_t chunk = 0;
     uint32_t grid = 0;
     bool use_graph = true;
-    bool zero_outputs = true;
+    bool overwrite = true;                   // each run overwrites the result tables
+    bool shared_tables = false;              // result tables of two instances overlap: zeroed, then added to
     std::string cache;
     DevMem d_inst, d_items, d_base, d_scratch, d_cursor;
-    cudaStream_t aux = nullptr;              // the register-planes kernel runs beside the table kernel
-    cudaEvent_t fork = nullptr, join = nullptr;
     ~q1_batch() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
-        if (aux) cudaStreamDestroy(aux);
-        if (fork) cudaEventDestroy(fork);
-        if (join) cudaEventDestroy(join);
     }
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -218,9 +218,9 @@ struct q1_batch {
 // Items of every instance (only < 0) or of one instance, grouped by engine, and the grid roles.
 static void build_items(q1_batch* b, uint32_t chunk, int only = -1) {
     for (uint32_t i = 0; i < b->n; ++i) b->inst[i].mode = b->modes[i];
-    plan_items(b->inst.data(), b->n, std::max<uint32_t>(1, chunk), only, b->items, b->roles.item_begin);
+    plan_items(b->inst.data(), b->n, chunk, b->grid, only, b->items, b->roles.item_begin);
     plan_roles(b->items, b->roles.item_begin, b->grid, b->roles);
-    b->launch_grid = b->roles.grid_regs + b->roles.grid_tables;
+    b->launch_grid = b->roles.grid;
 }
 
 static q1_status upload(q1_batch* b) {
@@ -243,10 +243,8 @@ static q1_status upload(q1_batch* b) {
 
 // The launches of one execution (graph body).
 static q1_status enqueue(q1_batch* b, cudaStream_t s) {
-    if (b->zero_outputs && b->total_groups) {
-        Q1_CUDA(launch_batch_zero_outputs(static_cast<const BatchInstanceDev*>(b->d_inst.p),
-                                          static_cast<const uint64_t*>(b->d_base.p), b->n, b->total_groups, s));
-    }
+    if (b->overwrite && b->shared_tables)
+        for (uint32_t i = 0; i < b->n; ++i) Q1_CUDA(cudaMemsetAsync(b->inst[i].out, 0, 96ull * b->inst[i].num_groups, s));
     Q1_CUDA(cudaMemsetAsync(b->d_scratch.p, 0, b->total_groups * 64ull, s));
     Q1_CUDA(cudaMemsetAsync(b->d_cursor.p, 0, 4 * kEngines, s));
     if (!b->items.empty()) {
@@ -255,10 +253,11 @@ static q1_status enqueue(q1_batch* b, cudaStream_t s) {
         prm.items = static_cast<const BatchItem*>(b->d_items.p);
         prm.cursor = static_cast<uint32_t*>(b->d_cursor.p);
         prm.status = b->di->status;
-        Q1_CUDA(launch_batch(prm, prm.grid_regs, prm.grid_tables, s, b->aux, b->fork, b->join));
+        Q1_CUDA(launch_batch(prm, s));
     }
     Q1_CUDA(launch_batch_finalize(static_cast<const BatchInstanceDev*>(b->d_inst.p),
-                                  static_cast<const uint64_t*>(b->d_base.p), b->n, b->total_groups, s));
+                                  static_cast<const uint64_t*>(b->d_base.p), b->n, b->total_groups,
+                                  b->overwrite && !b->shared_tables, s));
     return Q1_OK;
 }
 
@@ -282,9 +281,7 @@ static q1_status time_batch(q1_batch* b, cudaStream_t s, int reps, float* best_m
     return check_device_status(s, b->di->status);
 }
 
-// Work-item size: about 16 items per CTA. Smaller items keep the CTAs reading neighbouring tiles
-// of the same instance at the same time; on 256 instances of 1.49 G rows, 64-tile items ran
-// 5.14 ms against 5.25 ms for 256-tile items.
+// A fixed work-item size for the tuner to compare with pieces of falling size: about 16 items per CTA.
 static uint32_t default_chunk(const q1_batch* b) {
     const uint64_t tiles = (b->total_rows + kBatchTileRows - 1) / kBatchTileRows;
     uint64_t c = tiles / (uint64_t)(b->grid ? b->grid * 16 : 1);
@@ -310,15 +307,10 @@ q1_status q1_batch_create(const q1_batch_instance* in, uint32_t n, const q1_batc
     cudaStream_t s = (cudaStream_t)cuda_stream;
     Q1_CUDA(cudaGetDevice(&b->device));
     q1_status st = device_info(b->device, &b->di);
-    if (st == Q1_OK) {
-        Q1_CUDA(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
-        Q1_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-        Q1_CUDA(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
-    }
     if (st != Q1_OK) return st;
     b->n = n;
     b->use_graph = opts ? opts->use_graph != 0 : true;
-    b->zero_outputs = opts ? opts->accumulate == 0 : true;
+    b->overwrite = opts ? opts->accumulate == 0 : true;
     b->cache = (opts && opts->tune_cache) ? opts->tune_cache : "";
     const int tune = opts ? opts->tune : 0;
     b->grid = (uint32_t)b->di->sm_count;
@@ -351,9 +343,15 @@ q1_status q1_batch_create(const q1_batch_instance* in, uint32_t n, const q1_batc
         d.out = reinterpret_cast<unsigned long long*>(x.aggregates);
         b->group_base[i + 1] = b->group_base[i] + x.num_groups;
         b->total_rows += x.rows;
-        b->modes[i] = x.num_groups <= 4 ? kModeRegisters : kModeShared;   // heuristic default
     }
     b->total_groups = b->group_base[n];
+    std::vector<uint32_t> by_table(n);
+    for (uint32_t i = 0; i < n; ++i) by_table[i] = i;
+    std::sort(by_table.begin(), by_table.end(), [&](uint32_t a, uint32_t c) { return b->inst[a].out < b->inst[c].out; });
+    for (uint32_t i = 1; i < n; ++i) {
+        const BatchInstanceDev& d = b->inst[by_table[i - 1]];
+        b->shared_tables |= b->inst[by_table[i]].out < d.out + 12ull * d.num_groups;
+    }
     if ((st = b->d_inst.alloc(sizeof(BatchInstanceDev) * std::max<uint32_t>(1, n))) != Q1_OK) return st;
     if ((st = b->d_base.alloc(sizeof(uint64_t) * (n + 1))) != Q1_OK) return st;
     if ((st = b->d_scratch.alloc(b->total_groups * 64ull)) != Q1_OK) return st;
@@ -380,7 +378,7 @@ q1_status q1_batch_create(const q1_batch_instance* in, uint32_t n, const q1_batc
         b->cls[i] = ClassKey((int)std::log2((double)std::max<uint64_t>(1, d.rows)), d.num_groups, dec);
     }
 
-    b->chunk = (opts && opts->chunk_tiles > 0) ? (uint32_t)opts->chunk_tiles : default_chunk(b.get());
+    b->chunk = (opts && opts->chunk_tiles > 0) ? (uint32_t)opts->chunk_tiles : 0;   // 0: pieces of falling size
     if (tune > 0) {
         std::lock_guard<std::mutex> lk(g_cache_mutex);
         load_cache(b->cache);
@@ -398,10 +396,7 @@ q1_status q1_batch_create(const q1_batch_instance* in, uint32_t n, const q1_batc
                 modes[kv.first] = b->modes[i];
                 continue;
             }
-            std::vector<uint32_t> cands;
-            if (b->inst[i].num_groups <= 4) cands.push_back(kModeRegisters);
-            cands.push_back(kModeShared);
-            cands.push_back(kModeGlobal);
+            std::vector<uint32_t> cands = {kModeShared, kModeGlobal};
             // the heuristic placement keeps the class unless another is faster by more than 3%
             uint32_t best = saved_modes[i];
             float best_ms = 1e30f;
@@ -437,7 +432,7 @@ q1_status q1_batch_create(const q1_batch_instance* in, uint32_t n, const q1_batc
                 b->chunk = chunks[sig];
             } else {
                 const uint32_t base = default_chunk(b.get());
-                std::vector<uint32_t> cands = {std::max<uint32_t>(2, base / 4), base, std::min<uint32_t>(4096, base * 4)};
+                std::vector<uint32_t> cands = {0, std::max<uint32_t>(2, base / 4), base, std::min<uint32_t>(4096, base * 4)};
                 float best_ms = 1e30f;
                 for (uint32_t c : cands) {
                     build_items(b.get(), c);
@@ -492,7 +487,7 @@ q1_status q1_batch_describe(q1_batch* b, q1_batch_desc* d) {
     memset(d, 0, sizeof(*d));
     d->instances = b->n;
     d->items = (uint32_t)b->items.size();
-    d->chunk_tiles = b->chunk;
+    for (const BatchItem& it : b->items) d->chunk_tiles = std::max(d->chunk_tiles, it.num_tiles);
     d->tile_rows = kBatchTileRows;
     d->grid = b->launch_grid;
     d->total_rows = b->total_rows;

@@ -300,22 +300,6 @@ struct PlaneRegs {
                : a == kAggCharge                               ? warp_sum<63>(v).lo
                                                                : warp_sum<54>(v).lo;
     }
-    // Warp sums of the per-thread partials into the scratch; every lane of the warp calls it.
-    __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t num_groups, uint32_t lane) {
-#pragma unroll
-        for (int i = 0; i < NG; ++i) {
-            if ((uint32_t)i < num_groups) {
-                const uint64_t ch = g[i].value(kAggCharge), dp = g[i].value(kAggDiscPrice);
-                const uint64_t cnt = warp_sum_u64(g[i].cnt);
-                const uint64_t q = warp_sum_u64(g[i].q), d = warp_sum_u64(g[i].d);
-                const uint64_t p = warp_sum_u64(g[i].value(kAggBasePrice));
-                const uint64_t dpl = warp_sum_u64(dp & 0xFFFFFFFFull), dph = warp_sum_u64(dp >> 32);
-                const uint64_t chl = warp_sum_u64(ch & 0xFFFFFFFFull), chh = warp_sum_u64(ch >> 32);
-                if (lane == 0 && cnt) scratch_add(acc, (uint32_t)i, cnt, q, d, p, dpl, dph, chl, chh);
-            }
-            g[i].zero();
-        }
-    }
 };
 
 // ---------------------------------------------------------------------------------------------

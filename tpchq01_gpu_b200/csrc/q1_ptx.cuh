@@ -167,11 +167,5 @@ __device__ __forceinline__ Sum128 warp_sum(uint64_t v) {
     return s;
 }
 
-__device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    return v;
-}
-
 }  // namespace ptx
 }  // namespace q1
