@@ -186,3 +186,50 @@ def test_batch_tables_are_stored_or_summed(cuda, shared, offset):
         g = t if shared else inst[t][2]
         got = q.decode_aggregates(out.cpu().numpy().view(np.uint64)[offset : offset + g * 12], g)
         assert np.array_equal(got, total), (t, g)
+
+
+@pytest.mark.parametrize("chunk", [0, 1])
+def test_batch_many_small_instances(cuda, chunk):
+    """Rows at the edges of a ring tile and of a team's turn, more instances per CTA than it keeps run descriptors
+    for, and every engine (the cells, the slots and, from a cache file, the global one) in the same CTAs."""
+    rows = [1, 1023, 1024, 1025, 2048, 2049, 3072, 3073, 5 * 1024 + 7]
+    groups = [1, 4, 64, 65, 1024, 1025, 3000]
+    inst = []
+    for i in range(63):
+        n, g = rows[i % len(rows)], groups[i % len(groups)]
+        comp = gen_np.compress(gen_np.generate(4000 + i, 0, n))
+        inst.append((comp, gen_np.group_keys_uniform(4000 + i, 0, n, g), g, 729999))
+    want = oracle_tables(inst)
+    arr, outs, keep = to_device(inst)
+    copies = 45   # 2835 instances
+    big = (_lib.BatchInstance * (len(inst) * copies))(*[arr[i % len(inst)] for i in range(len(inst) * copies)])
+    tables = []
+    for i in range(len(big)):
+        tables.append(torch.full((inst[i % len(inst)][2] * 12,), 5, dtype=torch.int64, device="cuda"))
+        big[i].aggregates = tables[i].data_ptr()
+    stream = torch.cuda.current_stream().cuda_stream
+    run_batch(big, len(big), _lib.BatchOpts(1, 0, chunk, 0, None), stream)
+    torch.cuda.synchronize()
+    for i in range(len(big)):
+        got = tables[i].cpu().numpy().view(np.uint64)
+        assert np.array_equal(got, want[i % len(inst)]), (i, inst[i % len(inst)][2], len(inst[i % len(inst)][1]))
+
+
+def test_batch_modes_from_a_cache_file(cuda, tmp_path):
+    """Placements read from a cache file: global for some classes; 0, an earlier file's register placement, is the
+    shared table."""
+    inst = []
+    for i, (n, g) in enumerate([(5000, 4), (5000, 64), (70001, 65), (70001, 3000), (5000, 1), (70001, 1024)]):
+        comp = gen_np.compress(gen_np.generate(4100 + i, 0, n))
+        inst.append((comp, gen_np.group_keys_uniform(4100 + i, 0, n, g), g, 740000))
+    want = oracle_tables(inst)
+    arr, outs, keep = to_device(inst)
+    mode = [0, 2, 2, 1, 2, 0]
+    cache = tmp_path / "tune.txt"
+    lines = [f"mode {int(np.log2(len(k)))} {g} 10 {m}" for (c, k, g, d), m in zip(inst, mode)]
+    cache.write_text("# cache\n" + "\n".join(lines) + "\n")
+    stream = torch.cuda.current_stream().cuda_stream
+    desc, modes = run_batch(arr, len(inst), _lib.BatchOpts(1, 0, 0, 1, str(cache).encode()), stream)
+    assert modes == [m or 1 for m in mode] and desc.tuned_classes == 0
+    for i, (comp, keys, g, cutoff) in enumerate(inst):
+        assert np.array_equal(read(outs[i], g), want[i]), (i, g)

@@ -105,19 +105,21 @@ uint32_t q1::batch_engine(uint32_t mode, uint32_t num_groups) {
 
 namespace {
 
-// Relative cost of a row per engine (time per row of the group-key kernel on a B200 at 100% pass,
-// uniform keys, 64 groups = 1: 1.87 ms per 600 M rows, 1024 groups 2.26 ms, 4096 groups 2.79 ms): used
-// only to split the grid.
-constexpr double kEngineCost[kEngines] = {1.0, 1.21, 1.50, 8.4};
+// Relative cost of a row per engine, 64 groups = 1 (one instance of 10^8 rows, uniform keys: 64 groups
+// 212 us, 1024 groups 282 us): used only to split the grid.
+constexpr double kEngineCost[kEngines] = {1.0, 1.33, 1.6, 8.4};
 
 // Work items: every instance in pieces of `chunk` tiles or, with chunk 0, of falling size: an engine's
 // largest instances first, each piece three quarters of an equal share of the tiles its engine's CTAs still
-// have to do, down to 16 tiles (a CTA's share, if that is less). Every change of instance costs a CTA a
-// flush of its table (5 us for 64 groups' cells), so most of the work is in few large pieces, and the
-// small ones at the end even out the CTAs. 64 instances of 10^4 to 10^7 rows with 5, 64 and 1024 groups:
-// 291 us, 321 in pieces of one size; 64 of 1024 groups: 324 and 391.
+// have to do, down to 16 tiles (a CTA's share, if that is less). At every change of
+// instance a CTA's teams wait for each other and flush the table, so most of the work is in few large
+// pieces, and the small ones at the end even out the CTAs. 64 instances of 10^4 to 10^7 rows with 4, 64
+// and 1024 groups: 245 us; the best of pieces of one size (64 tiles) 274, falling from half of the share
+// 252, from a third 257, down to 8 tiles 263.
 void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32_t grid, int only,
-                std::vector<BatchItem>& items, uint32_t begin[kEngines + 1]) {
+                std::vector<BatchItem>& items, BatchParams& prm) {
+    uint32_t* const begin = prm.item_begin;
+    uint32_t max_groups[kEngines] = {};
     std::vector<uint32_t> of[kEngines];   // instances by engine, the largest first
     uint64_t tiles[kEngines] = {};
     auto tiles_of = [&](uint32_t i) { return (inst[i].rows + kBatchTileRows - 1) / kBatchTileRows; };
@@ -126,6 +128,7 @@ void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32
         if (only >= 0 && i != (uint32_t)only) continue;
         const uint32_t e = batch_engine(inst[i].mode, inst[i].num_groups);
         of[e].push_back(i);
+        max_groups[e] = std::max(max_groups[e], inst[i].num_groups);
         tiles[e] += tiles_of(i);
         total += (double)tiles_of(i) * kEngineCost[e];
     }
@@ -138,7 +141,8 @@ void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32
         for (uint32_t i : of[e]) {
             const uint64_t all = tiles_of(i);
             for (uint64_t t = 0; t < all;) {
-                const uint64_t most = chunk ? chunk : std::max(least, (uint64_t)((double)left / (1.33 * ctas)));
+                const uint64_t piece = chunk ? chunk : std::max(least, (uint64_t)((double)left / (1.33 * ctas)));
+                const uint64_t most = std::min<uint64_t>(piece, kBatchMaxItemTiles);
                 BatchItem it{};
                 it.instance = i;
                 it.first_tile = (uint32_t)t;
@@ -158,6 +162,7 @@ void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32
         items.insert(items.end(), per[e].begin(), per[e].end());
     }
     begin[kEngines] = (uint32_t)items.size();
+    batch_tables(max_groups, prm);
 }
 
 // At most `grid` CTAs, no more than items, and which queue each starts with: the engines' shares of the
@@ -182,7 +187,7 @@ void plan_roles(const std::vector<BatchItem>& items, const uint32_t begin[kEngin
 
 void q1::batch_plan(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32_t grid, std::vector<BatchItem>& items,
                     BatchParams& prm) {
-    plan_items(inst, n, chunk, grid, -1, items, prm.item_begin);
+    plan_items(inst, n, chunk, grid, -1, items, prm);
     plan_roles(items, prm.item_begin, grid, prm);
 }
 
@@ -205,7 +210,8 @@ struct q1_batch {
     bool overwrite = true;                   // each run overwrites the result tables
     bool shared_tables = false;              // result tables of two instances overlap: zeroed, then added to
     std::string cache;
-    DevMem d_inst, d_items, d_base, d_scratch, d_cursor;
+    DevMem d_inst, d_items, d_base;
+    DevMem d_scratch;   // accumulators of all groups, then the queue cursors
     ~q1_batch() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -218,7 +224,7 @@ struct q1_batch {
 // Items of every instance (only < 0) or of one instance, grouped by engine, and the grid roles.
 static void build_items(q1_batch* b, uint32_t chunk, int only = -1) {
     for (uint32_t i = 0; i < b->n; ++i) b->inst[i].mode = b->modes[i];
-    plan_items(b->inst.data(), b->n, chunk, b->grid, only, b->items, b->roles.item_begin);
+    plan_items(b->inst.data(), b->n, chunk, b->grid, only, b->items, b->roles);
     plan_roles(b->items, b->roles.item_begin, b->grid, b->roles);
     b->launch_grid = b->roles.grid;
 }
@@ -245,13 +251,12 @@ static q1_status upload(q1_batch* b) {
 static q1_status enqueue(q1_batch* b, cudaStream_t s) {
     if (b->overwrite && b->shared_tables)
         for (uint32_t i = 0; i < b->n; ++i) Q1_CUDA(cudaMemsetAsync(b->inst[i].out, 0, 96ull * b->inst[i].num_groups, s));
-    Q1_CUDA(cudaMemsetAsync(b->d_scratch.p, 0, b->total_groups * 64ull, s));
-    Q1_CUDA(cudaMemsetAsync(b->d_cursor.p, 0, 4 * kEngines, s));
+    Q1_CUDA(cudaMemsetAsync(b->d_scratch.p, 0, b->total_groups * 64ull + 4 * kEngines, s));
     if (!b->items.empty()) {
         BatchParams prm = b->roles;
         prm.inst = static_cast<const BatchInstanceDev*>(b->d_inst.p);
         prm.items = static_cast<const BatchItem*>(b->d_items.p);
-        prm.cursor = static_cast<uint32_t*>(b->d_cursor.p);
+        prm.cursor = static_cast<uint32_t*>(b->d_scratch.p) + 16 * b->total_groups;
         prm.status = b->di->status;
         Q1_CUDA(launch_batch(prm, s));
     }
@@ -354,8 +359,7 @@ q1_status q1_batch_create(const q1_batch_instance* in, uint32_t n, const q1_batc
     }
     if ((st = b->d_inst.alloc(sizeof(BatchInstanceDev) * std::max<uint32_t>(1, n))) != Q1_OK) return st;
     if ((st = b->d_base.alloc(sizeof(uint64_t) * (n + 1))) != Q1_OK) return st;
-    if ((st = b->d_scratch.alloc(b->total_groups * 64ull)) != Q1_OK) return st;
-    if ((st = b->d_cursor.alloc(4 * kEngines)) != Q1_OK) return st;
+    if ((st = b->d_scratch.alloc(b->total_groups * 64ull + 4 * kEngines)) != Q1_OK) return st;
     unsigned long long* scratch = static_cast<unsigned long long*>(b->d_scratch.p);
     for (uint32_t i = 0; i < n; ++i) b->inst[i].acc = scratch + 8ull * b->group_base[i];
     Q1_CUDA(cudaMemcpy(b->d_base.p, b->group_base.data(), sizeof(uint64_t) * (n + 1), cudaMemcpyHostToDevice));

@@ -9,6 +9,7 @@
 namespace q1 {
 
 constexpr uint32_t kBatchTileRows = 2048;
+constexpr uint32_t kBatchMaxItemTiles = 4096;   // 2^23 rows: what a table takes between flushes
 
 // Placement of one instance inside the batch kernel.
 enum BatchMode : uint32_t {
@@ -51,6 +52,8 @@ struct BatchParams {
     uint32_t item_begin[kEngines + 1];
     uint32_t role_end[kEngines];        // CTAs [role_end[e-1], role_end[e]) start with queue e
     uint32_t grid;                      // CTAs
+    uint32_t stages[kEngines];          // ring stages beside the engine's table
+    uint32_t table_words[kEngines];     // the table of the engine's largest instance, in 32-bit words
     uint32_t* cursor;                   // kEngines claim counters, zeroed before every launch
     uint32_t* status;
 };
@@ -61,7 +64,8 @@ struct BatchParams {
 void batch_plan(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32_t grid, std::vector<BatchItem>& items,
                 BatchParams& prm);
 
-uint32_t batch_smem_bytes();
+// Table sizes and ring stages, from the most groups an instance of each engine has.
+void batch_tables(const uint32_t max_groups[kEngines], BatchParams& prm);
 cudaError_t batch_prepare_launch();
 cudaError_t launch_batch(const BatchParams& prm, cudaStream_t stream);
 // Scratch of every instance into its result table: stored (every group, empty ones too) or added.

@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(tbl::kThreads, 1) tbl_parse_kernel(const char*
         const bool listed = !__any_sync(0xffffffffu, wl > kWarpList);   // (the same in every warp)
         if (control) {
             if (lane == 0) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                fence_proxy_async();
                 start_load(s == 0 ? kRing - 1 : s - 1, ticket);   // tile i - 1's stage
                 if (extra) starts[0] = off;
             }
