@@ -140,7 +140,7 @@ struct q1_ctx {
 
     // Aggregates.
     DevBuf daggs;
-    PinnedBuf haggs;
+    PinnedBuf haggs;   // the table, then the device's status word
 
     // Streamed mode: per-stream chunk buffers.
     DevBuf dchunks;
@@ -234,7 +234,7 @@ q1_status q1_open(q1_ctx** out, const q1_device_opts* opts) {
     Q1_CUDA(cudaEventCreateWithFlags(&ctx->ev_zeroed, cudaEventDisableTiming));
     st = ctx->daggs.alloc(Q1_NUM_POTENTIAL_GROUPS * Q1_NUM_AGGREGATES * 16);
     if (st != Q1_OK) return st;
-    st = ctx->haggs.alloc(Q1_NUM_POTENTIAL_GROUPS * Q1_NUM_AGGREGATES * 16);
+    st = ctx->haggs.alloc(Q1_NUM_POTENTIAL_GROUPS * Q1_NUM_AGGREGATES * 16 + 16);
     if (st != Q1_OK) return st;
     int threads = opts ? opts->cpu_threads : 0;
     if (threads <= 0) {
@@ -825,13 +825,25 @@ static q1_status run_once(q1_ctx* ctx, const q1_params* prm, Agg128* total, doub
             if (e != cudaSuccess) st = cuda_error(e, "stream join");
         }
     }
+    // The status word comes back on the stream, behind the aggregates: a blocking copy of it after the
+    // synchronisation made the smallest query take 62 us instead of 52. Only a word that is set is read
+    // again, and cleared.
+    volatile uint32_t* const hstatus = reinterpret_cast<uint32_t*>(ctx->haggs.p + ctx->daggs.n);
+    bool status_read = false;
     if (st == Q1_OK) {
+        *hstatus = 0;
         cudaError_t e = cudaEventRecord(ctx->ev_stop, s0);
         if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->haggs.p, ctx->daggs.p, ctx->daggs.n, cudaMemcpyDeviceToHost, s0);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(ctx->haggs.p + ctx->daggs.n, ctx->di->status, 4, cudaMemcpyDeviceToHost, s0);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
         if (e != cudaSuccess) st = cuda_error(e, "aggregate read-back");
+        status_read = e == cudaSuccess;
     }
-    q1_status dev_st = q1_sync_check(s0);
-    if (st == Q1_OK) st = dev_st;
+    if (!status_read || *hstatus) {
+        const q1_status dev_st = q1_sync_check(s0);
+        if (st == Q1_OK) st = dev_st;
+    }
     if (cpu_job) {
         ctx->queue.close();
         if (!ctx->pool->wait() && st == Q1_OK) st = set_error(Q1_ERR_CPU_WORKER, "CPU worker failed: " + ctx->pool->error());
