@@ -188,3 +188,44 @@ def test_device_generator_matches_host(cuda):
         else:
             assert np.array_equal(out["returnflag"].cpu().numpy().view(np.uint32), ref["returnflag"])
             assert np.array_equal(out["linestatus"].cpu().numpy().view(np.uint32), ref["linestatus"])
+
+
+@pytest.mark.parametrize("placement", PLACEMENTS)
+@pytest.mark.parametrize("packing", ["pair", "sep"])
+@pytest.mark.parametrize("use_filter", [False, True])
+def test_wide_kernel_edges(cuda, placement, packing, use_filter):
+    """Rows per CTA around the line from which the kernels of more warps run (131,072), whole and ragged tiles of both
+    kernels, tails of several rows a thread and spread over the CTAs."""
+    most = 3 * 131072 + 5760
+    cols = gen_np.generate(35, 0, most)
+    comp = gen_np.compress(cols, packing)
+    cutoff = 729906
+    if use_filter:
+        comp["filter"] = gen_np.filter_bitmap(comp["shipdate"], cutoff)
+    c, keep = device_compressed(comp)
+    stream = torch.cuda.current_stream().cuda_stream
+    line = 131072
+    for blocks, sizes in [(1, [line - 1, line, line + 1, 23 * 5760 - 1, 23 * 5760, 23 * 5760 + 1, 24 * 5760 - 1]),
+                          (2, [2 * line - 1, 2 * line, 46 * 5760 + 961, 47 * 5760 - 1]), (3, [3 * line + 5759]),
+                          (0, [5759, 5760 * 2 + 481, most])]:
+        for rows in sizes:
+            buf = aggs_buffer()
+            q.launch_compressed(placement, c, rows, cutoff, use_filter, buf.data_ptr(), stream,
+                                config=_lib.LaunchConfig(0, 0, blocks))
+            q.sync_check(stream)
+            want = O.q1_uncompressed({k: v[:rows] for k, v in cols.items()}, cutoff)[0]
+            assert np.array_equal(read(buf), want), (blocks, rows)
+
+
+@pytest.mark.parametrize("placement", PLACEMENTS)
+@pytest.mark.parametrize("rows", [1407, 1408, 1409, 1408 * 148, 1408 * 148 * 2 + 1407, 1408 * 149 + 353])
+def test_uncompressed_tile_edges(cuda, placement, rows):
+    cols = gen_np.generate(36, 0, rows)
+    keep = {k: dev(v) for k, v in cols.items()}
+    c = _lib.Columns(*(keep[k].data_ptr() for k in ["shipdate", "discount", "extendedprice", "tax", "quantity",
+                                                    "returnflag", "linestatus"]))
+    buf = aggs_buffer()
+    stream = torch.cuda.current_stream().cuda_stream
+    q.launch_uncompressed(placement, c, rows, 729906, buf.data_ptr(), stream)
+    q.sync_check(stream)
+    assert np.array_equal(read(buf), O.q1_uncompressed(cols, 729906)[0])

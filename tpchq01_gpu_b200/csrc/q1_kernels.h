@@ -27,21 +27,36 @@ enum ScanPlacement : int {
 
 // Consumer warps per CTA (plus one producer warp), per input layout, as measured on the 600 M-row
 // table (100 M uncompressed). More warps per SM sub-partition hide more of the decode's issue latency
-// where the registers allow. 12 warps leave 128 registers a thread (13 warps, which the allocator
-// rounds up to 16 warps' worth): the compressed layouts' kernels fit, the separate-flag ones by
-// keeping only four groups' planes in registers (A/O and R/O go to the CTA's shared table). Pair
-// layout 0.909 -> 0.871 ms, separate flags 1.129 ms with 8 warps and six planes, 1.044 with 10, 0.980
-// with 12. The uncompressed layout runs 10: it needs up to 168 registers (per-thread 0.625 -> 0.600 ms
-// although one register spills; shared 0.670 -> 0.548).
-template <int L, int P>
+// where the registers allow. The register file is given out four warps at a time: 15 consumer warps (or 12:
+// 13 warps take the room of 16) leave 128 registers a thread, and the compressed layouts' kernels fit, the
+// separate-flag ones by keeping only four groups' planes in registers (A/O and R/O go to the CTA's shared
+// table). Separate flags took 1.129 ms with 8 warps and six planes, 1.044 with 10, 0.980 with 12.
+// kWide, 15 warps: large tables (scan_is_wide): 600 M rows, pair 871 -> 832 us, separate flags
+// 1005 -> 920, with filter 1205 -> 1084; 14 warps 886, 1000, 1156. Their larger tile (a small table is a
+// few tiles per CTA) costs 60,175 rows 2 us. The shared placement's tables leave no room for it.
+// The uncompressed layout and in_registers over separate flags need up to 168 registers: 11 warps with
+// the producer's 12 (10: uncompressed 100 M rows per-thread 582 us instead of 536; the shared
+// placement's table again leaves no room).
+constexpr bool scan_needs_168(int L, int P) {
+    return L == kLayUncomp || ((L == kLaySep || L == kLaySepFilter) && P == kPlaceInRegisters);
+}
+constexpr bool scan_has_wide(int L, int P) { return !scan_needs_168(L, P) && P != kPlaceSharedMemPerThread; }
+template <int L, int P, bool kWide>
 inline constexpr uint32_t kConsumerWarps =
-    L == kLayUncomp || ((L == kLaySep || L == kLaySepFilter) && P == kPlaceInRegisters) ? 10u : 12u;
+    scan_needs_168(L, P) ? (P == kPlaceSharedMemPerThread ? 10u : 11u) : (kWide && scan_has_wide(L, P) ? 15u : 12u);
+// Rows of the launch for each CTA it may have from which on a wide kernel runs (148 CTAs: 12 M rows take
+// 27.1 us with 12 warps and 28.1 with 15, 25 M rows 46.9 and 45.9; separate flags with filter 35.1 and
+// 35.0, 60.9 and 59.1).
+inline constexpr uint64_t kWideRowsPerCta = 1u << 17;
+constexpr bool scan_is_wide(int L, int P, uint64_t rows, uint32_t ctas) {
+    return scan_has_wide(L, P) && rows >= kWideRowsPerCta * ctas;
+}
 // Rows per tile (one bulk copy per column per tile): a multiple of 128, so that every column slice
 // of every tile starts on a 16-byte boundary down to 1-bit columns, and of the consumer threads x
 // the rows of a step, so that a tile's steps divide evenly among the consumer threads.
-template <int L, int P>
+template <int L, int P, bool kWide>
 inline constexpr uint32_t kTileRows =
-    (L == kLayUncomp ? 128u : 384u) * kConsumerWarps<L, P>;
+    (L == kLayUncomp ? 128u : 384u) * kConsumerWarps<L, P, kWide>;
 // Shared-memory ring depth: 3 where the shared placement's tables take the room of the fourth.
 template <int L, int P>
 inline constexpr uint32_t kStages = (P == kPlaceSharedMemPerThread && L != kLayPair && L != kLayPairFilter) ? 3u : 4u;
@@ -72,7 +87,7 @@ struct ScanParams {
 // Launch the scan kernel for one layout x placement. max_blocks <= 0: one CTA per SM.
 cudaError_t launch_scan(int layout, int placement, const ScanParams& prm, int sm_count, int max_blocks,
                         cudaStream_t stream);
-// Rows per tile of the layout x placement (a multiple of 128).
+// Rows per tile of the layout x placement's kernel for small tables (a multiple of 128).
 uint32_t scan_tile_rows(int layout, int placement);
 // Grid size launch_scan uses for `rows` rows of the layout x placement.
 uint32_t scan_grid_blocks(int layout, int placement, uint64_t rows, int sm_count, int max_blocks);

@@ -28,6 +28,8 @@
 // products overflow, which the reference's KernelHyPer reports through handle_overflow
 // (cpu/kernel_hyper.hpp:65-91), sets kStatusDomain.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 #include <stdint.h>
 
 #include "q1_common.cuh"
@@ -179,7 +181,7 @@ struct AccPerThread {
     // With the six (returnflag, linestatus) groups of the separate flag layout, A/O and R/O (codes
     // 1 and 5) need a receipt date before the ship date and do not occur in TPC-H data: their rows
     // go straight into the CTA's 128-bit shared table (red) behind one warp vote, so that only the
-    // four other groups' planes take registers (a kernel of 128 registers a thread, 12 warps).
+    // four other groups' planes take registers (a kernel of 128 registers a thread).
     static constexpr bool kCold = (G == 6) && !kWideQty;
     static constexpr int kPlanes = kWideQty ? 1 : (kCold ? 4 : G);
     GroupRegs g[kWideQty ? G : 1];      // row-wise path (uncompressed layout)
@@ -704,13 +706,13 @@ __device__ __forceinline__ void process_row_global(const ScanParams& prm, uint64
 // The kernel
 // ---------------------------------------------------------------------------------------------
 
-template <int L, int P>
-__global__ void __launch_bounds__((kConsumerWarps<L, P> + 1) * 32, 1)
+template <int L, int P, bool kWide>
+__global__ void __launch_bounds__((kConsumerWarps<L, P, kWide> + 1) * 32, 1)
 q1_scan_kernel(const __grid_constant__ ScanParams prm) {
     using T = LayoutTraits<L>;
-    constexpr uint32_t R = kTileRows<L, P>;
+    constexpr uint32_t R = kTileRows<L, P, kWide>;
     constexpr uint32_t S = kStages<L, P>;
-    constexpr uint32_t W = kConsumerWarps<L, P>;
+    constexpr uint32_t W = kConsumerWarps<L, P, kWide>;
     constexpr uint32_t kStage = stage_bytes<L>(R);
     constexpr int G = T::kCodes;
     static_assert(kStage % 16 == 0, "stage must keep 16-byte alignment");
@@ -781,28 +783,31 @@ q1_scan_kernel(const __grid_constant__ ScanParams prm) {
         // The in_registers and global placements sum a warp's buffers in 64 bits: at most 2048 rows
         // a lane of charges below 100 (2^32 - 1) 355 < 2^47.2 stays below 2^64.
         static_assert(kRowsPerThreadTile * kCombineTiles <= 2048u, "warp sums must stay below 2^64");
-        bool ok = true;
+        // Tail rows [num_tiles * R, rows), a row a thread, while the first tiles are on their way: spread over the
+        // CTAs, those with a tile less first. (One CTA taking all of them after its tiles: up to R / (32 W)
+        // trips to global memory one after the other: 700,000 rows 14.5 us instead of 10.4.)
+        {
+            const uint32_t extra = (uint32_t)(num_tiles % gridDim.x);
+            const uint32_t turn = blockIdx.x >= extra ? blockIdx.x - extra : blockIdx.x + gridDim.x - extra;
+            uint64_t i = num_tiles * R + (uint64_t)turn * (W * 32);
+            if (i < prm.rows) {
+                for (; i < prm.rows; i += (uint64_t)gridDim.x * (W * 32))
+                    if (i + ctid < prm.rows) process_row_global<L>(prm, i + ctid, acc, bad);
+                acc.tile_done(prm, lane);
+            }
+        }
         uint32_t k = 0;
         for (uint64_t t = blockIdx.x; t < num_tiles; t += gridDim.x, ++k) {
             const uint32_t s = k % S;
             // Every lane waits (acquiring the bulk-copy writes); the warp proceeds only together.
             const bool landed = mbar_wait(smem_addr(&full_bar[s]), (k / S) & 1u, prm.status);
-            if (!__all_sync(0xffffffffu, landed)) {
-                ok = false;
-                break;
-            }
+            if (!__all_sync(0xffffffffu, landed)) break;
             const uint32_t base = ring + s * kStage;
 #pragma unroll
             for (uint32_t it = 0; it < kSteps / (W * 32); ++it)
                 process_step<L, R>(prm, base, ctid + it * (W * 32), prm.cutoff, lut, acc, bad);
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_addr(&empty_bar[s]));
-            acc.tile_done(prm, lane);
-        }
-        // Tail rows [num_tiles * R, rows): handled by the CTA next in the round robin.
-        if (ok && blockIdx.x == (uint32_t)(num_tiles % gridDim.x)) {
-            const uint64_t first = num_tiles * R;
-            for (uint64_t i = first + ctid; i < prm.rows; i += W * 32) process_row_global<L>(prm, i, acc, bad);
             acc.tile_done(prm, lane);
         }
         acc.finish(prm, lane);
@@ -866,20 +871,32 @@ q1_scan_kernel(const __grid_constant__ ScanParams prm) {
 // Host launch table
 // ---------------------------------------------------------------------------------------------
 
-template <int L, int P>
-static cudaError_t launch_one(const ScanParams& prm, int sm_count, int max_blocks, cudaStream_t stream) {
-    constexpr uint32_t R = kTileRows<L, P>;
+template <int L, int P, bool kWide>
+static cudaError_t launch_sized(const ScanParams& prm, int sm_count, int max_blocks, cudaStream_t stream) {
+    constexpr uint32_t R = kTileRows<L, P, kWide>;
     constexpr uint32_t S = kStages<L, P>;
-    constexpr uint32_t W = kConsumerWarps<L, P>;
+    constexpr uint32_t W = kConsumerWarps<L, P, kWide>;
     constexpr int G = LayoutTraits<L>::kCodes;
     constexpr uint32_t dyn =
         S * stage_bytes<L>(R) + (P == kPlaceSharedMemPerThread ? 8u * Entry<L == kLayUncomp>::kWords * G * W * 32u : 0u);
     static_assert(dyn + sizeof(ulonglong2) * W * G * kNumAggs + 2048 <= 227 * 1024, "ring and tables beside the static shared memory");
-    cudaError_t e = cudaFuncSetAttribute(q1_scan_kernel<L, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    cudaError_t e = cudaFuncSetAttribute(q1_scan_kernel<L, P, kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = scan_grid_blocks(L, P, prm.rows, sm_count, max_blocks);
-    q1_scan_kernel<L, P><<<blocks, (W + 1) * 32, dyn, stream>>>(prm);
+    q1_scan_kernel<L, P, kWide><<<blocks, (W + 1) * 32, dyn, stream>>>(prm);
     return cudaGetLastError();
+}
+
+static uint32_t most_ctas(int sm_count, int max_blocks) {   // one CTA per SM (shared-memory bound)
+    return max_blocks > 0 && max_blocks < sm_count ? (uint32_t)max_blocks : (uint32_t)sm_count;
+}
+
+template <int L, int P>
+static cudaError_t launch_one(const ScanParams& prm, int sm_count, int max_blocks, cudaStream_t stream) {
+    if constexpr (scan_has_wide(L, P))
+        if (scan_is_wide(L, P, prm.rows, most_ctas(sm_count, max_blocks)))
+            return launch_sized<L, P, true>(prm, sm_count, max_blocks, stream);
+    return launch_sized<L, P, false>(prm, sm_count, max_blocks, stream);
 }
 
 template <int L>
@@ -911,46 +928,48 @@ namespace {
 struct Geometry {
     uint32_t warps, tile_rows;
 };
-template <int L>
+template <int L, bool kWide>
 Geometry geometry_of(int placement) {
     switch (placement) {
-        case kPlaceInRegisters: return {kConsumerWarps<L, kPlaceInRegisters>, kTileRows<L, kPlaceInRegisters>};
+        case kPlaceInRegisters:
+            return {kConsumerWarps<L, kPlaceInRegisters, kWide>, kTileRows<L, kPlaceInRegisters, kWide>};
         case kPlaceInRegistersPerThread:
-            return {kConsumerWarps<L, kPlaceInRegistersPerThread>, kTileRows<L, kPlaceInRegistersPerThread>};
-        case kPlaceLocalMem: return {kConsumerWarps<L, kPlaceLocalMem>, kTileRows<L, kPlaceLocalMem>};
+            return {kConsumerWarps<L, kPlaceInRegistersPerThread, kWide>, kTileRows<L, kPlaceInRegistersPerThread, kWide>};
+        case kPlaceLocalMem: return {kConsumerWarps<L, kPlaceLocalMem, kWide>, kTileRows<L, kPlaceLocalMem, kWide>};
         case kPlaceSharedMemPerThread:
-            return {kConsumerWarps<L, kPlaceSharedMemPerThread>, kTileRows<L, kPlaceSharedMemPerThread>};
-        default: return {kConsumerWarps<L, kPlaceGlobal>, kTileRows<L, kPlaceGlobal>};
+            return {kConsumerWarps<L, kPlaceSharedMemPerThread, kWide>, kTileRows<L, kPlaceSharedMemPerThread, kWide>};
+        default: return {kConsumerWarps<L, kPlaceGlobal, kWide>, kTileRows<L, kPlaceGlobal, kWide>};
     }
 }
-Geometry geometry(int layout, int placement) {
+template <int L>
+Geometry geometry_of(int placement, bool wide) {
+    return wide ? geometry_of<L, true>(placement) : geometry_of<L, false>(placement);
+}
+Geometry geometry(int layout, int placement, bool wide) {
     switch (layout) {
-        case kLayPair: return geometry_of<kLayPair>(placement);
-        case kLayPairFilter: return geometry_of<kLayPairFilter>(placement);
-        case kLaySep: return geometry_of<kLaySep>(placement);
-        case kLaySepFilter: return geometry_of<kLaySepFilter>(placement);
-        default: return geometry_of<kLayUncomp>(placement);
+        case kLayPair: return geometry_of<kLayPair>(placement, wide);
+        case kLayPairFilter: return geometry_of<kLayPairFilter>(placement, wide);
+        case kLaySep: return geometry_of<kLaySep>(placement, wide);
+        case kLaySepFilter: return geometry_of<kLaySepFilter>(placement, wide);
+        default: return geometry_of<kLayUncomp>(placement, wide);
     }
 }
 
 }  // namespace
 
 uint64_t scan_max_rows_per_launch(int layout, int placement, uint32_t grid) {
-    const Geometry g = geometry(layout, placement);
+    const Geometry g = geometry(layout, placement, false);   // the fewer threads
     uint64_t n = (uint64_t)grid * g.warps * 32ull * 32768ull;   // every consumer thread sums its own rows
     if (n > (1ull << 31)) n = 1ull << 31;
     return n / g.tile_rows * g.tile_rows;
 }
 
 uint32_t scan_grid_blocks(int layout, int placement, uint64_t rows, int sm_count, int max_blocks) {
-    const uint64_t tiles = rows / scan_tile_rows(layout, placement);
-    uint64_t blocks = tiles ? tiles : 1;
-    uint64_t cap = (uint64_t)sm_count;  // one CTA per SM (shared-memory bound)
-    if (max_blocks > 0 && (uint64_t)max_blocks < cap) cap = (uint64_t)max_blocks;
-    if (blocks > cap) blocks = cap;
-    return (uint32_t)blocks;
+    const uint32_t cap = most_ctas(sm_count, max_blocks);
+    const uint64_t tiles = rows / geometry(layout, placement, scan_is_wide(layout, placement, rows, cap)).tile_rows;
+    return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(tiles, 1), cap);
 }
 
-uint32_t scan_tile_rows(int layout, int placement) { return geometry(layout, placement).tile_rows; }
+uint32_t scan_tile_rows(int layout, int placement) { return geometry(layout, placement, false).tile_rows; }
 
 }  // namespace q1
