@@ -187,36 +187,50 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + kTeams) 
     __syncthreads();
 
     if (warp >= W) {
-        // a producer warp per team: its tiles, into every kTeams-th stage
-        if (lane == 0) {
+        // a producer warp per team: its tiles, into every kTeams-th stage. Beside the larger tables lane c
+        // issues column c's copies (100 M rows: 600 groups 238 -> 232 us, 1000 273 -> 264, 4096 358 -> 349);
+        // elsewhere one lane issues all six (register planes, 4 groups 206 -> 217 with a lane per column; 64
+        // groups 200 either way).
+        constexpr bool kLanes = kTab == kTableCube || kTab == kTableSlots;
+        if (kLanes || lane == 0) {
             const uint64_t pol = policy_evict_first();
+            const uint32_t c = lane < 6 ? lane : 5;
+            const uint32_t dst = ring + ka::TileLayout<R>::col_off((int)c), bytes = ka::TileLayout<R>::col_bytes((int)c);
             // stage s and phase ph of the tile, stepped rather than divided (S is a launch parameter)
             uint32_t s = warp - W, ph = 0;
-            const uint64_t step = (uint64_t)kTeams * gridDim.x;
-            uint64_t t = blockIdx.x + (uint64_t)(warp - W) * gridDim.x;
-            for (; t < num_tiles; t += step) {
-                if (!mbar_wait(smem_addr(&empty_bar[s]), ph ^ 1u, prm.status)) break;
-                const uint32_t fb = smem_addr(&full_bar[s]);
-                mbar_arrive_expect_tx(fb, kStage);
-#pragma unroll
-                for (int c = 0; c < 6; ++c)
-                    bulk_g2s(ring + s * kStage + ka::TileLayout<R>::col_off(c),
-                             prm.col[c] + t * (uint64_t)ka::TileLayout<R>::col_bytes(c),
-                             ka::TileLayout<R>::col_bytes(c), fb, pol);
+            auto next = [&]() {
                 s += kTeams;
                 if (s >= S) {
                     s -= S;
                     ph ^= 1u;
                 }
+            };
+            const uint64_t step = (uint64_t)kTeams * gridDim.x;
+            uint64_t t = blockIdx.x + (uint64_t)(warp - W) * gridDim.x;
+            const uint8_t* src = prm.col[c] + t * bytes;
+            for (; t < num_tiles; t += step, src += step * bytes) {
+                const bool empty = mbar_wait(smem_addr(&empty_bar[s]), ph ^ 1u, prm.status);
+                const uint32_t fb = smem_addr(&full_bar[s]);
+                if constexpr (kLanes) {
+                    if (!__all_sync(0xffffffffu, empty)) break;
+                    if (lane == 0) mbar_arrive_expect_tx(fb, kStage);
+                    __syncwarp();
+                    if (lane < 6) bulk_g2s(dst + s * kStage, src, bytes, fb, pol);
+                } else {
+                    if (!empty) break;
+                    mbar_arrive_expect_tx(fb, kStage);
+#pragma unroll
+                    for (int k = 0; k < 6; ++k)
+                        bulk_g2s(ring + s * kStage + ka::TileLayout<R>::col_off(k),
+                                 prm.col[k] + t * (uint64_t)ka::TileLayout<R>::col_bytes(k),
+                                 ka::TileLayout<R>::col_bytes(k), fb, pol);
+                }
+                next();
             }
             // Never leave with copies in flight: wait for the last tiles issued to land.
             for (uint32_t i = 0; i < S; i += kTeams) {
                 mbar_wait(smem_addr(&full_bar[s]), ph ^ 1u, prm.status);
-                s += kTeams;
-                if (s >= S) {
-                    s -= S;
-                    ph ^= 1u;
-                }
+                next();
             }
         }
     } else {
@@ -309,11 +323,16 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + kTeams) 
                     ph ^= 1u;
                 }
             }
-            // the rows after the last full tile, by one CTA straight from global memory
-            if (ok && blockIdx.x == (uint32_t)(num_tiles % gridDim.x) && num_tiles * R < prm.rows) {
+            // the rows after the last full tile, straight from global memory: spread over the CTAs, those with
+            // a tile less first (register planes, whose loop that made 2% slower: by one CTA)
+            constexpr bool kSpread = P != kPlaceInRegistersPerThread;
+            const uint32_t extra = (uint32_t)(num_tiles % gridDim.x);
+            const uint32_t turn = blockIdx.x >= extra ? blockIdx.x - extra : blockIdx.x + gridDim.x - extra;
+            uint64_t i0 = kSpread || turn == 0 ? num_tiles * R + (uint64_t)turn * (W * 32) : prm.rows;
+            if (ok && i0 < prm.rows) {
                 if (flushes && rows_since + kTeams * R > ka::kTableFlushRows) table_flush();
                 // every lane runs every round (the table engines vote across the warp)
-                for (uint64_t i0 = num_tiles * R; i0 < prm.rows; i0 += W * 32) {
+                for (; i0 < prm.rows; i0 += (uint64_t)(kSpread ? gridDim.x : 1u) * (W * 32)) {
                     const uint64_t i = i0 + ctid;
                     add(i < prm.rows ? ka::load_row(prm.col, i, prm.cutoff, bad) : ka::empty_quad());
                 }
