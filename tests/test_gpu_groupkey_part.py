@@ -17,6 +17,7 @@ import torch
 
 import gen_np
 import tpchq01_gpu_b200 as q
+from oracle import py_oracle as O
 from tpchq01_gpu_b200 import _lib
 from test_gpu_groupkey import check, device_cols, keys_for, run_gpu, widen, zipf_cdf
 
@@ -172,3 +173,39 @@ def test_one_key_many_rows(table, monkeypatch, num_groups, blocks):
     for forced in ["single", "partitioned"] if num_groups > 4096 else ["single"]:
         monkeypatch.setenv("Q1_GROUPKEY_PATH", forced)
         check(comp, keys, num_groups, 730089, run_gpu(c, keys, num_groups, "shared_mem_per_thread", 730089, blocks))
+
+
+@pytest.mark.parametrize("num_groups,rows", [(3000, (1 << 25) - 1), (3000, 1 << 25), (4096, (1 << 25) + 1),
+                                             (4097, (3 << 19) - 1), (4097, 3 << 19), (65536, (3 << 19) + 1)])
+@pytest.mark.parametrize("dist", ["uniform", "zipf"])
+def test_path_choice_lines(table, monkeypatch, num_groups, rows, dist):
+    """Rows around the lines from which the path is chosen on the device: the table over and over, for cutoffs that
+    let no row, few rows and all rows pass."""
+    monkeypatch.delenv("Q1_GROUPKEY_PATH", raising=False)
+    comp, _, _ = table
+    keys, _ = keys_for(num_groups, dist)
+    whole, rest = divmod(rows, ROWS)
+
+    def repeat(t, n):
+        return torch.cat([t.view(-1, n // ROWS).repeat(whole, 1).view(-1), t[: rest * (n // ROWS)]])
+
+    names = ["shipdate", "quantity", "discount", "tax", "extendedprice"]
+    dev = {k: torch.from_numpy(np.ascontiguousarray(comp[k]).view(np.uint8).copy()).cuda() for k in names}
+    dev = {k: repeat(t, t.numel()) for k, t in dev.items()}
+    dkeys = torch.from_numpy(keys.astype(np.uint32).view(np.uint8).copy()).cuda()
+    dkeys = repeat(dkeys, dkeys.numel())
+    c = _lib.CompressedColumns()
+    for k in names:
+        setattr(c, k, dev[k].data_ptr())
+    scratch = torch.zeros(int(q.lib().q1_groupkey_scratch_bytes(num_groups)) // 8 + 2, dtype=torch.int64, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    for cutoff in [727000, 727600, 730089]:
+        out = torch.zeros(num_groups * 12, dtype=torch.int64, device="cuda")
+        _lib.check(q.lib().q1_launch_groupkey(3, ctypes.byref(c), dkeys.data_ptr(), num_groups, rows, cutoff, None,
+                                              scratch.data_ptr(), out.data_ptr(), stream))
+        _lib.check(q.lib().q1_sync_check(stream))
+        got = q.decode_aggregates(out.cpu().numpy().view(np.uint64), num_groups)
+        part = {k: (v[:rest] if isinstance(v, np.ndarray) and len(v) == ROWS else v) for k, v in comp.items()}
+        want = whole * q.decode_aggregates(O.q1_groupkey(comp, keys, num_groups, cutoff)[0], num_groups)
+        want = want + q.decode_aggregates(O.q1_groupkey(part, keys[:rest], num_groups, cutoff)[0], num_groups)
+        assert np.array_equal(got, want), cutoff

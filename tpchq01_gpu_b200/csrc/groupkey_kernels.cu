@@ -17,9 +17,10 @@
 //                            kernel with keys < 4096 in
 //                            slots and larger keys reduced straight into the global
 //                            accumulators, or the two-pass partitioned path of
-//                            groupkey_part.cu; above 256 groups the path (and the global
-//                            placement's, when few rows pass over spread keys) is chosen on the
-//                            device from a sample of the rows (q1_groupkey_choose)
+//                            groupkey_part.cu; above 1024 groups the path is chosen on the
+//                            device from a sample of the rows of a large table
+//                            (q1_groupkey_choose), which may be the global placement's, when few
+//                            rows pass over spread keys
 //   global                   every passing row reduces into the global accumulators
 //
 // Accumulators live in scratch memory (per launch, zeroed first): per group 8 x u64 (see
@@ -49,16 +50,16 @@ namespace gk {
 
 constexpr uint32_t kMaxStages = 10;   // ring stages
 constexpr uint32_t kWideSlots = 4096; // slot-table keys of the single-pass kernel
-constexpr uint32_t kChooseAbove = 256; // the shared placement's path is chosen on the device above
 constexpr uint32_t kMaxDynSmem = 227 * 1024;
-// Consumer warps. Register planes: 8, or 12 for four groups' planes on a large table (kWide: their 110
-// registers a thread fit the 128 that 13 warps leave, and a third warp per scheduler hides more of the
-// planes' issue latency: 600 M rows 1.49 -> 1.24 ms). Global placement: 16. Shared tables: 24, whose
-// atomics need many warps in flight to hide their latency (64 groups, 100 M rows: 237 us with 16, 199
-// with 24).
+// Consumer warps. Register planes: 8, or 15 for four groups' planes on a large table (kWide: their 115
+// registers a thread fit the 128 that 16 warps leave, and four warps per scheduler hide more of the
+// planes' issue latency: 100 M rows 206 us with 12, 188 with 15). Eight groups' planes take 168 registers,
+// which 11 consumer warps would leave too (100 M rows 322 -> 316 us, but 6 M 27.4 -> 28.8). Global
+// placement: 16. Shared tables: 24, whose atomics need many warps in flight to hide their latency (64
+// groups, 100 M rows: 237 us with 16, 199 with 24).
 template <int P, int NG, bool kWide>
 __host__ __device__ constexpr uint32_t consumer_warps() {
-    return P == kPlaceInRegistersPerThread ? ((NG <= 4 && kWide) ? 12u : 8u)
+    return P == kPlaceInRegistersPerThread ? (kWide ? 15u : 8u)
                                            : (P == kPlaceSharedMemPerThread ? 24u : 16u);
 }
 // Rows per tile: two quads of a tile for every consumer thread of the register planes (at most 8
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + kTeams) 
     __shared__ uint64_t warp_rec[P == kPlaceInRegistersPerThread ? W : 1][kRegValues];
     __shared__ __align__(16) unsigned long long wide[2 * kRegValues];
     // a path chosen on the device: this kernel (its table, or no table: the global path) unless partitioned
-    constexpr bool kChosen = kTab == kTableCube || kTab == kTableSlots;
+    constexpr bool kChosen = kTab == kTableSlots;
     bool no_table = false;
     if (kChosen && prm.mode) {
         const uint32_t mode = *prm.mode;
@@ -419,12 +420,18 @@ static cudaError_t launch_table(uint32_t table, uint32_t teams, const GroupKeyPa
 }
 
 static uint64_t acc_bytes(uint32_t num_groups) { return 64ull * num_groups; }
-// The shared placement chooses its path on the device above 256 groups.
-static bool chosen_on_device(int placement, uint32_t num_groups) {
-    return placement == kPlaceSharedMemPerThread && num_groups > gk::kChooseAbove;
+// Whether the shared placement's path is chosen on the device, by rows of the launch; elsewhere it is the
+// single pass. The choice costs a launch (10 us, 20 us before the partition's kernels) and the global path
+// gains little on the tables: with fewer than 2% of the rows passing, 1000 groups, 60 M rows 154 us against
+// 145 with the table; 4096 groups 25 M rows 81 and 80, 60 M rows 153 and 163. Above 4096 groups the
+// partition gains nothing on small tables: 65,536 uniform groups, all rows passing, 1.0 M rows 78 us
+// chosen, 58 in a single pass, 2.0 M rows 83 and 91 (Zipf keys 81 and 58).
+static bool chosen_on_device(int placement, uint32_t num_groups, uint64_t rows) {
+    if (placement != kPlaceSharedMemPerThread || num_groups <= ka::kCubeMaxGroups) return false;
+    return rows >= (num_groups >= groupkey_part_min_groups() ? 3ull << 19 : 1ull << 25);
 }
 
-// Chooses the path of the shared placement for more than 256 groups from 8192 evenly spaced
+// Chooses the path of the shared placement for more than 1024 groups from 8192 evenly spaced
 // sample rows and writes it to *mode (every path gives identical results):
 //   kModeGlobalPath   every passing row straight into the global accumulators, when fewer than
 //                     2% of the rows pass and no key occurs more than 3 times among the sampled
@@ -509,9 +516,7 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
     cudaError_t e = direct ? cudaSuccess : cudaMemsetAsync(scratch, 0, acc_bytes(num_groups), stream);
     if (e != cudaSuccess) return e;
     uint8_t* workspace = reinterpret_cast<uint8_t*>(scratch) + ((acc_bytes(num_groups) + 255) & ~255ull);
-    const bool choose = chosen_on_device(placement, num_groups);
     const bool part = num_groups >= groupkey_part_min_groups();
-    uint32_t* mode = choose ? reinterpret_cast<uint32_t*>(workspace + groupkey_part_mode_offset()) : nullptr;
     // Q1_GROUPKEY_PATH=single|partitioned|global overrides the sample-based choice (tests, tuning)
     uint32_t force = 0;
     if (const char* env = std::getenv("Q1_GROUPKEY_PATH")) {
@@ -529,6 +534,10 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
         prm.cutoff = cutoff_rel;
         prm.num_groups = num_groups;
         const uint32_t table = gk::table_kind(placement, num_groups);
+        uint32_t* mode = nullptr;   // the path, when it is not the single pass throughout
+        if (table == gk::kTableSlots && (force ? force != kModeSinglePass : chosen_on_device(placement, num_groups, n)))
+            mode = reinterpret_cast<uint32_t*>(workspace + groupkey_part_mode_offset());
+        const bool global_cells = force == kModeGlobalPath && table == gk::kTableCube && num_groups > 256;
         prm.acc = scratch;
         prm.out = out;
         prm.status = status;
@@ -554,7 +563,8 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
                 break;
             }
             case kPlaceSharedMemPerThread:
-                e = launch_table(table, gk::table_teams(table, num_groups), prm, sm_count, max_blocks, stream);
+                e = global_cells ? launch_gk<kPlaceGlobal, 4>(prm, sm_count, max_blocks, stream)
+                                 : launch_table(table, gk::table_teams(table, num_groups), prm, sm_count, max_blocks, stream);
                 break;
             case kPlaceGlobal: e = launch_gk<kPlaceGlobal, 4>(prm, sm_count, max_blocks, stream); break;
             default: return cudaErrorInvalidValue;
@@ -578,12 +588,12 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
     return cudaSuccess;
 }
 
-// The accumulators; above 256 groups also the mode word of the shared placement's path choice,
-// and above 4096 groups the partition workspace (which holds that word).
+// The accumulators; above 1024 groups also the mode word of the shared placement's path choice (room for it
+// from 257 on), and above 4096 groups the partition workspace (which holds that word).
 uint64_t groupkey_scratch_bytes(uint32_t num_groups) {
     const uint64_t a = (acc_bytes(num_groups) + 255) & ~255ull;
     if (num_groups >= groupkey_part_min_groups()) return a + groupkey_part_workspace_bytes();
-    if (num_groups > gk::kChooseAbove) return a + 256;   // the path choice's mode word
+    if (num_groups > 256) return a + 256;   // the path choice's mode word
     return acc_bytes(num_groups);
 }
 
