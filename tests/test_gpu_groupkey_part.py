@@ -175,7 +175,7 @@ def test_one_key_many_rows(table, monkeypatch, num_groups, blocks):
         check(comp, keys, num_groups, 730089, run_gpu(c, keys, num_groups, "shared_mem_per_thread", 730089, blocks))
 
 
-@pytest.mark.parametrize("num_groups,rows", [(3000, (1 << 25) - 1), (3000, 1 << 25), (4096, (1 << 25) + 1),
+@pytest.mark.parametrize("num_groups,rows", [(3000, 1 << 25), (3500, (1 << 25) - 1), (3500, 1 << 25), (4096, (1 << 25) + 1),
                                              (4097, (3 << 19) - 1), (4097, 3 << 19), (65536, (3 << 19) + 1)])
 @pytest.mark.parametrize("dist", ["uniform", "zipf"])
 def test_path_choice_lines(table, monkeypatch, num_groups, rows, dist):

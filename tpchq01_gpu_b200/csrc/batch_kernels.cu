@@ -112,7 +112,7 @@ __device__ __forceinline__ uint32_t consume_engine(const BatchParams& prm, uint3
     uint8_t* const tab = smem + S * kStage;   // all zero between runs
     const uint32_t lane = threadIdx.x & 31u, ctid = threadIdx.x, ttid = ctid % (kTeamWarps * 32);
     ka::Cube3Table cube3;
-    ka::CubeTableT<false> cube;
+    ka::CubeTable cube;
     ka::SlotTable slots;
     unsigned long long* acc = nullptr;
     uint32_t num_groups = 0, hot = 0;   // hot: keys below it go to the shared table

@@ -4,9 +4,10 @@
 // The per-row arithmetic is the reference's (src/kernels/ht_in_global_mem.hpp:31-49); only the
 // group index changes: group = key[i] (< num_groups) instead of (rf << 1) + ls.
 //
-// Input tile (2048 rows): ship u16 | qty u8 | disc u8 | tax u8 | price u32 | key u32 (13 B/row),
-// streamed with one cp.async.bulk per column into a 4-stage shared-memory ring exactly like the
-// scan kernel (scan_kernels.cu); 8 consumer warps decode 4 rows per step (q1_keyagg.cuh).
+// Input tiles (1024 to 3840 rows by placement and table): ship u16 | qty u8 | disc u8 | tax u8 |
+// price u32 | key u32 (13 B/row), streamed with one cp.async.bulk per column into a shared-memory
+// ring like the scan kernel's (scan_kernels.cu); the consumer warps decode 4 rows per step
+// (q1_keyagg.cuh).
 //
 // Placements:
 //   in_registers_per_thread  num_groups <= 8: per-thread dp4a byte planes (PlaneRegs<4|8>)
@@ -17,7 +18,7 @@
 //                            kernel with keys < 4096 in
 //                            slots and larger keys reduced straight into the global
 //                            accumulators, or the two-pass partitioned path of
-//                            groupkey_part.cu; above 1024 groups the path is chosen on the
+//                            groupkey_part.cu; above about 3100 groups the path is chosen on the
 //                            device from a sample of the rows of a large table
 //                            (q1_groupkey_choose), which may be the global placement's, when few
 //                            rows pass over spread keys
@@ -93,13 +94,21 @@ __host__ __device__ constexpr uint32_t table_bytes(uint32_t kind, uint32_t num_g
                                                                                                  : kWideSlots)
                                                                             : 0u));
 }
-// As many stages as fit beside the table (static shared memory: less than 4 KB), at most 4 of those
-// of 2048 rows and more, the same number for each team.
+// Stages of the ring in `bytes` of shared memory: at most 4 of 2048 rows and more, the same number for
+// each team.
 template <int P, int NG, bool kWide, uint32_t kTeams>
-__host__ constexpr uint32_t ring_stages(uint32_t kind, uint32_t num_groups) {
-    const uint32_t fit = (kMaxDynSmem - 4096 - table_bytes(kind, num_groups)) / stage_bytes<P, NG, kWide, kTeams>();
+__host__ constexpr uint32_t stages_in(uint32_t bytes) {
+    const uint32_t fit = bytes / stage_bytes<P, NG, kWide, kTeams>();
     const uint32_t most = kTeams == 1 ? 4u : kMaxStages;
     return (fit < most ? fit : most) / kTeams * kTeams;
+}
+// As many as fit beside the table and the static shared memory (the register placement's records: less
+// than 4 KB; the others' barriers: less than 1 KB, which leaves six stages beside the cells of 1024
+// groups, where three took 600 M rows 2.35 ms instead of 1.49).
+template <int P, int NG, bool kWide, uint32_t kTeams>
+__host__ constexpr uint32_t ring_stages(uint32_t kind, uint32_t num_groups) {
+    return stages_in<P, NG, kWide, kTeams>(kMaxDynSmem - (P == kPlaceInRegistersPerThread ? 4096 : 1024) -
+                                           table_bytes(kind, num_groups));
 }
 // Teams of the shared tables. One while three stages of its 3072-row tiles fit beside the table, then
 // three (100 M rows, 600 groups: 238 us with one team, 244 with two or three; 1000 groups: 303, 280 and
@@ -110,9 +119,9 @@ static uint32_t table_teams(uint32_t kind, uint32_t num_groups) {
     if (kind == kTableCube3) return 2;
     return ring_stages<kPlaceSharedMemPerThread, 4, false, 1>(kind, num_groups) >= 3 ? 1 : kSmallTeams;
 }
-static_assert(ring_stages<kPlaceSharedMemPerThread, 4, false, kSmallTeams>(kTableCube, ka::kCubeMaxGroups) >= kSmallTeams &&
-                  ring_stages<kPlaceSharedMemPerThread, 4, false, kSmallTeams>(kTableSlots, kWideSlots) >= kSmallTeams,
-              "a stage for every team beside the largest tables");
+static_assert(ring_stages<kPlaceSharedMemPerThread, 4, false, kSmallTeams>(kTableCube, ka::kCubeMaxGroups) >= 2 * kSmallTeams &&
+                  ring_stages<kPlaceSharedMemPerThread, 4, false, kSmallTeams>(kTableSlots, kWideSlots) >= 2 * kSmallTeams,
+              "two stages for every team beside the largest tables");
 
 }  // namespace gk
 
@@ -122,6 +131,7 @@ struct GroupKeyParams {
     int32_t cutoff;                 // cutoff_day - 727563
     uint32_t num_groups;
     uint32_t stages;                // ring stages
+    uint32_t stages_no_table;       // and where the global path leaves the table's room free
     unsigned long long* acc;        // scratch: num_groups x 8 u64, zeroed (shared and global placements)
     unsigned long long* out;        // [num_groups][6][lo, hi] (register placement)
     uint32_t* status;
@@ -134,7 +144,7 @@ struct GroupKeyParams {
 // 255 us instead of 240 once the global path was a fourth alternative.)
 template <uint32_t kTab>
 struct TableOf { using T = ka::SlotTable; };
-template <> struct TableOf<gk::kTableCube> { using T = ka::CubeTableT<true>; };
+template <> struct TableOf<gk::kTableCube> { using T = ka::CubeTable; };
 template <> struct TableOf<gk::kTableCube3> { using T = ka::Cube3Table; };
 
 template <int P, int NG, bool kWide = false, uint32_t kTab = gk::kTableNone, uint32_t kTeams = 1>
@@ -157,14 +167,14 @@ __global__ void __launch_bounds__((gk::consumer_warps<P, NG, kWide>() + kTeams) 
     __shared__ uint64_t warp_rec[P == kPlaceInRegistersPerThread ? W : 1][kRegValues];
     __shared__ __align__(16) unsigned long long wide[2 * kRegValues];
     // a path chosen on the device: this kernel (its table, or no table: the global path) unless partitioned
-    constexpr bool kChosen = kTab == kTableSlots;
+    constexpr bool kChosen = kTab == kTableSlots && kTeams > 1;
     bool no_table = false;
     if (kChosen && prm.mode) {
         const uint32_t mode = *prm.mode;
         if (mode == kModePartitioned) return;
         no_table = mode == kModeGlobalPath;
     }
-    const uint32_t S = prm.stages;
+    const uint32_t S = no_table ? prm.stages_no_table : prm.stages;
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint64_t num_tiles = prm.rows / R;
@@ -395,6 +405,7 @@ static cudaError_t launch_gk(GroupKeyParams prm, int sm_count, int max_blocks, c
     constexpr uint32_t R = tile_rows<P, NG, kWide, kTeams>();
     prm.stages = ring_stages<P, NG, kWide, kTeams>(kTab, prm.num_groups);
     const uint32_t dyn = prm.stages * stage_bytes<P, NG, kWide, kTeams>() + table_bytes(kTab, prm.num_groups);
+    prm.stages_no_table = stages_in<P, NG, kWide, kTeams>(dyn);
     cudaError_t e = cudaFuncSetAttribute(q1_groupkey_kernel<P, NG, kWide, kTab, kTeams>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
@@ -420,18 +431,23 @@ static cudaError_t launch_table(uint32_t table, uint32_t teams, const GroupKeyPa
 }
 
 static uint64_t acc_bytes(uint32_t num_groups) { return 64ull * num_groups; }
-// Whether the shared placement's path is chosen on the device, by rows of the launch; elsewhere it is the
-// single pass. The choice costs a launch (10 us, 20 us before the partition's kernels) and the global path
-// gains little on the tables: with fewer than 2% of the rows passing, 1000 groups, 60 M rows 154 us against
-// 145 with the table; 4096 groups 25 M rows 81 and 80, 60 M rows 153 and 163. Above 4096 groups the
-// partition gains nothing on small tables: 65,536 uniform groups, all rows passing, 1.0 M rows 78 us
-// chosen, 58 in a single pass, 2.0 M rows 83 and 91 (Zipf keys 81 and 58).
+// Whether the kernel of the shared placement takes a path chosen on the device (the largest tables').
+static bool takes_choice(int placement, uint32_t num_groups) {
+    const uint32_t table = gk::table_kind(placement, num_groups);
+    return table == gk::kTableSlots && gk::table_teams(table, num_groups) > 1;
+}
+// Whether the path is chosen, by rows of the launch; elsewhere it is the single pass. The choice costs a
+// launch (10 us, 20 us before the partition's kernels) and the global path gains little on the tables:
+// with 1% of the rows passing, 200 M rows, 1030 groups 485 us against 406 with the table, 2500 groups 482
+// and 432, 4096 groups 396 and 497, where 25 M rows take 81 and 80. Above 4096 groups the partition gains
+// nothing on small tables: 65,536 uniform groups, all rows passing, 1.0 M rows 78 us chosen, 58 in a
+// single pass, 2.0 M rows 83 and 91 (Zipf keys 81 and 58).
 static bool chosen_on_device(int placement, uint32_t num_groups, uint64_t rows) {
-    if (placement != kPlaceSharedMemPerThread || num_groups <= ka::kCubeMaxGroups) return false;
-    return rows >= (num_groups >= groupkey_part_min_groups() ? 3ull << 19 : 1ull << 25);
+    return takes_choice(placement, num_groups) &&
+           rows >= (num_groups >= groupkey_part_min_groups() ? 3ull << 19 : 1ull << 25);
 }
 
-// Chooses the path of the shared placement for more than 1024 groups from 8192 evenly spaced
+// Chooses the path of the shared placement's largest tables (takes_choice) from 8192 evenly spaced
 // sample rows and writes it to *mode (every path gives identical results):
 //   kModeGlobalPath   every passing row straight into the global accumulators, when fewer than
 //                     2% of the rows pass and no key occurs more than 3 times among the sampled
@@ -535,9 +551,10 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
         prm.num_groups = num_groups;
         const uint32_t table = gk::table_kind(placement, num_groups);
         uint32_t* mode = nullptr;   // the path, when it is not the single pass throughout
-        if (table == gk::kTableSlots && (force ? force != kModeSinglePass : chosen_on_device(placement, num_groups, n)))
+        if (force ? force != kModeSinglePass && takes_choice(placement, num_groups)
+                  : chosen_on_device(placement, num_groups, n))
             mode = reinterpret_cast<uint32_t*>(workspace + groupkey_part_mode_offset());
-        const bool global_cells = force == kModeGlobalPath && table == gk::kTableCube && num_groups > 256;
+        const bool forced_global = force == kModeGlobalPath && num_groups > 256 && !mode;
         prm.acc = scratch;
         prm.out = out;
         prm.status = status;
@@ -563,7 +580,7 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
                 break;
             }
             case kPlaceSharedMemPerThread:
-                e = global_cells ? launch_gk<kPlaceGlobal, 4>(prm, sm_count, max_blocks, stream)
+                e = forced_global ? launch_gk<kPlaceGlobal, 4>(prm, sm_count, max_blocks, stream)
                                  : launch_table(table, gk::table_teams(table, num_groups), prm, sm_count, max_blocks, stream);
                 break;
             case kPlaceGlobal: e = launch_gk<kPlaceGlobal, 4>(prm, sm_count, max_blocks, stream); break;
@@ -588,7 +605,7 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
     return cudaSuccess;
 }
 
-// The accumulators; above 1024 groups also the mode word of the shared placement's path choice (room for it
+// The accumulators; for the largest tables also the mode word of the shared placement's path choice (room for it
 // from 257 on), and above 4096 groups the partition workspace (which holds that word).
 uint64_t groupkey_scratch_bytes(uint32_t num_groups) {
     const uint64_t a = (acc_bytes(num_groups) + 255) & ~255ull;

@@ -95,7 +95,7 @@ __device__ __forceinline__ void bar_sync(uint32_t id, uint32_t threads) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Pass 2's table: (group, discount) cells like ka::CubeTableT, with the quantity in the cell too (a
+// Pass 2's table: (group, discount) cells like ka::CubeTable, with the quantity in the cell too (a
 // partition of skewed keys can be almost all one group: its rows then spread over eleven words).
 // ---------------------------------------------------------------------------------------------
 struct CellTable {

@@ -10,10 +10,9 @@
 //                  row with a price >= 2^24 goes to the global path); no atomics until a flush.
 //   Cube3Table     num_groups <= 64: a shared-memory table per (group, discount, tax) cell; a
 //                  row adds its count, its quantity and its price: three atomics.
-//   CubeTableT     num_groups <= 1024: a shared-memory table per (group, discount) cell. A row
+//   CubeTable      num_groups <= 1024: a shared-memory table per (group, discount) cell. A row
 //                  adds its count, price and tax * price to its cell and its quantity to its
-//                  group's word (the batch kernel's form: to one of four by discount & 3); the
-//                  discounted sums follow exactly at the flush, because the
+//                  group's word; the discounted sums follow exactly at the flush, because the
 //                  discount of a cell is known there: sum (100-d) p = sum_d (100-d) P_d and
 //                  sum (100-d)(100+t) p = sum_d (100-d) (100 P_d + TP_d).
 //   SlotTable      one shared-memory slot per key below the table's size (2048 in the batch
@@ -34,8 +33,7 @@
 // (wraps, and the cells' 100 - d summed over price and over tax-price wraps), from which the
 // flush adds what the wraps are worth. (Sending each wrap's 2^32 straight to the group's scratch
 // sums in global memory serialised on the L2 when one key holds many rows: Zipf keys over 1024
-// groups at full pass 2.98 ms per 600 M rows, 1.57 ms without those global atomics. The batch
-// kernel, whose instances' keys are uniform, keeps that form: see CubeTableT.) Rows
+// groups at full pass 2.98 ms per 600 M rows, 1.57 ms without those global atomics.) Rows
 // outside the tables' fast domain
 // (discount > 10, tax > 8 or price >= 2^24; TPC-H data has none) take the global path, so every
 // result is exact over the whole compressed domain.
@@ -71,15 +69,6 @@ struct TileLayout {
                       : (c == 1 ? kOffQty : (c == 2 ? kOffDisc : (c == 3 ? kOffTax : (c == 4 ? kOffPrice : kOffKey))));
     }
 };
-// The 2048-row tile of the batch kernels, the partitioned path and the group-key kernel's table
-// and global placements.
-constexpr uint32_t R = 2048;
-constexpr uint32_t kOffShip = TileLayout<R>::kOffShip, kOffQty = TileLayout<R>::kOffQty,
-                   kOffDisc = TileLayout<R>::kOffDisc, kOffTax = TileLayout<R>::kOffTax,
-                   kOffPrice = TileLayout<R>::kOffPrice, kOffKey = TileLayout<R>::kOffKey;
-constexpr uint32_t kStageBytes = TileLayout<R>::kStageBytes;
-__host__ __device__ constexpr uint32_t col_bytes(int c) { return TileLayout<R>::col_bytes(c); }
-__host__ __device__ constexpr uint32_t col_off(int c) { return TileLayout<R>::col_off(c); }
 
 // Flush cadences. Plane partials: at most 2^15 rows per thread; every consumer thread handles at
 // most 8 rows of a tile (the kernels assert it), so 4032 tiles leave room for one more partial
@@ -205,7 +194,7 @@ struct KeyQuad {
 
 // Rows 4j..4j+3 of the TR-row tile at shared address `base`. `bad` becomes nonzero for a value
 // outside the compressed domain (ship offset > 32767, discount > 100).
-template <uint32_t TR = R>
+template <uint32_t TR>
 __device__ __forceinline__ KeyQuad load_quad(uint32_t base, uint32_t j, int32_t cut, uint32_t& bad) {
     using TL = TileLayout<TR>;
     KeyQuad x;
@@ -305,18 +294,14 @@ struct PlaneRegs {
 // ---------------------------------------------------------------------------------------------
 // CubeTable: shared (group, discount) cells
 // ---------------------------------------------------------------------------------------------
-// kSharedCarries: wraps counted in the group's shared words (the group-key kernel); otherwise
-// each wrap's worth goes straight to the group's scratch sums and the group's four words hold its
-// quantity four ways, by discount & 3 (the batch kernel, whose combined engines measured 4-5% slower
-// with the shared counters although its 1024-group instances do not contend: 256 instances 4.02
-// -> 4.20 ms).
-template <bool kSharedCarries>
-struct CubeTableT {
+// Wraps are counted in the group's shared words. (Sent straight to the group's scratch sums instead, as the
+// batch kernel did: 64 instances of 1024 groups 299 us instead of 292, and frequent keys serialise.)
+struct CubeTable {
     uint32_t* w;       // [kCubeWords][cells]: count, price, tax * price (low words)
-    uint32_t* gw;      // kSharedCarries: [kCubeGroupWords][groups], word-major (consecutive groups'
-                       // words in consecutive banks): quantity; wraps of the group's cells' price
-                       // words; sum (100 - d) over those wraps; sum (100 - d) over wraps of tax *
-                       // price words. Otherwise [groups][kCubeGroupWords]: quantity by discount & 3.
+    uint32_t* gw;      // [kCubeGroupWords][groups], word-major (consecutive groups' words in
+                       // consecutive banks): quantity; wraps of the group's cells' price words;
+                       // sum (100 - d) over those wraps; sum (100 - d) over wraps of tax * price
+                       // words
     uint32_t cells, groups;
     __device__ __forceinline__ void bind(uint8_t* base, uint32_t num_groups) {
         w = reinterpret_cast<uint32_t*>(base);
@@ -347,10 +332,7 @@ struct CubeTableT {
             op[r] = ot[r] = 0;
             if ((m >> r) & 1u) {
                 atomicAdd(w + c[r], 1u);
-                if constexpr (kSharedCarries)
-                    atomicAdd(gw + key[r], (Q >> (8 * r)) & 0xFFu);
-                else
-                    atomicAdd(gw + key[r] * kCubeGroupWords + ((D >> (8 * r)) & 3u), (Q >> (8 * r)) & 0xFFu);
+                atomicAdd(gw + key[r], (Q >> (8 * r)) & 0xFFu);
                 op[r] = atomicAdd(w + cells + c[r], p[r]);
                 ot[r] = atomicAdd(w + 2 * cells + c[r], vt[r]);
             }
@@ -364,22 +346,12 @@ struct CubeTableT {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const uint32_t a = 100u - ((D >> (8 * r)) & 0xFFu);
-                if constexpr (kSharedCarries) {
-                    uint32_t* g = gw + key[r];
-                    if (op[r] > ~p[r]) {
-                        atomicAdd(g + groups, 1u);
-                        atomicAdd(g + 2 * groups, a);
-                    }
-                    if (ot[r] > ~vt[r]) atomicAdd(g + 3 * groups, a);
-                } else {
-                    unsigned long long* sg = acc + 8ull * key[r];
-                    if (op[r] > ~p[r]) {
-                        red_add(sg + 3, 1ull << 32);
-                        red_add(sg + 5, a);
-                        red_add(sg + 7, 100u * a);
-                    }
-                    if (ot[r] > ~vt[r]) red_add(sg + 7, a);
+                uint32_t* g = gw + key[r];
+                if (op[r] > ~p[r]) {
+                    atomicAdd(g + groups, 1u);
+                    atomicAdd(g + 2 * groups, a);
                 }
+                if (ot[r] > ~vt[r]) atomicAdd(g + 3 * groups, a);
             }
         }
     }
@@ -389,18 +361,9 @@ struct CubeTableT {
                                           uint32_t first = 0) {
         for (uint32_t i = tid; i < num_groups; i += nthreads) {
             const uint32_t g = i + first < num_groups ? i + first : i + first - num_groups;
-            uint64_t q = 0, pw = 0, aw = 0, tw = 0;
-            if constexpr (kSharedCarries) {
-                q = gw[g], pw = gw[groups + g], aw = gw[2 * groups + g], tw = gw[3 * groups + g];
+            const uint64_t q = gw[g], pw = gw[groups + g], aw = gw[2 * groups + g], tw = gw[3 * groups + g];
 #pragma unroll
-                for (uint32_t j = 0; j < kCubeGroupWords; ++j) gw[j * groups + g] = 0;
-            } else {
-#pragma unroll
-                for (uint32_t j = 0; j < kCubeGroupWords; ++j) {
-                    q += gw[g * kCubeGroupWords + j];
-                    gw[g * kCubeGroupWords + j] = 0;
-                }
-            }
+            for (uint32_t j = 0; j < kCubeGroupWords; ++j) gw[j * groups + g] = 0;
             uint64_t cnt = 0, dsum = 0, P = pw << 32;
             unsigned __int128 DP = (unsigned __int128)aw << 32, CH = (unsigned __int128)(100u * aw + tw) << 32;
 #pragma unroll
