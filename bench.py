@@ -734,11 +734,11 @@ def bench_tbl(args):
             "gpu_parse": {"ms": ms, "text_gbs": nbytes / (ms / 1e3) / 1e9, "moved_gbs": moved / (ms / 1e3) / 1e9,
                           "frac_hbm": moved / (ms / 1e3) / 1e9 / peak, "peak_kind": kind,
                           "wall_ms": wall_ms,
-                          "note": "CUDA events around the synchronous call on its stream (three kernels, two "
-                                  "memsets, two small reads); wall_ms adds the host side"},
+                          "note": "CUDA events around the synchronous call on its stream (one kernel, its "
+                                  "memsets and a small read); wall_ms adds the host side"},
             "file": {"ms": file_ms, "rows_per_s": rows / (file_ms / 1e3),
                      "note": "q1_tbl_read_file from the page cache: read, H2D, parse, D2H of the columns"},
-            "reference_cpu": ref, "clocks": clocks, "gpu_launches": 3}
+            "reference_cpu": ref, "clocks": clocks, "gpu_launches": 1}
     print(json.dumps(line), flush=True)
     return 0
 
