@@ -150,6 +150,9 @@ struct GroupRegs {
     }
 };
 
+// Most rows a thread adds in one launch (scan_max_rows_per_launch).
+constexpr uint32_t kMaxThreadRows = 1u << 15;
+
 // Warp-wide sum of aggregate a's per-thread partials. Per thread and launch at most 2^15 rows: count
 // < 2^16, quantity (compressed) < 2^23, discount < 2^22, price and reference-typed quantity < 2^47,
 // disc_price < 2^53.7, charge < 2^62.2.
@@ -361,6 +364,9 @@ template <bool kWideQty>
 struct Entry {
     static constexpr int kWords = kWideQty ? 5 : 4;
     static constexpr int kQtyShift = 16, kDiscShift = kWideQty ? 16 : 39;
+    static_assert(kMaxThreadRows < 1u << kQtyShift && (kWideQty || 255ull * kMaxThreadRows < 1ull << (kDiscShift - kQtyShift)) &&
+                      100ull * kMaxThreadRows < 1ull << (64 - kDiscShift),
+                  "the packed sums' fields");
     // word w of a group's sums
     template <class Buf>
     static __device__ __forceinline__ uint64_t word(const Buf& b, int i, int w) {
@@ -959,9 +965,11 @@ Geometry geometry(int layout, int placement, bool wide) {
 
 uint64_t scan_max_rows_per_launch(int layout, int placement, uint32_t grid) {
     const Geometry g = geometry(layout, placement, false);   // the fewer threads
-    uint64_t n = (uint64_t)grid * g.warps * 32ull * 32768ull;   // every consumer thread sums its own rows
-    if (n > (1ull << 31)) n = 1ull << 31;
-    return n / g.tile_rows * g.tile_rows;
+    // Whole tiles of a CTA, each thread its rows of every one, less one that leaves room for its tail rows (at
+    // most a tile's).
+    const uint32_t rows_per_thread = g.tile_rows / (g.warps * 32u);
+    const uint64_t n = (uint64_t)grid * (kMaxThreadRows / rows_per_thread - 1u) * g.tile_rows;
+    return std::min<uint64_t>(n, (1ull << 31) / g.tile_rows * g.tile_rows);
 }
 
 uint32_t scan_grid_blocks(int layout, int placement, uint64_t rows, int sm_count, int max_blocks) {
