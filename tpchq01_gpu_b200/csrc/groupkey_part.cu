@@ -67,11 +67,16 @@ constexpr uint32_t kP2Ctas = 1;                   // CTAs of pass 2 per SM
 constexpr uint32_t kQuads = 2;                    // times four records per thread and stage
 constexpr uint32_t kStageChunks = kQuads * kP2Threads * 4 / kChunk;
 
-// Chunks a segment may reserve: its records', an open one per CTA and partition, the unused part of
-// a CTA's last grab, and what a grab leaves of the one before (the chunks of one partition's run stay
-// together: fewer than kP1Rows / kChunk of every kGrab).
-constexpr uint64_t kPoolChunks = (kSegRows / kChunk) * (kGrab + kP1Rows / kChunk) / kGrab +
-                                 (uint64_t)kMaxGrid * (kParts + kGrab + 4 * (kP1Rows / kChunk));
+// Most chunks the CTAs of a segment reserve. A partition's list takes its records' chunks and, in every CTA,
+// an open one. Of every grab but a CTA's last, fewer than kRun chunks stay unused (a partition's chunks of one
+// round stay together), and all of the last may.
+constexpr uint32_t kRun = kP1Rows / kChunk;       // chunks one partition takes in a round at most
+static_assert(kP1Rows % kChunk == 0 && kParts + kRun <= kGrab, "a grab holds any round's chunks");
+__host__ __device__ constexpr uint64_t max_chunks(uint64_t rows, uint64_t ctas) {
+    const uint64_t used = rows / kChunk + ctas * kParts, of_grab = kGrab - (kRun - 1);
+    return (used * kGrab + of_grab - 1) / of_grab + ctas * kGrab;
+}
+constexpr uint64_t kPoolChunks = max_chunks(kSegRows, kMaxGrid);
 static_assert(kPoolChunks < (1u << 20), "a chunk id takes 20 bits of a list entry");
 
 struct Ctl {
@@ -181,6 +186,7 @@ struct PartParams {
     uint32_t* status;
     const uint32_t* mode;           // when set, the kernels run only if *mode == kModePartitioned
     gp::Ctl* ctl;
+    uint32_t max_chunks;            // of the segment: directory entries cleared
     uint16_t* dir;
     uint32_t* lists;
     uint2* pool;
@@ -334,7 +340,7 @@ __global__ void __launch_bounds__((gp::kP1Warps + 1) * 32, gp::kP1Ctas)
         } else {
             free += need;
         }
-        if (first + want > kPoolChunks) {    // (the pool is sized so that this cannot be)
+        if (first + want > prm.max_chunks) {   // (gp::max_chunks is such that this cannot be)
             if (prm.status) atomicOr(prm.status, kStatusInternal);
             first = 0;
         }
@@ -429,7 +435,7 @@ __global__ void __launch_bounds__((gp::kP1Warps + 1) * 32, gp::kP1Ctas)
     if (staged) write_out(parity ^ 1u);
     if (tid < kParts) {
         // the records of the open chunk
-        if (next < end && (next & (kChunk - 1)) && next / kChunk < kPoolChunks)
+        if (next < end && (next & (kChunk - 1)) && next / kChunk < prm.max_chunks)
             prm.dir[next / kChunk] = (uint16_t)((tid + 1) << 8 | ((next & (kChunk - 1)) - 1));
         if (chunks) atomicAdd(&prm.ctl->part_chunks[tid], chunks);
     }
@@ -462,7 +468,7 @@ __global__ void __launch_bounds__(256) q1_gk_lists_kernel(const __grid_constant_
     __shared__ uint32_t hist[kParts], base[kParts], off[kParts + 1], part_sum[kParts / 32];
     if (prm.mode && *prm.mode != kModePartitioned) return;
     const uint32_t tid = threadIdx.x;
-    const uint32_t n = min(prm.ctl->pool_next, (uint32_t)kPoolChunks);
+    const uint32_t n = min(prm.ctl->pool_next, prm.max_chunks);
     if (tid < kParts) list_offsets(prm, tid, off, part_sum);
     for (uint64_t t0 = (uint64_t)blockIdx.x * kTile; t0 < n; t0 += (uint64_t)gridDim.x * kTile) {
         if (tid < kParts) hist[tid] = 0;
@@ -481,7 +487,7 @@ __global__ void __launch_bounds__(256) q1_gk_lists_kernel(const __grid_constant_
         for (uint32_t j = 0; j < kPer; ++j) {
             if (e[j]) {
                 const uint32_t at = base[(e[j] >> 8) - 1] + rk[j];
-                if (at < kPoolChunks) prm.lists[at] = (uint32_t)(t0 + j * 256 + tid) | (e[j] & 0xFFu) << 20;
+                if (at < prm.max_chunks) prm.lists[at] = (uint32_t)(t0 + j * 256 + tid) | (e[j] & 0xFFu) << 20;
                 else if (prm.status) atomicOr(prm.status, kStatusInternal);
             }
         }
@@ -632,6 +638,8 @@ uint32_t groupkey_part_min_groups() { return 4097; }
 
 uint64_t groupkey_part_mode_offset() { return 192; }
 
+uint64_t groupkey_part_max_chunks(uint64_t rows, uint32_t ctas) { return gp::max_chunks(rows, ctas); }
+
 cudaError_t launch_groupkey_part(const uint8_t* const cols[6], uint64_t rows, int32_t cutoff_rel,
                                  uint32_t num_groups, unsigned long long* acc, uint8_t* workspace,
                                  const uint32_t* mode, uint32_t* status, int sm_count, int max_blocks,
@@ -665,14 +673,12 @@ cudaError_t launch_groupkey_part(const uint8_t* const cols[6], uint64_t rows, in
         prm.rows = n;
         const uint64_t tiles = n / kP1Rows;
         const uint32_t g1 = (uint32_t)(tiles == 0 ? 1 : (tiles < grid ? tiles : grid));
-        // most chunks the segment can reserve: the directory entries to clear and to list
-        const uint64_t max_chunks = (n / kChunk) * (kGrab + kP1Rows / kChunk) / kGrab +
-                                    (uint64_t)g1 * (kParts + kGrab + 4 * (kP1Rows / kChunk));
-        e = cudaMemsetAsync(prm.ctl, 0, kOffDir - kOffCtl + 2 * max_chunks, stream);
+        prm.max_chunks = (uint32_t)max_chunks(n, g1);
+        e = cudaMemsetAsync(prm.ctl, 0, kOffDir - kOffCtl + 2ull * prm.max_chunks, stream);
         if (e != cudaSuccess) return e;
         q1_gk_partition_kernel<<<g1, (kP1Warps + 1) * 32, kP1Smem, stream>>>(prm);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        uint64_t gl = (max_chunks + 2047) / 2048;
+        uint64_t gl = (prm.max_chunks + 2047) / 2048;
         if (gl > 4ull * (uint64_t)sm_count) gl = 4ull * (uint64_t)sm_count;
         q1_gk_lists_kernel<<<(unsigned)gl, 256, 0, stream>>>(prm);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -114,6 +114,8 @@ uint64_t groupkey_part_workspace_bytes();
 uint64_t groupkey_part_mode_offset();
 // fewest groups for which the shared placement has the partitioned path
 uint32_t groupkey_part_min_groups();
+// most chunks of 256 records that `ctas` CTAs reserve for a segment of `rows` rows
+uint64_t groupkey_part_max_chunks(uint64_t rows, uint32_t ctas);
 cudaError_t launch_generate_keys(uint64_t seed, uint64_t first_row, uint64_t rows, uint32_t num_groups,
                                  const uint32_t* dev_cdf, uint32_t* dev_keys, cudaStream_t stream);
 
