@@ -422,8 +422,8 @@ q1_status q1_batch_create(const q1_batch_instance* instances, uint32_t n, const 
 /* One execution of every instance (asynchronous; q1_sync_check reports device errors). */
 q1_status q1_batch_run(q1_batch* b, void* cuda_stream);
 q1_status q1_batch_describe(q1_batch* b, q1_batch_desc* out);
-/* Placement chosen for instance i: 1 shared table, 2 global (0, registers, is no longer chosen: the
- * table is the faster one for up to four groups too). */
+/* Placement chosen for instance i: 1 shared table, 2 global (0, registers, is no longer chosen: for up to
+ * four groups the tables by lane are faster on ordinary values and as fast on any). */
 q1_status q1_batch_instance_mode(q1_batch* b, uint32_t i, int32_t* mode);
 q1_status q1_batch_destroy(q1_batch* b);
 

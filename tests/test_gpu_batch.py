@@ -233,3 +233,148 @@ def test_batch_modes_from_a_cache_file(cuda, tmp_path):
     assert modes == [m or 1 for m in mode] and desc.tuned_classes == 0
     for i, (comp, keys, g, cutoff) in enumerate(inst):
         assert np.array_equal(read(outs[i], g), want[i]), (i, g)
+
+
+def few_group_columns(kind, rows, seed):
+    """Columns of instances of up to four groups: ordinary, all rows alike, over the whole compressed
+    domain, or all at its upper edge."""
+    comp = gen_np.compress(gen_np.generate(seed, 0, rows))
+    r = np.random.default_rng(seed)
+    if kind == "alike":
+        for k, v in [("quantity", 50), ("discount", 5), ("tax", 5), ("extendedprice", 10_494_950), ("shipdate", 7)]:
+            comp[k][:] = v
+    elif kind == "domain":
+        comp["discount"][:] = r.integers(0, 101, rows)
+        comp["tax"][:] = r.integers(0, 256, rows)
+        comp["extendedprice"][:] = r.integers(0, 2**32, rows, dtype=np.uint64).astype(np.uint32)
+        comp["quantity"][:] = r.integers(0, 256, rows)
+        comp["shipdate"][:] = r.integers(0, 32768, rows)
+    elif kind == "edge":
+        for k, v in [("quantity", 255), ("discount", 0), ("tax", 255), ("extendedprice", 0xFFFFFFFF), ("shipdate", 32767)]:
+            comp[k][:] = v
+    return comp
+
+
+@pytest.mark.parametrize("chunk", [0, 1])
+@pytest.mark.parametrize("kind", ["ordinary", "alike", "domain", "edge"])
+def test_batch_of_few_groups(cuda, kind, chunk):
+    """One to five groups, rows at the edges of a ring tile and of a team's turn, one key for nearly all rows or
+    keys spread evenly, beside instances of the other engines."""
+    inst = []
+    for i, rows in enumerate([1, 255, 256, 1023, 1024, 1025, 2 * 1024 + 7, 3 * 1024, 50_001, 300_011]):
+        for g in [1, 2, 3, 4, 5, 64, 1000]:
+            keys = gen_np.group_keys_uniform(600 + i, 0, rows, g)
+            if (i + g) % 2:
+                keys[rows // 10:] = g - 1
+            inst.append((few_group_columns(kind, rows, 5000 + 10 * i + g), keys, g, [729999, 760330][i % 2]))
+    want = oracle_tables(inst)
+    arr, outs, keep = to_device(inst)
+    stream = torch.cuda.current_stream().cuda_stream
+    run_batch(arr, len(inst), _lib.BatchOpts(1, 0, chunk, 0, None), stream)
+    for i, (comp, keys, g, cutoff) in enumerate(inst):
+        assert np.array_equal(read(outs[i], g), want[i]), (len(keys), g)
+
+
+def test_few_group_key_out_of_range_is_reported(cuda):
+    inst = make_instances(seed=12, n=30)
+    inst = [x for x in inst if x[2] == 4 and len(x[1]) > 1000][:1]
+    comp, keys, g, _ = inst[0]
+    keys = keys.copy()
+    keys[len(keys) // 2] = 4
+    arr, outs, keep = to_device([(comp, keys, g, 740000)])
+    stream = torch.cuda.current_stream().cuda_stream
+    with pytest.raises(q.Q1Error) as e:
+        run_batch(arr, 1, _lib.BatchOpts(1, 0, 0, 0, None), stream)
+    assert e.value.status == 6
+
+
+@pytest.fixture(scope="module")
+def alike_rows(cuda):
+    """18 million rows for every SM, all alike: each CTA gets more than 2^24 of them."""
+    n = 18_000_003 * torch.cuda.get_device_properties(0).multi_processor_count
+    cols = {k: torch.full((n,), v, dtype=d, device="cuda") for k, v, d in [
+        ("shipdate", 7, torch.int16), ("quantity", 255, torch.uint8), ("discount", 0, torch.uint8),
+        ("tax", 0, torch.uint8), ("extendedprice", 0, torch.int32)]}
+    cols["keys"] = torch.zeros(n, dtype=torch.int32, device="cuda")
+    return n, cols
+
+
+@pytest.mark.parametrize("num_groups,price,discount,tax", [
+    (1, (1 << 24) - 1, 10, 8), (4, (1 << 24) - 1, 10, 8), (64, (1 << 24) - 1, 10, 8), (1024, (1 << 24) - 1, 10, 8),
+    (2500, (1 << 24) - 1, 10, 8), (1, (1 << 32) - 1, 0, 255), (4, (1 << 32) - 1, 0, 255)])
+def test_batch_flushes_within_an_instance(alike_rows, num_groups, price, discount, tax):
+    """More than 2^24 rows of one instance in every CTA, all of one cell with the largest quantity: without a
+    flush after at most 2^23 of them, the cell's 32-bit quantity would wrap. Of up to four groups also with
+    values outside the cells' domain: without a flush after 2^21 of them, the slots' words would."""
+    n, cols = alike_rows
+    key = num_groups - 1
+    cols["keys"].fill_(key)
+    cols["discount"].fill_(discount)
+    cols["tax"].fill_(tax)
+    cols["extendedprice"].fill_(price if price < 1 << 31 else price - (1 << 32))
+    out = torch.zeros(num_groups * 12, dtype=torch.int64, device="cuda")
+    bi = (_lib.BatchInstance * 1)()
+    for k in ["shipdate", "discount", "extendedprice", "tax", "quantity"]:
+        setattr(bi[0].cols, k, cols[k].data_ptr())
+    bi[0].keys, bi[0].rows, bi[0].cutoff_day, bi[0].num_groups = cols["keys"].data_ptr(), n, 729999, num_groups
+    bi[0].aggregates = out.data_ptr()
+    stream = torch.cuda.current_stream().cuda_stream
+    run_batch(bi, 1, _lib.BatchOpts(1, 0, 0, 0, None), stream, runs=1)
+    got = q.decode_aggregates(read(out, num_groups), num_groups)
+    dp = (100 - discount) * price
+    want = np.zeros((num_groups, 6), dtype=object)
+    want[key] = [n, n * 25500, n * price, n * discount, n * dp, n * dp * (100 + tax)]
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("num_groups", [1, 2, 4])
+def test_few_groups_take_no_longer_for_rows_alike(cuda, num_groups):
+    """The time of an instance of up to four groups does not hang on its values: rows of one key, discount and tax,
+    and rows of any discount and tax, against ordinary ones (1.5 times allowed; cells that all rows add to took
+    2.7 times)."""
+    rows = 20_000_001
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+
+    def column(lo, hi, dtype):
+        return torch.randint(lo, hi, (rows,), generator=g, device="cuda", dtype=dtype)
+
+    cols = {"shipdate": column(0, 2500, torch.int16), "quantity": column(1, 51, torch.uint8),
+            "discount": column(0, 11, torch.uint8), "tax": column(0, 9, torch.uint8),
+            "extendedprice": column(90_000, 10_494_950, torch.int32), "keys": column(0, num_groups, torch.int32)}
+    out = torch.zeros(num_groups * 12, dtype=torch.int64, device="cuda")
+    bi = (_lib.BatchInstance * 1)()
+    for k in ["shipdate", "discount", "extendedprice", "tax", "quantity"]:
+        setattr(bi[0].cols, k, cols[k].data_ptr())
+    bi[0].keys, bi[0].rows, bi[0].cutoff_day, bi[0].num_groups = cols["keys"].data_ptr(), rows, 729999, num_groups
+    bi[0].aggregates = out.data_ptr()
+    stream = torch.cuda.current_stream()
+    b = ctypes.c_void_p()
+    opts = _lib.BatchOpts(1, 0, 0, 0, None)
+    _lib.check(q.lib().q1_batch_create(bi, 1, ctypes.byref(opts), ctypes.c_void_p(stream.cuda_stream), ctypes.byref(b)))
+
+    def best():
+        times = []
+        for _ in range(12):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            for _ in range(5):
+                _lib.check(q.lib().q1_batch_run(b, ctypes.c_void_p(stream.cuda_stream)))
+            ev[1].record()
+            torch.cuda.synchronize()
+            times.append(ev[0].elapsed_time(ev[1]))
+        return min(times)
+    try:
+        ordinary = best()
+        cols["tax"].copy_(column(0, 256, torch.int32))
+        cols["discount"].copy_(column(0, 101, torch.int32))
+        any_value = best()
+        cols["tax"].fill_(5)
+        cols["discount"].fill_(5)
+        cols["keys"].fill_(0)
+        alike = best()
+        _lib.check(q.lib().q1_sync_check(ctypes.c_void_p(stream.cuda_stream)))
+    finally:
+        torch.cuda.synchronize()
+        q.lib().q1_batch_destroy(b)
+    assert any_value < 1.5 * ordinary and alike < 1.5 * ordinary, (ordinary, any_value, alike)

@@ -15,14 +15,17 @@
 // the consumers straight from global memory instead). The teams aggregate into one table; when the
 // instance changes all of them flush it into the instance's scratch (red.global.add), according to
 // the instance's placement mode:
-//   kModeShared     num_groups <= 64: shared (group, discount, tax) cells (ka::Cube3Table);
-//                   <= 1024: shared (group, discount) cells (ka::CubeTable); more groups:
-//                   shared slots for keys < 2048 (ka::SlotTable), the rest spilled
+//   kModeShared     num_groups <= 4: (group, discount, tax) cells and slots by lane (ka::FewTable); <= 64:
+//                   shared (group, discount, tax) cells (ka::Cube3Table); <= 1024: shared (group,
+//                   discount) cells (ka::CubeTable); more groups: shared slots for keys < 2048
+//                   (ka::SlotTable), the rest spilled
 //   kModeGlobal     every passing row reduces straight into the scratch accumulators
-// Instances of up to four groups take the cells as well. (Byte planes in registers for them were slower
-// in every mix when the kernel had 16 warps and one producer: in a kernel of their own, beside the tables'
-// on a share of the SMs, 64 instances of 10^4 to 10^7 rows 330 us instead of 293, one of 10^8 rows and 4
-// groups 299 instead of 277; in the same kernel they spill.)
+// Few groups: 100 M rows of 4 groups 210 us, of one group 216 (byte planes in registers, in a kernel of their
+// own, 299 and 290: in this one they spill). Eight tables by lane instead of one: 4.0 M rows of one group with one
+// discount and tax 29 us instead of 72 (planes 29). Slots by lane instead of the scratch for rows outside the
+// cells' domain: with taxes up to 19, 35 us instead of 9,480 (planes 29); prices of 2^24 and more 35 us instead of
+// 19,800 (planes 19,400). Sums of every thread's own in shared memory, for rows of any values, took 257 us per
+// 100 M rows.
 // Bound: 64 instances as above take 245 us, their bytes 191 at the copy rate; with 64 groups all, 217: the
 // shared atomics of a row and the last pieces. 16 consumer warps in one team with one producer: 291.
 // (engines in q1_keyagg.cuh). Scratch per instance: num_groups x 8 u64, folded into the
@@ -47,7 +50,13 @@ namespace bk {
 constexpr uint32_t kWarps = 24, kTeams = 3, kTeamWarps = kWarps / kTeams;
 constexpr uint32_t R = kTeamWarps * 128;   // rows of a ring tile: one quad per consumer thread
 static_assert(kBatchTileRows % R == 0, "whole ring tiles in a work item's tile");
-static_assert((uint64_t)kBatchMaxItemTiles * kBatchTileRows <= ka::kTableFlushRows, "an item in one run");
+// Rows of a run, between two flushes of an engine's table.
+__host__ __device__ constexpr uint32_t flush_rows(uint32_t engine) {
+    return (uint32_t)(engine == kEngFew ? ka::kFewFlushRows : ka::kTableFlushRows);
+}
+static_assert((uint64_t)kBatchMaxItemTiles * kBatchTileRows <= flush_rows(kEngGlobal) &&
+                  (uint64_t)kBatchMaxFewItemTiles * kBatchTileRows <= flush_rows(kEngFew), "an item in one run");
+static_assert(kTeamWarps <= ka::kFewTeamWarps, "rows of a lane");
 using Tile = ka::TileLayout<R>;
 constexpr uint32_t kStage = Tile::kStageBytes;
 constexpr uint32_t kMaxStages = 9;         // of the ring
@@ -56,7 +65,8 @@ constexpr uint32_t kDynBytes = 227 * 1024 - kStaticBytes;   // ring, then table
 constexpr uint32_t kKindFull = 0, kKindPartial = 1, kKindEnd = 2;
 
 constexpr uint32_t table_bytes(uint32_t engine, uint32_t groups) {
-    return engine == kEngCube3  ? ka::cube3_bytes(groups)
+    return engine == kEngFew     ? ka::few_bytes(groups)
+           : engine == kEngCube3 ? ka::cube3_bytes(groups)
            : engine == kEngCube ? ka::cube_bytes(groups)
            : engine == kEngSlots ? ka::slot_bytes(groups < ka::kSlots ? groups : ka::kSlots)
                                  : 0;
@@ -66,7 +76,8 @@ constexpr uint32_t stages_beside(uint32_t bytes) {
     const uint32_t fit = (kDynBytes - bytes) / kStage;
     return (fit < kMaxStages ? fit : kMaxStages) / kTeams * kTeams;
 }
-static_assert(stages_beside(table_bytes(kEngCube3, ka::kCube3MaxGroups)) == 9 &&
+static_assert(stages_beside(table_bytes(kEngFew, ka::kFewGroups)) == 9 &&
+                  stages_beside(table_bytes(kEngCube3, ka::kCube3MaxGroups)) == 9 &&
                   stages_beside(table_bytes(kEngCube, ka::kCubeMaxGroups)) == 6 &&
                   stages_beside(table_bytes(kEngSlots, ka::kSlots)) == 9,
               "ring beside the largest tables");
@@ -78,7 +89,7 @@ struct __align__(16) StageMeta {
     uint32_t rows;       // rows | the tile's high word << 16
 };
 
-// A run: consecutive tiles of one instance in this CTA, at most ka::kTableFlushRows rows; the table
+// A run: consecutive tiles of one instance in this CTA, at most flush_rows() of them; the table
 // is flushed at its end. Every team's producer numbers all runs alike and writes their descriptors for
 // its own team before the next stage that it posts. A team's next stage is at most a few of its tiles
 // past the last one it released (a ring's worth and one), and so many times three of the CTA's, each of
@@ -102,15 +113,24 @@ struct Place {
 // Consumer side of one engine: processes the team's stages until the producer's end-of-engine
 // marker, flushing the table at the end of every run (a barrier of all consumer warps: each team goes
 // through all runs, also those none of its tiles belong to). Returns the engine to go on with, kEngines
-// at the end or if a bounded wait expired (the kernel then stops).
+// at the end or if a bounded wait expired (the kernel then stops). (A function of its own for each engine: inlined
+// in one, 64 instances of 64 groups took 218 us instead of 215, of 1024 groups 302 instead of 292.)
 template <int E>
-__device__ __forceinline__ uint32_t consume_engine(const BatchParams& prm, uint32_t ring, uint8_t* smem,
-                                                   uint64_t* full_bar, uint64_t* empty_bar, const StageMeta* meta,
-                                                   const Run* runs, Place& at, ka::ConsumerBarrier& cb,
-                                                   uint32_t& bad) {
+static __device__ __noinline__ uint32_t consume_engine(const BatchParams& prm, uint32_t ring, uint8_t* smem,
+                                                       uint64_t* full_bar, uint64_t* empty_bar, const StageMeta* meta,
+                                                       const Run* runs, Place& at_, ka::ConsumerBarrier& cb_,
+                                                       uint32_t& bad_) {
+    Place at = at_;
+    ka::ConsumerBarrier cb = cb_;
+    uint32_t bad = bad_;
+    auto leave = [&](uint32_t e) {
+        at_ = at, cb_ = cb, bad_ = bad;
+        return e;
+    };
     const uint32_t S = prm.stages[E];
     uint8_t* const tab = smem + S * kStage;   // all zero between runs
     const uint32_t lane = threadIdx.x & 31u, ctid = threadIdx.x, ttid = ctid % (kTeamWarps * 32);
+    ka::FewTable few;
     ka::Cube3Table cube3;
     ka::CubeTable cube;
     ka::SlotTable slots;
@@ -124,12 +144,15 @@ __device__ __forceinline__ uint32_t consume_engine(const BatchParams& prm, uint3
         num_groups = r.num_groups;
         cutoff = r.cutoff;
         hot = (E == kEngSlots && num_groups > ka::kSlots) ? ka::kSlots : num_groups;
+        if constexpr (E == kEngFew) few.bind(tab, num_groups, lane);
         if constexpr (E == kEngCube3) cube3.bind(tab, num_groups);
         if constexpr (E == kEngCube) cube.bind(tab, num_groups);
         if constexpr (E == kEngSlots) slots.bind(tab, hot);
     };
     auto add = [&](const ka::KeyQuad& x) {
-        if constexpr (E == kEngCube3) {
+        if constexpr (E == kEngFew) {
+            ka::table_quad(few, x, num_groups, hot, acc, bad);
+        } else if constexpr (E == kEngCube3) {
             ka::table_quad(cube3, x, num_groups, hot, acc, bad);
         } else if constexpr (E == kEngCube) {
             ka::table_quad(cube, x, num_groups, hot, acc, bad);
@@ -154,7 +177,7 @@ __device__ __forceinline__ uint32_t consume_engine(const BatchParams& prm, uint3
     uint32_t current = kUnbound;   // tag of a full tile of run at.run, once the fields above are that run's
     for (;;) {
         const bool landed = mbar_wait(smem_addr(&full_bar[at.s]), at.ph, prm.status);
-        if (!__all_sync(0xffffffffu, landed)) return kEngines;
+        if (!__all_sync(0xffffffffu, landed)) return leave(kEngines);
         const uint32_t tag = meta[at.s].tag;
         uint32_t n = 0, next = kEngines;   // rows of a partial tile, engine after this one
         if (tag != current) {
@@ -162,7 +185,8 @@ __device__ __forceinline__ uint32_t consume_engine(const BatchParams& prm, uint3
                 if constexpr (E != kEngGlobal) {
                     if (current == kUnbound) bind();
                     cb.sync(lane, prm.status);
-                    if constexpr (E == kEngCube3) cube3.flush(acc, num_groups, ctid, kWarps * 32);
+                    if constexpr (E == kEngFew) few.flush(acc, ctid >> 5, lane);
+                    else if constexpr (E == kEngCube3) cube3.flush(acc, num_groups, ctid, kWarps * 32);
                     else if constexpr (E == kEngCube) cube.flush(acc, num_groups, ctid, kWarps * 32);
                     else slots.flush(acc, hot, ctid, kWarps * 32);
                     cb.sync(lane, prm.status);
@@ -195,7 +219,7 @@ __device__ __forceinline__ uint32_t consume_engine(const BatchParams& prm, uint3
             at.s -= S;
             at.ph ^= 1u;
         }
-        if ((tag & 3u) == kKindEnd) return next;
+        if ((tag & 3u) == kKindEnd) return leave(next);
     }
 }
 
@@ -329,9 +353,9 @@ __global__ void __launch_bounds__((bk::kWarps + bk::kTeams) * 32, 1)
             }
             const BatchInstanceDev& in = prm.inst[it.instance];
             const uint64_t row0 = (uint64_t)it.first_tile * kBatchTileRows;
-            const uint64_t left = in.rows - row0;   // an item has at most ka::kTableFlushRows rows
+            const uint64_t left = in.rows - row0;   // an item has at most flush_rows(engine) rows
             const uint32_t rows = left < it.num_tiles * kBatchTileRows ? (uint32_t)left : it.num_tiles * kBatchTileRows;
-            if (it.instance != run_instance || run_rows + rows > ka::kTableFlushRows) {
+            if (it.instance != run_instance || run_rows + rows > flush_rows(engine)) {
                 ++run;
                 run_instance = it.instance;
                 run_rows = 0;
@@ -378,6 +402,7 @@ __global__ void __launch_bounds__((bk::kWarps + bk::kTeams) * 32, 1)
         Place at{team, 0, 0};
         for (uint32_t e = first_engine;;) {
             switch (e) {
+                case kEngFew: e = consume_engine<kEngFew>(prm, ring, smem, full_bar, empty_bar, meta, runs[team], at, cb, bad); break;
                 case kEngCube3: e = consume_engine<kEngCube3>(prm, ring, smem, full_bar, empty_bar, meta, runs[team], at, cb, bad); break;
                 case kEngCube: e = consume_engine<kEngCube>(prm, ring, smem, full_bar, empty_bar, meta, runs[team], at, cb, bad); break;
                 case kEngSlots: e = consume_engine<kEngSlots>(prm, ring, smem, full_bar, empty_bar, meta, runs[team], at, cb, bad); break;

@@ -98,6 +98,7 @@ void save_cache(const std::string& path) {
 
 uint32_t q1::batch_engine(uint32_t mode, uint32_t num_groups) {
     if (mode == kModeGlobal) return kEngGlobal;
+    if (num_groups <= 4) return kEngFew;        // ka::kFewGroups
     if (num_groups <= 64) return kEngCube3;     // ka::kCube3MaxGroups
     if (num_groups <= 1024) return kEngCube;    // ka::kCubeMaxGroups
     return kEngSlots;
@@ -107,7 +108,7 @@ namespace {
 
 // Relative cost of a row per engine, 64 groups = 1 (one instance of 10^8 rows, uniform keys: 64 groups
 // 212 us, 1024 groups 282 us): used only to split the grid.
-constexpr double kEngineCost[kEngines] = {1.0, 1.33, 1.6, 8.4};
+constexpr double kEngineCost[kEngines] = {1.0, 1.0, 1.33, 1.6, 8.4};
 
 // Work items: every instance in pieces of `chunk` tiles or, with chunk 0, of falling size: an engine's
 // largest instances first, each piece three quarters of an equal share of the tiles its engine's CTAs still
@@ -142,7 +143,7 @@ void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32
             const uint64_t all = tiles_of(i);
             for (uint64_t t = 0; t < all;) {
                 const uint64_t piece = chunk ? chunk : std::max(least, (uint64_t)((double)left / (1.33 * ctas)));
-                const uint64_t most = std::min<uint64_t>(piece, kBatchMaxItemTiles);
+                const uint64_t most = std::min<uint64_t>(piece, e == kEngFew ? kBatchMaxFewItemTiles : kBatchMaxItemTiles);
                 BatchItem it{};
                 it.instance = i;
                 it.first_tile = (uint32_t)t;

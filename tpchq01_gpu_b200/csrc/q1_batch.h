@@ -10,6 +10,7 @@ namespace q1 {
 
 constexpr uint32_t kBatchTileRows = 2048;
 constexpr uint32_t kBatchMaxItemTiles = 4096;   // 2^23 rows: what a table takes between flushes
+constexpr uint32_t kBatchMaxFewItemTiles = 1023;   // and what the one of few groups does
 
 // Placement of one instance inside the batch kernel.
 enum BatchMode : uint32_t {
@@ -38,11 +39,12 @@ struct BatchItem {
 
 // Engine that aggregates an instance inside the batch kernel (q1_keyagg.cuh).
 enum BatchEngine : uint32_t {
-    kEngCube3 = 0,       // (group, discount, tax) cells, <= 64 groups
-    kEngCube = 1,        // (group, discount) cells, <= 1024 groups
-    kEngSlots = 2,       // slots for keys < 2048, larger keys spilled
-    kEngGlobal = 3,      // straight into scratch
-    kEngines = 4,
+    kEngFew = 0,         // (group, discount, tax) cells and slots by lane, <= 4 groups
+    kEngCube3 = 1,       // (group, discount, tax) cells, <= 64 groups
+    kEngCube = 2,        // (group, discount) cells, <= 1024 groups
+    kEngSlots = 3,       // slots for keys < 2048, larger keys spilled
+    kEngGlobal = 4,      // straight into scratch
+    kEngines = 5,
 };
 uint32_t batch_engine(uint32_t mode, uint32_t num_groups);
 

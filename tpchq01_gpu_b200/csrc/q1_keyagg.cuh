@@ -10,6 +10,8 @@
 //                  row with a price >= 2^24 goes to the global path); no atomics until a flush.
 //   Cube3Table     num_groups <= 64: a shared-memory table per (group, discount, tax) cell; a
 //                  row adds its count, its quantity and its price: three atomics.
+//   FewTable       num_groups <= 4, in the batch kernel: eight of those tables, by lane, and a slot
+//                  per lane and group for rows outside their domain.
 //   CubeTable      num_groups <= 1024: a shared-memory table per (group, discount) cell. A row
 //                  adds its count, price and tax * price to its cell and its quantity to its
 //                  group's word; the discounted sums follow exactly at the flush, because the
@@ -314,7 +316,7 @@ struct CubeTable {
     }
     // Rows r of a quad with bit r of `m` set (passing, key < num_groups, fast domain). All
     // atomics of the quad are issued before any carry is checked, so their latencies overlap.
-    static constexpr bool kPacked = true;
+    static constexpr bool kPacked = true, kSlots = false;
     // The quantity, discount and tax bytes of the four rows packed in Q, D, X; acc: the scratch. A
     // cell's count and a group's quantity cannot wrap between flushes (at most 2^23 rows per CTA:
     // count < 2^24, quantity <= 255 * 2^23 < 2^32), so their atomics need no result. A wrap of a
@@ -401,7 +403,7 @@ struct Cube3Table {
     __device__ __forceinline__ void zero(uint32_t tid, uint32_t nthreads) {
         for (uint32_t i = tid; i < kCube3Words * cells; i += nthreads) w[i] = 0;
     }
-    static constexpr bool kPacked = true;
+    static constexpr bool kPacked = true, kSlots = false;
     // Rows r of a quad with bit r of `m` set (fast domain), the quantity, discount and tax bytes
     // of the four rows packed in Q, D, X (D and X zero in rows outside the fast domain). There
     // 9 d + t < 99 fits a byte, so one shift-and-add gives the four (discount, tax) cell offsets.
@@ -479,10 +481,125 @@ struct Cube3Table {
 };
 
 // ---------------------------------------------------------------------------------------------
+// FewTable: num_groups <= kFewGroups, in the batch kernel. kFewCopies (group, discount, tax) tables: a lane adds to
+// the one of its number modulo kFewCopies, so that at most four lanes of a warp meet in a cell, as they do in a bank
+// for spread values. A quad with a row outside the cells' domain goes to slots instead, one per lane and group, whose
+// lanes lie in all 32 banks. So the time does not hang on the values.
+// ---------------------------------------------------------------------------------------------
+constexpr uint32_t kFewGroups = 4, kFewCopies = 8;
+// A slot's words: count, quantity, discount, then price, disc_price and charge in pieces of 16 bits (2, 3, 3), whose sums
+// over a lane's rows between flushes need no carry: at most kFewFlushRows / 32 rows and, of a last tile, one more in each
+// of a team's kFewTeamWarps warps.
+constexpr uint32_t kFewSlotWords = 11, kFewTeamWarps = 8;
+constexpr uint64_t kFewFlushRows = (1ull << 21) - 2048;
+static_assert((kFewFlushRows / 32 + kFewTeamWarps) * 0xFFFFull < 1ull << 32 && kFewFlushRows < kTableFlushRows, "a word's sum");
+// words from one table to the next: the tables start four banks apart
+constexpr __host__ __device__ uint32_t few_stride(uint32_t num_groups) {
+    const uint32_t words = cube3_bytes(num_groups) / 4;
+    return words + (32u / kFewCopies + 32u - words % 32u) % 32u;
+}
+constexpr __host__ __device__ uint32_t few_bytes(uint32_t num_groups) {
+    return 4 * (kFewCopies * few_stride(num_groups) + kFewSlotWords * num_groups * 32);
+}
+// Rows r of a quad with bit r of m set into the slots at slot + 32 key, n words from word to word. (A function of its
+// own, and a small one: what it needs in registers is taken from the cells' path beside it.)
+static __device__ __noinline__ void few_slot_rows(uint32_t* slot, uint32_t n, uint32_t m, const KeyQuad x) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        if (!((m >> r) & 1u)) continue;
+        const uint32_t q = (x.Q >> (8 * r)) & 0xFFu, d = (x.D >> (8 * r)) & 0xFFu, t = (x.X >> (8 * r)) & 0xFFu, p = x.p[r];
+        const uint32_t a = 100u - d;
+        const uint64_t dp = (uint64_t)a * p, ch = (uint64_t)(a * (100u + t)) * p;   // below 2^38.7, 2^47.2
+        uint32_t* const w = slot + x.k[r] * 32;
+        atomicAdd(w, 1u);
+        atomicAdd(w + n, q);
+        atomicAdd(w + 2 * n, d);
+        atomicAdd(w + 3 * n, p & 0xFFFFu);
+        atomicAdd(w + 4 * n, p >> 16);
+        atomicAdd(w + 5 * n, (uint32_t)dp & 0xFFFFu);
+        atomicAdd(w + 6 * n, (uint32_t)dp >> 16);
+        atomicAdd(w + 7 * n, (uint32_t)(dp >> 32));
+        atomicAdd(w + 8 * n, (uint32_t)ch & 0xFFFFu);
+        atomicAdd(w + 9 * n, (uint32_t)ch >> 16);
+        atomicAdd(w + 10 * n, (uint32_t)(ch >> 32));
+    }
+}
+struct FewTable {
+    Cube3Table cells;   // the lane's
+    uint32_t* slot;     // the lane's of group 0, [kFewSlotWords][groups][32 lanes]
+    uint32_t groups;
+    __device__ __forceinline__ void bind(uint8_t* base, uint32_t num_groups, uint32_t lane) {
+        cells.bind(base, num_groups);
+        slot = cells.w + kFewCopies * few_stride(num_groups) + lane;
+        cells.w += lane % kFewCopies * few_stride(num_groups);
+        groups = num_groups;
+    }
+    static constexpr bool kPacked = true, kSlots = true;
+    __device__ __forceinline__ void add_quad_packed(uint32_t m, const uint32_t key[4], uint32_t Q, uint32_t D, uint32_t X,
+                                                    const uint32_t p[4], unsigned long long* acc) {
+        cells.add_quad_packed(m, key, Q, D, X, p, acc);
+    }
+    // Rows r of a quad with bit r of m set, of any values, into the lane's slots.
+    __device__ __forceinline__ void slot_rows(uint32_t m, const KeyQuad& x) const { few_slot_rows(slot, groups * 32, m, x); }
+    // All tables' and slots' sums -> scratch, and zero again: a warp per group, half of the tables to each half of its
+    // lanes. The caller synchronises the consumers around it; all lanes of the warps call. Of kFewFlushRows
+    // rows a group's price sum is below 2^53, its disc_price below 2^60.
+    __device__ __forceinline__ void flush(unsigned long long* acc, uint32_t g, uint32_t lane) {
+        if (g >= groups) return;
+        const uint32_t d = lane & 15u, n = groups * 32, stride = few_stride(groups), per_word = cells.cells;
+        uint32_t cnt = 0, q = 0;
+        uint64_t P = 0, T = 0;   // of the lane's cells: sum over the taxes of the price, and of tax * price
+        if (d < kCubeDisc) {
+            uint32_t* const first = cells.w - lane % kFewCopies * stride + (g * kCubeDisc + d) * kCubeTax;
+            for (uint32_t k = lane / 16; k < kFewCopies; k += 2) {
+                uint32_t* const w = first + k * stride;
+#pragma unroll
+                for (uint32_t t = 0; t < kCubeTax; ++t) {
+                    const uint64_t Pt = ((uint64_t)w[3 * per_word + t] << 32) | w[2 * per_word + t];
+                    cnt += w[t];
+                    q += w[per_word + t];
+                    P += Pt;
+                    T += t * Pt;
+#pragma unroll
+                    for (uint32_t j = 0; j < kCube3Words; ++j) w[j * per_word + t] = 0;
+                }
+            }
+        }
+        uint32_t disc = d * cnt;
+        uint64_t DP = (100u - d) * P, CH = (100u - d) * (100u * P + T);
+        uint64_t chl = CH & 0xFFFFFFFFull, chh = CH >> 32;
+        uint32_t* const s = slot + g * 32;
+        if (__any_sync(0xffffffffu, *s)) {
+            uint64_t w[kFewSlotWords];
+#pragma unroll
+            for (uint32_t j = 0; j < kFewSlotWords; ++j) {
+                w[j] = s[j * n];
+                s[j * n] = 0;
+            }
+            cnt += (uint32_t)w[0];
+            q += (uint32_t)w[1];
+            disc += (uint32_t)w[2];
+            P += w[3] + (w[4] << 16);
+            DP += w[5] + (w[6] << 16) + (w[7] << 32);
+            chl += w[8] + (w[9] << 16);
+            chh += w[10];
+        }
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        q = __reduce_add_sync(0xffffffffu, q);
+        disc = __reduce_add_sync(0xffffffffu, disc);
+        P = warp_sum<64>(P).lo, DP = warp_sum<64>(DP).lo, chl = warp_sum<54>(chl).lo, chh = warp_sum<54>(chh).lo;
+        // lane j adds the group's word j
+        const uint64_t s01 = lane & 1u ? q : cnt, s23 = lane & 1u ? P : disc,
+                       s45 = lane & 1u ? DP >> 32 : DP & 0xFFFFFFFFull, s67 = lane & 1u ? chh : chl;
+        if (lane < 8) red_add(acc + 8ull * g + lane, lane & 4u ? (lane & 2u ? s67 : s45) : (lane & 2u ? s23 : s01));
+    }
+};
+
+// ---------------------------------------------------------------------------------------------
 // SlotTable: shared per-group slots for keys < slots
 // ---------------------------------------------------------------------------------------------
 struct SlotTable {
-    static constexpr bool kPacked = false;
+    static constexpr bool kPacked = false, kSlots = false;
     uint32_t* w;       // [kSlotWords][slots]
     uint32_t slots;
     __device__ __forceinline__ void bind(uint8_t* base, uint32_t n) {
@@ -555,8 +672,8 @@ struct SlotTable {
     }
 };
 
-// One quad into a shared table (CubeTable or SlotTable): rows in the table's fast domain go to the
-// table, other passing rows with key < num_groups straight to the scratch, passing rows with
+// One quad into a shared table: rows in the table's fast domain go to the table, other passing rows
+// with key < num_groups straight to the scratch (a FewTable's to its slots), passing rows with
 // key >= num_groups make `bad` nonzero.
 // All lanes of the warp call it (the slow path, the tables' early exit when no lane of the warp
 // has a row to add, and the carries use warp votes).
@@ -591,11 +708,16 @@ __device__ __forceinline__ void table_quad(Table& tab, const KeyQuad& x, uint32_
     }
     // rows outside the tables' fast domain (none in TPC-H data): one vote skips the path
     if (__any_sync(0xffffffffu, slow)) {
+        if constexpr (Table::kSlots) {   // as good for the warp's other rows, and one path is shorter than two
+            tab.slot_rows(m | slow, x);
+            return;
+        } else {
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-            if ((slow >> r) & 1u)
-                scratch_row(acc, x.k[r], (x.Q >> (8 * r)) & 0xFFu, (x.D >> (8 * r)) & 0xFFu,
-                            (x.X >> (8 * r)) & 0xFFu, x.p[r]);
+            for (int r = 0; r < 4; ++r)
+                if ((slow >> r) & 1u)
+                    scratch_row(acc, x.k[r], (x.Q >> (8 * r)) & 0xFFu, (x.D >> (8 * r)) & 0xFFu,
+                                (x.X >> (8 * r)) & 0xFFu, x.p[r]);
+        }
     }
     if constexpr (Table::kPacked) {
         // discount and tax bytes of in-domain rows only (d <= 10, t <= 8), so that byte-wise
