@@ -229,3 +229,27 @@ def test_groupkey_tile_and_team_edges(table, num_groups, blocks):
             want, flag = O.q1_groupkey(part, keys[:rows], num_groups, cutoff)
             assert flag == 0
             assert np.array_equal(got, want), (rows, cutoff)
+
+
+@pytest.mark.parametrize("rows,blocks", [(r, 1) for r in [122_879, 122_880, 122_881, 126_719, 126_720, 150_001]] +
+                         [(r, 4) for r in [491_519, 491_520, 491_521, 499_201]])
+@pytest.mark.parametrize("num_groups", [1, 4])
+def test_wide_register_planes_ragged_tiles(cuda, rows, blocks, num_groups):
+    """Row counts around the tiles of the register planes' kernel for large tables (15 warps over 3840-row tiles
+    from 32 of them per CTA on), with prices of 2^24 and more."""
+    part = widen(gen_np.compress(gen_np.generate(SEED + 16, 0, rows)), 17, frac=0.01)
+    c, keep = device_cols(part)
+    keys = gen_np.group_keys_uniform(SEED + 15, 0, rows, num_groups)
+    check(part, keys, num_groups, 729999,
+          run_gpu(c, keys, num_groups, "in_registers_per_thread", 729999, blocks=blocks))
+
+
+@pytest.mark.parametrize("num_groups", [3, 4])
+def test_wide_register_planes_flush_mid_launch(cuda, num_groups):
+    """One CTA over more than 4032 tiles of 3840 rows: its planes go to the result table inside the launch."""
+    rows = 4032 * 3840 + 2 * 3840 + 77
+    comp = widen(gen_np.compress(gen_np.generate(SEED + 18, 0, rows)), 19, frac=0.001)
+    c, keep = device_cols(comp)
+    keys = gen_np.group_keys_uniform(SEED + 17, 0, rows, num_groups)
+    check(comp, keys, num_groups, 740000,
+          run_gpu(c, keys, num_groups, "in_registers_per_thread", 740000, blocks=1))

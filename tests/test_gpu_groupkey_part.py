@@ -209,3 +209,26 @@ def test_path_choice_lines(table, monkeypatch, num_groups, rows, dist):
         want = whole * q.decode_aggregates(O.q1_groupkey(comp, keys, num_groups, cutoff)[0], num_groups)
         want = want + q.decode_aggregates(O.q1_groupkey(part, keys[:rest], num_groups, cutoff)[0], num_groups)
         assert np.array_equal(got, want), cutoff
+
+
+@pytest.mark.parametrize("num_groups", [5000, 65536])
+@pytest.mark.parametrize("blocks", [0, 1, 3])
+def test_path_choice_with_few_ctas_and_domain_edges(table, monkeypatch, num_groups, blocks):
+    """The choice on the device, on a table large enough for it, in few CTAs and with rows outside the tables'
+    fast domain; a key out of range is reported whatever path is taken."""
+    monkeypatch.delenv("Q1_GROUPKEY_PATH", raising=False)
+    comp, _, _ = table
+    comp = {k: np.tile(comp[k], 5) for k in ["shipdate", "quantity", "discount", "tax", "extendedprice"]}
+    assert len(comp["shipdate"]) > 3 << 19
+    wide = widen(comp, 77, frac=0.02)
+    c, keep = device_cols(wide)
+    for dist in ["uniform", "zipf"]:
+        keys = np.tile(keys_for(num_groups, dist)[0], 5)
+        for cutoff in [727600, 729999]:
+            check(wide, keys, num_groups, cutoff, run_gpu(c, keys, num_groups, "shared_mem_per_thread", cutoff, blocks))
+        keys[123_456] = num_groups
+        for cutoff in [727600, 740000]:
+            if cutoff == 740000 or wide["shipdate"][123_456] <= cutoff - 727563:
+                with pytest.raises(q.Q1Error) as e:
+                    run_gpu(c, keys, num_groups, "shared_mem_per_thread", cutoff, blocks)
+                assert e.value.status == 6
