@@ -100,3 +100,51 @@ def test_partition_chunks_of_small_and_uniform_segments():
             for _ in range(rounds):
                 pool.round({p: 3072 // spread for p in range(spread)})
             assert pool.reserved <= bound(rounds * 3072, 1), (rounds, spread)
+
+
+class BatchInstance(ctypes.Structure):
+    _fields_ = [("col", ctypes.c_void_p * 6), ("rows", ctypes.c_uint64), ("cutoff", ctypes.c_int32),
+                ("num_groups", ctypes.c_uint32), ("mode", ctypes.c_uint32), ("pad", ctypes.c_uint32),
+                ("acc", ctypes.c_void_p), ("out", ctypes.c_void_p)]
+
+
+class BatchItem(ctypes.Structure):
+    _fields_ = [("instance", ctypes.c_uint32), ("first_tile", ctypes.c_uint32), ("num_tiles", ctypes.c_uint32),
+                ("pad", ctypes.c_uint32)]
+
+
+def batch_items(rows, num_groups, ctas):
+    """The work items (instance, first tile, tiles) of a batch of equal group counts, in the order they are claimed."""
+    plan = internal("_ZN2q110batch_planEPKNS_16BatchInstanceDevEjjjRSt6vectorINS_9BatchItemESaIS4_EERNS_11BatchParamsE", None,
+                    [ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_void_p, ctypes.c_void_p])
+    inst = (BatchInstance * len(rows))()
+    for i, n in enumerate(rows):
+        inst[i].rows, inst[i].num_groups, inst[i].mode = n, num_groups, 1
+    vector = (ctypes.c_void_p * 3)()          # an empty std::vector: first, last, end of storage
+    params = ctypes.create_string_buffer(4096)
+    plan(inst, len(rows), 0, ctas, vector, params)
+    n = ((vector[1] or 0) - (vector[0] or 0)) // ctypes.sizeof(BatchItem)
+    items = ctypes.cast(vector[0], ctypes.POINTER(BatchItem))
+    return [(items[i].instance, items[i].first_tile, items[i].num_tiles) for i in range(n)]
+
+
+@pytest.mark.parametrize("num_groups", [4, 64, 1024, 2500])
+@pytest.mark.parametrize("rows,most", [([1_000_003], 1.7), ([2_000_003], 1.5), ([4_000_003], 1.3), ([5_000_001], 1.3), ([8_000_003], 1.2),
+                                       ([20_000_001], 1.2), ([100_000_003], 1.1), ([100_003] * 8, 1.7),
+                                       ([2_500_001] * 2, 1.4), ([500_001] * 8, 1.4), ([1_000_001] * 16, 1.4)])
+def test_batch_pieces_even_out_the_ctas(num_groups, rows, most):
+    """Every tile is in one item, and CTAs that claim the items in turn end within `most` times an equal share (a piece
+    in two CTAs and none in the others' second turn made it twice the share)."""
+    ctas = 148
+    tiles = [-(-n // 2048) for n in rows]
+    items = batch_items(rows, num_groups, ctas)
+    for i, n in enumerate(tiles):
+        own = sorted((first, size) for inst, first, size in items if inst == i)
+        assert [first for first, _ in own] == [sum(size for _, size in own[:k]) for k in range(len(own))]
+        assert sum(size for _, size in own) == n
+        assert all(0 < size <= (1023 if num_groups <= 4 else 4096) for _, size in own)
+    busy = [0] * ctas
+    for _, _, size in items:
+        k = busy.index(min(busy))
+        busy[k] += size
+    assert max(busy) <= most * sum(tiles) / ctas

@@ -112,7 +112,7 @@ constexpr double kEngineCost[kEngines] = {1.0, 1.0, 1.33, 1.6, 8.4};
 
 // Work items: every instance in pieces of `chunk` tiles or, with chunk 0, of falling size: an engine's
 // largest instances first, each piece three quarters of an equal share of the tiles its engine's CTAs still
-// have to do, down to 16 tiles (a CTA's share, if that is less). At every change of
+// have to do, down to 16 tiles (less where a CTA's share is small, see below). At every change of
 // instance a CTA's teams wait for each other and flush the table, so most of the work is in few large
 // pieces, and the small ones at the end even out the CTAs. 64 instances of 10^4 to 10^7 rows with 4, 64
 // and 1024 groups: 245 us; the best of pieces of one size (64 tiles) 274, falling from half of the share
@@ -137,7 +137,13 @@ void plan_items(const BatchInstanceDev* inst, uint32_t n, uint32_t chunk, uint32
     for (uint32_t e = 0; e < kEngines; ++e) {
         std::stable_sort(of[e].begin(), of[e].end(), [&](uint32_t a, uint32_t c) { return inst[a].rows > inst[c].rows; });
         const double ctas = std::max(1.0, grid * (double)tiles[e] * kEngineCost[e] / std::max(1.0, total));
-        const uint64_t least = std::max<uint64_t>(2, std::min<uint64_t>(16, (uint64_t)(tiles[e] / ctas)));
+        // The share rounded up, so that small work is one piece for every CTA (rounded down, 4.0 M rows were 151
+        // pieces of 13 tiles for 148 CTAs, three of which took two); half of it above 16 tiles. One instance alone
+        // has nothing to flush between pieces: they fall to a sixteenth.
+        const uint64_t share = (uint64_t)std::ceil((double)tiles[e] / ctas);
+        const uint64_t least = of[e].size() == 1 ? std::max<uint64_t>(1, std::min<uint64_t>(4, share / 16))
+                               : share <= 16     ? std::max<uint64_t>(2, share)
+                                                 : std::min<uint64_t>(16, (share + 1) / 2);
         uint64_t left = tiles[e];
         for (uint32_t i : of[e]) {
             const uint64_t all = tiles_of(i);
