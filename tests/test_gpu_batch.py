@@ -378,3 +378,64 @@ def test_few_groups_take_no_longer_for_rows_alike(cuda, num_groups):
         torch.cuda.synchronize()
         q.lib().q1_batch_destroy(b)
     assert any_value < 1.5 * ordinary and alike < 1.5 * ordinary, (ordinary, any_value, alike)
+
+
+@pytest.mark.parametrize("num_groups", [65, 97, 500, 1023, 1024])
+def test_batch_cells_of_spaced_keys(cuda, num_groups):
+    """Keys of every step-th group: the (group, discount) cells' groups' words lie in an order of their own."""
+    rows = 100_003
+    inst = []
+    for step in [1, 32, 128]:
+        comp = gen_np.compress(gen_np.generate(700 + step, 0, rows))
+        inst.append((comp, gen_np.group_keys_uniform(700 + step, 0, rows, num_groups) // step * step, num_groups, 740000))
+    want = oracle_tables(inst)
+    arr, outs, keep = to_device(inst)
+    run_batch(arr, len(inst), _lib.BatchOpts(1, 0, 0, 0, None), torch.cuda.current_stream().cuda_stream)
+    for i in range(len(inst)):
+        assert np.array_equal(read(outs[i], num_groups), want[i])
+
+
+def test_cells_of_spaced_keys_take_no_longer(cuda):
+    """1024 groups, the keys multiples of 128, against spread keys (1.5 times allowed; with the groups' words in the
+    order of the groups, and so in one bank, 2.1 times)."""
+    rows, groups = 60_000_001, 1024
+    g = torch.Generator(device="cuda")
+    g.manual_seed(4)
+
+    def column(lo, hi, dtype):
+        return torch.randint(lo, hi, (rows,), generator=g, device="cuda", dtype=dtype)
+
+    cols = {"shipdate": column(0, 2500, torch.int16), "quantity": column(1, 51, torch.uint8),
+            "discount": column(0, 11, torch.uint8), "tax": column(0, 9, torch.uint8),
+            "extendedprice": column(90_000, 10_494_950, torch.int32), "keys": column(0, groups, torch.int32)}
+    out = torch.zeros(groups * 12, dtype=torch.int64, device="cuda")
+    bi = (_lib.BatchInstance * 1)()
+    for k in ["shipdate", "discount", "extendedprice", "tax", "quantity"]:
+        setattr(bi[0].cols, k, cols[k].data_ptr())
+    bi[0].keys, bi[0].rows, bi[0].cutoff_day, bi[0].num_groups = cols["keys"].data_ptr(), rows, 729999, groups
+    bi[0].aggregates = out.data_ptr()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    b = ctypes.c_void_p()
+    opts = _lib.BatchOpts(1, 0, 0, 0, None)
+    _lib.check(q.lib().q1_batch_create(bi, 1, ctypes.byref(opts), stream, ctypes.byref(b)))
+
+    def best():
+        times = []
+        for _ in range(8):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            for _ in range(3):
+                _lib.check(q.lib().q1_batch_run(b, stream))
+            ev[1].record()
+            torch.cuda.synchronize()
+            times.append(ev[0].elapsed_time(ev[1]))
+        return min(times)
+    try:
+        spread = best()
+        cols["keys"].copy_(cols["keys"] % 8 * 128)
+        spaced = best()
+        _lib.check(q.lib().q1_sync_check(stream))
+    finally:
+        torch.cuda.synchronize()
+        q.lib().q1_batch_destroy(b)
+    assert spaced < 1.5 * spread, (spread, spaced)

@@ -253,3 +253,15 @@ def test_wide_register_planes_flush_mid_launch(cuda, num_groups):
     keys = gen_np.group_keys_uniform(SEED + 17, 0, rows, num_groups)
     check(comp, keys, num_groups, 740000,
           run_gpu(c, keys, num_groups, "in_registers_per_thread", 740000, blocks=1))
+
+
+@pytest.mark.parametrize("num_groups", [65, 96, 97, 500, 993, 1023, 1024])
+@pytest.mark.parametrize("step", [1, 32, 128])
+def test_cell_tables_of_spaced_keys(table, num_groups, step):
+    """(group, discount) cells for keys of every step-th group, group counts on both sides of a multiple of 32 (the
+    groups' words lie in an order of their own)."""
+    comp, _, _ = table
+    wide = widen(comp, 31 + num_groups, 0.01)
+    c, keep = device_cols(wide)
+    keys = keys_for(num_groups, "uniform")[0] // step * step
+    check(wide, keys, num_groups, 740000, run_gpu(c, keys, num_groups, "shared_mem_per_thread", 740000))
