@@ -357,9 +357,9 @@ uint64_t q1_groupkey_scratch_bytes(uint32_t num_groups);
 
 /* Placements: IN_REGISTERS_PER_THREAD (num_groups <= 8; per-thread byte-plane sums),
  * SHARED_MEM_PER_THREAD (per-CTA shared-memory tables: (group, discount, tax) cells for
- * num_groups <= 64, (group, discount) cells for <= 1024, one slot per group for <= 4096; on
- * large tables of more than about 3100 groups a kernel reads 8192 sample rows and picks on the device
- * the shared-table pass (keys >= 4096 into global atomics), the global path (few passing rows over
+ * num_groups <= 64, (group, discount) cells for <= 1024, one slot per group for <= 4096; above 4096
+ * groups (from 4096 rows on; of about 3100 to 4096 groups on tables of 2^25 rows) a kernel reads 8192
+ * sample rows and picks on the device the shared-table pass (keys >= 4096 into global atomics), the global path (few passing rows over
  * spread keys) or, above 4096 groups, a two-pass radix partition of the passing rows into 8-byte records, 100 M rows
  * at a time, aggregated per partition of every 64th key in shared cells; every path gives the same
  * result), GLOBAL (global atomics for every row). Reads ship, qty, disc, tax, price of dev_cols

@@ -232,3 +232,39 @@ def test_path_choice_with_few_ctas_and_domain_edges(table, monkeypatch, num_grou
                 with pytest.raises(q.Q1Error) as e:
                     run_gpu(c, keys, num_groups, "shared_mem_per_thread", cutoff, blocks)
                 assert e.value.status == 6
+
+
+@pytest.mark.parametrize("rows", [20_011, 300_007, 1_000_003])
+def test_frequent_large_keys_take_no_longer(cuda, monkeypatch, rows):
+    """65,536 groups: tables whose rows are nearly all of one key, or of eight, that the single pass has no slot
+    for, against spread keys (4 times allowed; 1.0 M rows of one key took 78 times as long in the single pass)."""
+    monkeypatch.delenv("Q1_GROUPKEY_PATH", raising=False)
+    groups = 65536
+    comp = gen_np.compress(gen_np.generate(SEED + 40, 0, rows))
+    c, keep = device_cols(comp)
+    out = torch.zeros(groups * 12, dtype=torch.int64, device="cuda")
+    scratch = torch.zeros(int(q.lib().q1_groupkey_scratch_bytes(groups)) // 8 + 2, dtype=torch.int64, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def best(keys):
+        d = torch.from_numpy(keys.astype(np.uint32).view(np.int32).copy()).cuda()
+        times = []
+        for _ in range(8):
+            out.zero_()
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda._sleep(200_000)   # the launches are queued before the first begins
+            ev[0].record()
+            _lib.check(q.lib().q1_launch_groupkey(3, ctypes.byref(c), ctypes.c_void_p(d.data_ptr()), groups, rows, 740000,
+                                                  None, ctypes.c_void_p(scratch.data_ptr()),
+                                                  ctypes.c_void_p(out.data_ptr()), stream))
+            ev[1].record()
+            _lib.check(q.lib().q1_sync_check(stream))
+            times.append(ev[0].elapsed_time(ev[1]))
+        check(comp, keys, groups, 740000, out.cpu().numpy().view(np.uint64))
+        return min(times)
+
+    spread = gen_np.group_keys_uniform(SEED + 41, 0, rows, groups)
+    one = np.where(np.arange(rows) % 10, 50_000, spread).astype(np.uint32)
+    eight = (spread & 7) * 8000 + 5000
+    t = [best(k) for k in [spread, one, eight.astype(np.uint32)]]
+    assert t[1] < 4 * t[0] and t[2] < 4 * t[0], t

@@ -18,8 +18,8 @@
 //                            kernel with keys < 4096 in
 //                            slots and larger keys reduced straight into the global
 //                            accumulators, or the two-pass partitioned path of
-//                            groupkey_part.cu; above about 3100 groups the path is chosen on the
-//                            device from a sample of the rows of a large table
+//                            groupkey_part.cu; above 4096 groups, and above about 3100 on a large
+//                            table, the path is chosen on the device from a sample of the rows
 //                            (q1_groupkey_choose), which may be the global placement's, when few
 //                            rows pass over spread keys
 //   global                   every passing row reduces into the global accumulators
@@ -439,12 +439,11 @@ static bool takes_choice(int placement, uint32_t num_groups) {
 // Whether the path is chosen, by rows of the launch; elsewhere it is the single pass. The choice costs a
 // launch (10 us, 20 us before the partition's kernels) and the global path gains little on the tables:
 // with 1% of the rows passing, 200 M rows, 1030 groups 485 us against 406 with the table, 2500 groups 482
-// and 432, 4096 groups 396 and 497, where 25 M rows take 81 and 80. Above 4096 groups the partition gains
-// nothing on small tables: 65,536 uniform groups, all rows passing, 1.0 M rows 78 us chosen, 58 in a
-// single pass, 2.0 M rows 83 and 91 (Zipf keys 81 and 58).
+// and 432, 4096 groups 396 and 497, where 25 M rows take 81 and 80. Above 4096 groups a key without a slot
+// may hold most of the rows, 4.3 ns each in the single pass: it is chosen from 4096 rows on, where that is 18 us.
 static bool chosen_on_device(int placement, uint32_t num_groups, uint64_t rows) {
     return takes_choice(placement, num_groups) &&
-           rows >= (num_groups >= groupkey_part_min_groups() ? 3ull << 19 : 1ull << 25);
+           rows >= (num_groups >= groupkey_part_min_groups() ? 1ull << 12 : 1ull << 25);
 }
 
 // Chooses the path of the shared placement's largest tables (takes_choice) from 8192 evenly spaced
@@ -461,7 +460,9 @@ static bool chosen_on_device(int placement, uint32_t num_groups, uint64_t rows) 
 // the rows that pass with a cold key, p = fraction that pass): single pass 0.73 + 3.5 c + 0.35 p (Zipf
 // keys over 5,000 to 65,536 groups 1.08, 1.49, 1.90 at full pass; uniform ones, all cold, 6.1 to 6.8),
 // partitioned 0.56 + 0.75 p and 8 us for its three kernels (1.26 and 1.35 uniform and Zipf at full
-// pass, 0.65 at 7%). The single pass wins when (0.17 + 3.5 c - 0.4 p) x rows < 1.5 M.
+// pass, 0.65 at 7%). Rows of one cold key wait for each other in the single pass, 860 ms for 200 M (1.0 M rows, all
+// of one cold key, 4.38 ms): h is the fullest of 8192 bins of the sampled cold keys, less 12 samples that spread
+// keys put in one, as a fraction. The single pass wins when (0.17 + 3.5 c - 0.4 p + 860 h) x rows < 1.5 M.
 // All loads of a thread's eight samples are in flight together: one block of 256 threads taking them
 // one after another was 31 us, two thirds of a launch on 100,000 rows.
 __global__ void __launch_bounds__(1024) q1_groupkey_choose(const uint16_t* __restrict__ ship,
@@ -475,7 +476,12 @@ __global__ void __launch_bounds__(1024) q1_groupkey_choose(const uint16_t* __res
     }
     __shared__ uint32_t cnt[4];       // passing, cold, listed, largest key multiplicity
     __shared__ uint32_t list[kList];  // keys of the sampled passing rows
+    __shared__ uint32_t bins[K];      // sampled cold keys by hash
+    __shared__ uint32_t fullest;
     if (threadIdx.x < 4) cnt[threadIdx.x] = 0;
+    if (threadIdx.x == 0) fullest = 0;
+#pragma unroll
+    for (uint32_t e = 0; e < kPer; ++e) bins[e * 1024 + threadIdx.x] = 0;
     uint32_t day[kPer], key[kPer];
 #pragma unroll
     for (uint32_t e = 0; e < kPer; ++e) {
@@ -484,18 +490,24 @@ __global__ void __launch_bounds__(1024) q1_groupkey_choose(const uint16_t* __res
         key[e] = __ldg(keys + i);
     }
     __syncthreads();
-    uint32_t pass = 0, cold = 0;
+    uint32_t pass = 0, cold = 0, most = 0;
 #pragma unroll
     for (uint32_t e = 0; e < kPer; ++e) {
         const bool in = (int32_t)day[e] <= cutoff;
         pass += in ? 1u : 0u;
-        cold += in && key[e] >= hot ? 1u : 0u;
+        if (in && key[e] >= hot) {
+            ++cold;
+            most = max(most, atomicAdd(&bins[key[e] * 0x9E3779B1u >> 19], 1u) + 1u);
+        }
     }
+    static_assert(K == 1u << (32 - 19), "a bin of 13 bits");
     pass = __reduce_add_sync(0xffffffffu, pass);
     cold = __reduce_add_sync(0xffffffffu, cold);
+    most = __reduce_max_sync(0xffffffffu, most);
     if ((threadIdx.x & 31u) == 0) {
         atomicAdd(&cnt[0], pass);
         atomicAdd(&cnt[1], cold);
+        atomicMax(&fullest, most);
     }
     __syncthreads();
     const uint32_t P = cnt[0], C = cnt[1];
@@ -519,7 +531,9 @@ __global__ void __launch_bounds__(1024) q1_groupkey_choose(const uint16_t* __res
         } else if (!allow_part) {
             *mode = kModeSinglePass;
         } else {
-            const int64_t score = 170ll * K + 3500ll * C - 400ll * P;   // 1000 x (0.17 + 3.5 c - 0.4 p) x K
+            // 1000 x (0.17 + 3.5 c - 0.4 p + 860 h) x K, within 2^32, so that its product with the rows is exact
+            const int64_t score = min(170ll * K + 3500ll * C - 400ll * P + 860000ll * (fullest > 12 ? fullest - 12 : 0),
+                                      4000000000ll);
             *mode = score * (int64_t)rows < 1500000000ll * K ? kModeSinglePass : kModePartitioned;
         }
     }
