@@ -195,3 +195,72 @@ def test_uncompressed_int64_overflow_is_reported(cuda):
     with pytest.raises(q.Q1Error) as e:
         q.sync_check(stream)
     assert e.value.status == 6
+
+
+def any_flags(cols, seed):
+    """Return flag and line status independent of each other and of the dates: all six groups, A/O and
+    R/O among them, which TPC-H data does not have."""
+    rng = np.random.default_rng(seed)
+    n = len(cols["shipdate"])
+    out = dict(cols)
+    out["returnflag"] = np.frombuffer(b"ANR", "S1")[rng.integers(0, 3, n)]
+    out["linestatus"] = np.frombuffer(b"FO", "S1")[rng.integers(0, 2, n)]
+    return out
+
+
+@pytest.mark.parametrize("use_filter", [False, True])
+@pytest.mark.parametrize("placement", PLACEMENTS)
+@pytest.mark.parametrize("rows", [1, 4607, 5761, ROWS])
+def test_separate_flags_of_all_groups(cuda, wide_cols, placement, use_filter, rows):
+    cols = any_flags({k: v[:rows] for k, v in wide_cols.items()}, 71)
+    comp = gen_np.compress(cols, "sep")
+    if use_filter:
+        comp["filter"] = gen_np.filter_bitmap(comp["shipdate"], CUTOFF)
+    c, keep = device_compressed(comp)
+    buf = aggs_buffer()
+    stream = torch.cuda.current_stream().cuda_stream
+    q.launch_compressed(placement, c, rows, CUTOFF, use_filter, buf.data_ptr(), stream)
+    q.sync_check(stream)
+    want = oracle_table(cols)
+    assert np.array_equal(read(buf), want)
+    assert rows < 100 or all(int(want[g, 0]) for g in range(6))
+
+
+@pytest.mark.parametrize("placement", ["in_registers", "local_mem", "shared_mem_per_thread"])
+def test_separate_flags_maximal_rows_of_the_rare_groups(cuda, placement):
+    """One CTA, all rows of A/O or R/O with the largest bytes: a thread's entry of one of them takes up to
+    32,768 rows of a launch."""
+    rows = 384 * (1 << 15) + 4099
+    cols = maximal_rows(rows, 808)
+    cols["returnflag"] = np.frombuffer(b"AR", "S1")[(np.arange(rows) >= rows // 2).astype(np.int64)]
+    cols["linestatus"] = np.full(rows, b"O", "S1")
+    c, keep = device_compressed(gen_np.compress(cols, "sep"))
+    buf = aggs_buffer()
+    stream = torch.cuda.current_stream().cuda_stream
+    q.launch_compressed(placement, c, rows, CUTOFF, False, buf.data_ptr(), stream, config=_lib.LaunchConfig(0, 0, 1))
+    q.sync_check(stream)
+    assert np.array_equal(read(buf), oracle_table(cols))
+
+
+@pytest.mark.parametrize("placement", ["in_registers", "local_mem", "shared_mem_per_thread"])
+def test_separate_flags_of_any_kind_take_no_longer(cuda, placement):
+    """All six groups against the four of TPC-H data (4 times allowed; 18 times when the rows of the other two went
+    through 128-bit shared atomics)."""
+    rows = 4_000_003
+    cols = gen_np.generate(72, 0, rows)
+    stream = torch.cuda.current_stream().cuda_stream
+    best = []
+    for flags in [cols, any_flags(cols, 73)]:
+        c, keep = device_compressed(gen_np.compress(flags, "sep"))
+        buf = aggs_buffer()
+        times = []
+        for _ in range(10):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda._sleep(200_000)   # the launch is queued before the first event
+            ev[0].record()
+            q.launch_compressed(placement, c, rows, CUTOFF, False, buf.data_ptr(), stream)
+            ev[1].record()
+            q.sync_check(stream)
+            times.append(ev[0].elapsed_time(ev[1]))
+        best.append(min(times))
+    assert best[1] < 4 * best[0], best

@@ -202,7 +202,8 @@ struct AccPerThread {
 #pragma unroll
         for (int i = 0; i < kPlanes; ++i) gq[i].zero();
     }
-    // One passing row of a cold group, exactly, into the CTA's table.
+    // One passing row of a cold group, exactly, into the CTA's table: where the rows of those groups go
+    // unless the caller of add() and add_quad() has a place of its own for them.
     __device__ __forceinline__ void cold_row(uint32_t grp, uint32_t q, uint32_t d, uint32_t a, uint32_t ab,
                                              uint32_t p) {
         unsigned long long* v = red + 2 * (grp * kNumAggs);
@@ -213,13 +214,31 @@ struct AccPerThread {
         atomic_add_u128_shared(v + 2 * kAggDiscPrice, (uint64_t)a * p, 0);
         atomic_add_u128_shared(v + 2 * kAggCharge, (uint64_t)ab * p, 0);
     }
+    struct ToCta {
+        AccPerThread& acc;
+        __device__ __forceinline__ void row(uint32_t grp, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) const {
+            acc.cold_row(grp, q, d, a, ab, p);
+        }
+        __device__ __forceinline__ void quad(const Quad& x) const {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const uint32_t b = (x.OH >> (8 * r)) & 0x22u;
+                if (b) acc.cold_row((b & 2u) ? 1u : 5u, (x.Q >> (8 * r)) & 0xFFu, (x.D >> (8 * r)) & 0xFFu, x.a[r], x.ab[r], x.p[r]);
+            }
+        }
+    };
     __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
+        add(c, q, d, a, ab, p, ToCta{*this});
+    }
+    template <class Cold>
+    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p,
+                                        Cold&& cold_to) {
         if constexpr (kWideQty) {
 #pragma unroll
             for (int i = 0; i < G; ++i) g[i].add(c == (uint32_t)i, q, d, a, ab, p);
         } else {
             if (kCold && (c == 1u || c == 5u)) {
-                cold_row(c, q, d, a, ab, p);
+                cold_to.row(c, q, d, a, ab, p);
                 return;
             }
             // one row through the quad path (tail rows)
@@ -239,27 +258,21 @@ struct AccPerThread {
         }
     }
     // Called by all lanes of the warp.
-    template <bool kTop>
-    __device__ __forceinline__ void add_quad_planes(const Quad& x) {
+    template <bool kTop, class Cold>
+    __device__ __forceinline__ void add_quad_planes(const Quad& x, Cold&& cold_to) {
 #pragma unroll
         for (int i = 0; i < kPlanes; ++i) gq[i].template add_quad<kTop>(x.OH, group_of(i), x);
         if constexpr (kCold) {
-            if (__any_sync(0xffffffffu, x.OH & 0x22222222u)) {
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const uint32_t b = (x.OH >> (8 * r)) & 0x22u;
-                    if (b)
-                        cold_row((b & 2u) ? 1u : 5u, (x.Q >> (8 * r)) & 0xFFu, (x.D >> (8 * r)) & 0xFFu, x.a[r],
-                                 x.ab[r], x.p[r]);
-                }
-            }
+            if (__any_sync(0xffffffffu, x.OH & 0x22222222u)) cold_to.quad(x);
         }
     }
-    __device__ __forceinline__ void add_quad(const Quad& x) {
+    __device__ __forceinline__ void add_quad(const Quad& x) { add_quad(x, ToCta{*this}); }
+    template <class Cold>
+    __device__ __forceinline__ void add_quad(const Quad& x, Cold&& cold_to) {
         if constexpr (!kWideQty) {
             // the prices' top byte plane is zero for the whole warp unless a price is >= 2^24
-            if (__any_sync(0xffffffffu, x.P[3])) add_quad_planes<true>(x);
-            else add_quad_planes<false>(x);
+            if (__any_sync(0xffffffffu, x.P[3])) add_quad_planes<true>(x, cold_to);
+            else add_quad_planes<false>(x, cold_to);
         }
     }
     // plane slot of group i (not called for cold groups)
@@ -289,73 +302,6 @@ struct AccPerThread {
     }
 };
 
-// The other placements keep their table elsewhere and write-combine: a thread sums its rows of some
-// tiles in registers (AccPerThread, four rows an instruction), then adds the sums to the table.
-// Adding every quad or row to the table directly made the table the bound: 600 M pair-layout rows
-// took 1.95 ms (in_registers: every lane of a table read all of its rows), 2.13 ms
-// (shared_mem_per_thread) and 3.19 ms (local_mem) against 0.88 ms in registers.
-template <int G, bool kWideQty>
-struct AccCombining {
-    AccPerThread<G, kWideQty> buf;
-    uint32_t tiles;   // in buf
-    __device__ __forceinline__ void init_buffer(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
-        buf.init(lane, ctid, scratch, red);
-        tiles = 0;
-    }
-    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
-        buf.add(c, q, d, a, ab, p);
-    }
-    __device__ __forceinline__ void add_quad(const Quad& x) { buf.add_quad(x); }
-    // Whether the buffer goes to the table now; called by all lanes after each tile.
-    __device__ __forceinline__ bool due() {
-        if (++tiles < kCombineTiles) return false;
-        tiles = 0;
-        return true;
-    }
-};
-
-// --- in_registers ("warp-lane tables", src/kernels/ht_in_registers.cuh:30-121): lane g of a warp
-// holds group g's sums in registers; the warp's buffers meet there through warp reductions. (In
-// the reference all lanes of a table read the same rows, each keeping those of its group.)
-template <int G, bool kWideQty>
-struct AccWarpLane : AccCombining<G, kWideQty> {
-    // lane g: group g. A launch gives a warp at most 2^20 rows: the charge sum takes 128 bits
-    // (2^47.2 a row), the others 64.
-    uint64_t t[kNumAggs], ch_hi;
-    __device__ __forceinline__ void init(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
-        this->init_buffer(lane, ctid, scratch, red);
-#pragma unroll
-        for (int a = 0; a < kNumAggs; ++a) t[a] = 0;
-        ch_hi = 0;
-    }
-    __device__ __forceinline__ void to_table(uint32_t lane) {
-#pragma unroll
-        for (int i = 0; i < G; ++i) {
-#pragma unroll
-            for (int a = 0; a < kNumAggs; ++a) {
-                const uint64_t v = warp_sum_agg<kWideQty>(a, this->buf.value(i, a)).lo;
-                if (lane == (uint32_t)i) {
-                    t[a] += v;
-                    if (a == kAggCharge) ch_hi += t[a] < v ? 1u : 0u;
-                }
-            }
-            this->buf.zero_group(i);
-        }
-    }
-    template <class P>
-    __device__ __forceinline__ void tile_done(const P&, uint32_t lane) {
-        if (this->due()) to_table(lane);
-    }
-    template <class P>
-    __device__ __forceinline__ void finish(const P&, uint32_t lane) { to_table(lane); }
-    __device__ __forceinline__ void flush(WarpRecord rec, uint32_t lane) {
-        if (lane < (uint32_t)G) {
-#pragma unroll
-            for (int a = 0; a < kNumAggs; ++a) rec.set((int)lane, a, Sum128{t[a], a == kAggCharge ? ch_hi : 0ull});
-        }
-    }
-};
-
 // A group's entry in the per-thread tables below: count, quantity and discount in one word (a thread
 // adds at most 2^15 rows per launch, so count < 2^16, quantity <= 255 * 2^15 < 2^23, discount
 // <= 100 * 2^15 < 2^22), then price, (100 - d) price and (100 - d)(100 + t) price. Reference-typed
@@ -380,6 +326,31 @@ struct Entry {
             default: return b.value(i, kAggQty);
         }
     }
+    // One row of compressed columns added to an entry, word(j) its word j.
+    template <class Word>
+    static __device__ __forceinline__ void add_row(Word&& word, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
+        word(0) = word(0) + (1ull | (uint64_t)q << kQtyShift | (uint64_t)d << kDiscShift);
+        word(1) = word(1) + p;
+        word(2) = mad_wide(a, p, word(2));
+        word(3) = mad_wide(ab, p, word(3));
+    }
+    // The rows of a quad with byte r of `rows` 1 (0 in the others).
+    template <class Word>
+    static __device__ __forceinline__ void add_quad(Word&& word, uint32_t rows, const Quad& x) {
+        uint64_t p = 0, dp = 0, ch = 0;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const uint32_t pr = (rows >> (8 * r)) & 1u ? x.p[r] : 0u;
+            p += pr;
+            dp = mad_wide(x.a[r], pr, dp);
+            ch = mad_wide(x.ab[r], pr, ch);
+        }
+        word(0) = word(0) + ((uint64_t)__popc(rows) | (uint64_t)__dp4a(rows, x.Q, 0u) << kQtyShift |
+                             (uint64_t)__dp4a(rows, x.D, 0u) << kDiscShift);
+        word(1) = word(1) + p;
+        word(2) = word(2) + dp;
+        word(3) = word(3) + ch;
+    }
     // aggregate a of the words w
     static __device__ __forceinline__ uint64_t value(const uint64_t w[kWords], int a) {
         switch (a) {
@@ -401,6 +372,124 @@ struct Entry {
     }
 };
 
+// Where rows of the cold groups (codes 1 and 5) go in a placement with per-thread entries: word(group, j) is word j
+// of the thread's entry of that group. (The groups are constants, which keeps a table that lies in local memory
+// apart from the rest of its accumulator.)
+template <class E, class Word>
+struct ToEntries {
+    Word word;
+    __device__ __forceinline__ void row(uint32_t grp, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) const {
+        if (grp == 1u) E::add_row([&](uint32_t j) -> auto& { return word(1u, j); }, q, d, a, ab, p);
+        else E::add_row([&](uint32_t j) -> auto& { return word(5u, j); }, q, d, a, ab, p);
+    }
+    __device__ __forceinline__ void quad(const Quad& x) const {
+        const uint32_t one = (x.OH >> 1) & 0x01010101u, five = (x.OH >> 5) & 0x01010101u;
+        if (one) E::add_quad([&](uint32_t j) -> auto& { return word(1u, j); }, one, x);
+        if (five) E::add_quad([&](uint32_t j) -> auto& { return word(5u, j); }, five, x);
+    }
+};
+template <class E, class Word>
+__device__ __forceinline__ ToEntries<E, Word> to_entries(Word word) { return ToEntries<E, Word>{word}; }
+
+// The other placements keep their table elsewhere and write-combine: a thread sums its rows of some
+// tiles in registers (AccPerThread, four rows an instruction), then adds the sums to the table.
+// Adding every quad or row to the table directly made the table the bound: 600 M pair-layout rows
+// took 1.95 ms (in_registers: every lane of a table read all of its rows), 2.13 ms
+// (shared_mem_per_thread) and 3.19 ms (local_mem) against 0.88 ms in registers. Rows of the two groups that
+// AccPerThread has no planes for go to entries of the thread's own, where the placement has such. (Separate flags
+// with line status at random, a quarter of the rows of those groups, 4.0 M rows: 24 to 28 us; into the CTA's
+// table, by 128-bit shared atomics, 270 to 296.)
+template <int G, bool kWideQty>
+struct AccCombining {
+    AccPerThread<G, kWideQty> buf;
+    uint32_t tiles;   // in buf
+    __device__ __forceinline__ void init_buffer(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
+        buf.init(lane, ctid, scratch, red);
+        tiles = 0;
+    }
+    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
+        buf.add(c, q, d, a, ab, p);
+    }
+    __device__ __forceinline__ void add_quad(const Quad& x) { buf.add_quad(x); }
+    // Whether the buffer goes to the table now; called by all lanes after each tile.
+    __device__ __forceinline__ bool due() {
+        if (++tiles < kCombineTiles) return false;
+        tiles = 0;
+        return true;
+    }
+};
+
+// --- in_registers ("warp-lane tables", src/kernels/ht_in_registers.cuh:30-121): lane g of a warp
+// holds group g's sums in registers; the warp's buffers meet there through warp reductions. (In
+// the reference all lanes of a table read the same rows, each keeping those of its group.)
+template <int G, bool kWideQty, uint32_t kThreads>
+struct AccWarpLane : AccCombining<G, kWideQty> {
+    using E = Entry<kWideQty>;
+    static constexpr bool kCold = AccPerThread<G, kWideQty>::kCold;
+    // lane g: group g. A launch gives a warp at most 2^20 rows: the charge sum takes 128 bits
+    // (2^47.2 a row), the others 64.
+    uint64_t t[kNumAggs], ch_hi;
+    uint64_t* cold_tab;   // this thread's column of [word][cold group][thread]
+    static constexpr uint32_t kTableBytes = kCold ? 8u * E::kWords * 2u * kThreads : 0u;
+    __device__ __forceinline__ uint64_t& cold_entry(uint32_t grp, uint32_t j) {
+        return cold_tab[(2u * j + (grp == 1u ? 0u : 1u)) * kThreads];
+    }
+    __device__ __forceinline__ void init(uint32_t lane, uint32_t ctid, uint8_t* scratch, unsigned long long* red) {
+        this->init_buffer(lane, ctid, scratch, red);
+#pragma unroll
+        for (int a = 0; a < kNumAggs; ++a) t[a] = 0;
+        ch_hi = 0;
+        if constexpr (kCold) {
+            cold_tab = reinterpret_cast<uint64_t*>(scratch) + ctid;
+#pragma unroll
+            for (uint32_t j = 0; j < 2u * E::kWords; ++j) cold_tab[j * kThreads] = 0;
+        }
+    }
+    __device__ __forceinline__ auto cold() {
+        return to_entries<E>([this](uint32_t grp, uint32_t j) -> uint64_t& { return cold_entry(grp, j); });
+    }
+    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
+        this->buf.add(c, q, d, a, ab, p, cold());
+    }
+    __device__ __forceinline__ void add_quad(const Quad& x) { this->buf.add_quad(x, cold()); }
+    __device__ __forceinline__ void to_table(uint32_t lane) {
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            if (this->buf.cold(i)) continue;
+#pragma unroll
+            for (int a = 0; a < kNumAggs; ++a) {
+                const uint64_t v = warp_sum_agg<kWideQty>(a, this->buf.value(i, a)).lo;
+                if (lane == (uint32_t)i) {
+                    t[a] += v;
+                    if (a == kAggCharge) ch_hi += t[a] < v ? 1u : 0u;
+                }
+            }
+            this->buf.zero_group(i);
+        }
+    }
+    template <class P>
+    __device__ __forceinline__ void tile_done(const P&, uint32_t lane) {
+        if (this->due()) to_table(lane);
+    }
+    template <class P>
+    __device__ __forceinline__ void finish(const P&, uint32_t lane) { to_table(lane); }
+    __device__ __forceinline__ void flush(WarpRecord rec, uint32_t lane) {
+        if (lane < (uint32_t)G && !(kCold && this->buf.cold((int)lane))) {
+#pragma unroll
+            for (int a = 0; a < kNumAggs; ++a) rec.set((int)lane, a, Sum128{t[a], a == kAggCharge ? ch_hi : 0ull});
+        }
+        if constexpr (kCold) {
+#pragma unroll
+            for (int i = 1; i <= 5; i += 4) {
+                uint64_t w[E::kWords];
+#pragma unroll
+                for (int j = 0; j < E::kWords; ++j) w[j] = cold_entry((uint32_t)i, j);
+                E::reduce(w, i, rec, lane);
+            }
+        }
+    }
+};
+
 // --- local_mem (src/kernels/ht_in_local_mem.cuh:11-74): per-thread tables in (L1-cached) local
 // memory.
 template <int G, bool kWideQty>
@@ -412,6 +501,13 @@ struct AccLocal : AccCombining<G, kWideQty> {
         for (int i = 0; i < G; ++i)
             for (int j = 0; j < E::kWords; ++j) t[i][j] = 0;
     }
+    __device__ __forceinline__ auto cold() {
+        return to_entries<E>([this](uint32_t grp, uint32_t j) -> volatile uint64_t& { return t[grp < G ? grp : 0][j]; });
+    }
+    __device__ __forceinline__ void add(uint32_t c, uint32_t q, uint32_t d, uint32_t a, uint32_t ab, uint32_t p) {
+        this->buf.add(c, q, d, a, ab, p, cold());
+    }
+    __device__ __forceinline__ void add_quad(const Quad& x) { this->buf.add_quad(x, cold()); }
     __device__ __forceinline__ void to_table() {
 #pragma unroll
         for (int i = 0; i < G; ++i) {
@@ -432,7 +528,7 @@ struct AccLocal : AccCombining<G, kWideQty> {
         for (int i = 0; i < G; ++i) {
             uint64_t w[E::kWords];
 #pragma unroll
-            for (int j = 0; j < E::kWords; ++j) w[j] = t[i][j];   // (zero in a cold group's entry)
+            for (int j = 0; j < E::kWords; ++j) w[j] = t[i][j];
             E::reduce(w, i, rec, lane);
         }
     }
@@ -463,9 +559,13 @@ struct AccSharedPerThread : AccCombining<G, kWideQty> {
                 entry(c, 3) = mad_wide(ab, p, entry(c, 3));
             }
         } else {
-            this->buf.add(c, q, d, a, ab, p);
+            this->buf.add(c, q, d, a, ab, p, cold());
         }
     }
+    __device__ __forceinline__ auto cold() {
+        return to_entries<E>([this](uint32_t grp, uint32_t j) -> uint64_t& { return entry(grp, j); });
+    }
+    __device__ __forceinline__ void add_quad(const Quad& x) { this->buf.add_quad(x, cold()); }
     __device__ __forceinline__ void to_table() {
         if constexpr (!kWideQty) {
 #pragma unroll
@@ -488,7 +588,7 @@ struct AccSharedPerThread : AccCombining<G, kWideQty> {
         for (int i = 0; i < G; ++i) {
             uint64_t w[E::kWords];
 #pragma unroll
-            for (int j = 0; j < E::kWords; ++j) w[j] = entry(i, j);   // (zero in a cold group's entry)
+            for (int j = 0; j < E::kWords; ++j) w[j] = entry(i, j);
             E::reduce(w, i, rec, lane);
         }
     }
@@ -530,7 +630,7 @@ struct AccGlobal : AccCombining<G, kWideQty> {
 
 template <int P, int G, bool W, uint32_t T>
 struct AccSel;
-template <int G, bool W, uint32_t T> struct AccSel<kPlaceInRegisters, G, W, T> { using A = AccWarpLane<G, W>; };
+template <int G, bool W, uint32_t T> struct AccSel<kPlaceInRegisters, G, W, T> { using A = AccWarpLane<G, W, T>; };
 template <int G, bool W, uint32_t T> struct AccSel<kPlaceInRegistersPerThread, G, W, T> { using A = AccPerThread<G, W>; };
 template <int G, bool W, uint32_t T> struct AccSel<kPlaceLocalMem, G, W, T> { using A = AccLocal<G, W>; };
 template <int G, bool W, uint32_t T> struct AccSel<kPlaceSharedMemPerThread, G, W, T> { using A = AccSharedPerThread<G, W, T>; };
@@ -884,7 +984,10 @@ static cudaError_t launch_sized(const ScanParams& prm, int sm_count, int max_blo
     constexpr uint32_t W = kConsumerWarps<L, P, kWide>;
     constexpr int G = LayoutTraits<L>::kCodes;
     constexpr uint32_t dyn =
-        S * stage_bytes<L>(R) + (P == kPlaceSharedMemPerThread ? 8u * Entry<L == kLayUncomp>::kWords * G * W * 32u : 0u);
+        S * stage_bytes<L>(R) +
+        (P == kPlaceSharedMemPerThread ? 8u * Entry<L == kLayUncomp>::kWords * G * W * 32u
+         : P == kPlaceInRegisters      ? AccWarpLane<G, L == kLayUncomp, W * 32u>::kTableBytes
+                                       : 0u);
     static_assert(dyn + sizeof(ulonglong2) * W * G * kNumAggs + 2048 <= 227 * 1024, "ring and tables beside the static shared memory");
     cudaError_t e = cudaFuncSetAttribute(q1_scan_kernel<L, P, kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
     if (e != cudaSuccess) return e;
