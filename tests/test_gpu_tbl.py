@@ -183,3 +183,65 @@ def test_missing_file(cuda, tmp_path):
     with pytest.raises(q.Q1Error) as e:
         q.tbl_read_file(str(tmp_path / "absent.tbl"))
     assert e.value.status == 1 and "cannot open" in str(e.value)
+
+
+SHORTEST = b"||||1|2|3|4|A|F|1992-1-1"
+
+
+@pytest.mark.parametrize("kind", ["shortest", "short", "mixed", "long"])
+@pytest.mark.parametrize("offset", [0, 7])
+def test_lines_of_any_length_match_oracle(cuda, kind, offset):
+    """Lines as short as one that parses can be (more than the newline search lists for dbgen text), long ones whose
+    fields end in the next tile or lie beyond what is staged, and both, the last one without a newline."""
+    r = np.random.default_rng(len(kind) + offset)
+    usual = q.tbl_format(q.generate_host(48, 0, 500)).split(b"\n")[:-1]
+    lines = []
+    for i in range(60_000 if kind in ("shortest", "short") else 8000):
+        if kind == "shortest" or (kind == "mixed" and i % 3):
+            lines.append(SHORTEST)
+        elif kind == "short":
+            lines.append(SHORTEST + b"|" * int(r.integers(0, 9)))
+        else:
+            p = usual[i % 500].split(b"|")
+            p[0] = p[0].rjust(int(r.integers(1, 400)), b"0")
+            p[-1] = b"c" * int(r.integers(0, 900))
+            lines.append(b"|".join(p))
+    text = b"\n".join(lines)
+    want, wrows, bad, _ = O.parse_tbl(text)
+    got, rows, st, msg = gpu_parse(text, offset=offset)
+    assert st == 0, msg
+    assert rows == wrows == len(lines) and bad == 0
+    check_same(got, want)
+
+
+def time_parses(texts, rows):
+    """Best time of a parse of each text, by events around the call."""
+    L = q.lib()
+    out = {k: torch.zeros(rows, dtype=t, device="cuda") for k, t in [
+        ("shipdate", torch.int32), ("returnflag", torch.uint8), ("linestatus", torch.uint8), ("discount", torch.int64),
+        ("tax", torch.int64), ("extendedprice", torch.int64), ("quantity", torch.int64)]}
+    o = _lib.ColumnsOut(*[v.data_ptr() for v in out.values()])
+    got = ctypes.c_uint64(0)
+    best = []
+    for text in texts:
+        dev = torch.frombuffer(bytearray(text), dtype=torch.uint8).cuda()
+        times = []
+        for _ in range(10):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            _lib.check(L.q1_tbl_parse_device(ctypes.c_void_p(dev.data_ptr()), len(text), ctypes.byref(o), rows,
+                                             ctypes.byref(got), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            ev[1].record()
+            torch.cuda.synchronize()
+            times.append(ev[0].elapsed_time(ev[1]))
+        assert got.value == rows
+        best.append(min(times))
+    return best
+
+
+def test_short_lines_take_no_longer(cuda):
+    """300,000 lines of 24 bytes against dbgen's (4 times allowed; they took 25 times as long when they were walked
+    without a list of their starts)."""
+    rows = 300_000
+    t = time_parses([q.tbl_format(q.generate_host(49, 0, rows)), (SHORTEST + b"\n") * rows], rows)
+    assert t[1] < 4 * t[0], t

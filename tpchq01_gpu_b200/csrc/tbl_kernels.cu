@@ -59,12 +59,14 @@ constexpr uint32_t kAhead = 128;                     // bytes after the tile kep
 constexpr uint32_t kFront = 16;                      // room before the tile for right-aligned field loads
 constexpr uint32_t kStageBytes = kFront + kTile + kAhead;
 constexpr uint32_t kRing = 3;                        // tiles in flight or in use a CTA
-constexpr uint32_t kWarpList = 96;                   // line starts listed a part (about 28 in dbgen text)
+constexpr uint32_t kWarpList = 192;                  // line starts listed a part (about 28 in dbgen text)
 static_assert(kStageBytes % 16 == 0, "stages stay 16-byte aligned");
 static_assert(kSubs % 2 == 1, "conflict-free loads of a lane's consecutive bytes");
-static_assert(kWarpList >= 64, "two newlines a lane");
+// The shortest line that parses is four empty fields, "1|1|1|1|A|F|1-1-1" and a newline. (Lists of 96, which left lines
+// of 25 bytes to the walk without a list: 1.0 M of them 2,630 us instead of 126.)
+static_assert(kWarpList >= 64 && kWarpList > kWarpBytes / 22, "every line that parses is listed");
 static_assert(kRing == 3, "a tile reloads the stage of the tile before it");
-static_assert(kTile <= 65535, "a tile's newlines fit 16 bits");
+static_assert(kTile + kAhead + 1 <= 65535, "a tile's newlines and line starts fit 16 bits");
 
 // Bit 7 of byte i set iff byte i of w equals the byte repeated in c4 (below 128; exact for every w).
 __device__ __forceinline__ uint32_t equal_bytes(uint32_t w, uint32_t c4) {
@@ -419,8 +421,8 @@ __global__ void __launch_bounds__(tbl::kThreads, 1) tbl_parse_kernel(const char*
     __shared__ __align__(8) uint64_t full_bar[kRing];
     __shared__ __align__(8) uint64_t prefix_bar;
     __shared__ unsigned long long tile_of[kRing];
-    __shared__ uint32_t starts[kWorkers * kWarpList + 2];       // line starts in the tile, in text order, then the next one
-    __shared__ uint32_t warp_starts[kWorkers][kWarpList];   // the line starts of each worker's part, in order
+    __shared__ uint16_t starts[kWorkers * kWarpList + 2];   // line starts in the tile, in text order, then the next one
+    __shared__ uint16_t warp_starts[kWorkers][kWarpList];   // the line starts of each worker's part, in order
     __shared__ uint32_t warp_lines[2][32];       // newlines of each worker's part, by tile parity
     __shared__ uint64_t prefix_s[2];             // newlines before the tile, by tile parity
     __shared__ uint32_t months[16];
