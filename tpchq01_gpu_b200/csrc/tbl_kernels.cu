@@ -1,5 +1,5 @@
 // lineitem text ingestion on the GPU: the reference's lineitem::FromFile (cpu/tpch_kit.cpp:155-172
-// with the TableReader tokenizer at :10-99) as three kernels over a device copy of the text.
+// with the TableReader tokenizer at :10-99) as one kernel over a device copy of the text.
 //
 // Format (dbgen .tbl): one row per '\n'-terminated line (the last line may lack the '\n'), fields
 // separated by '|'. Fields 5-11 (1-based) are read, the others skipped:
@@ -15,19 +15,23 @@
 // reports the count and the first malformed line's byte offset.
 //
 // Kernels:
-//   tbl_count_kernel  newlines of the whole text (16-byte loads, byte compares on 32-bit words)
+//   tbl_count_kernel  newlines of the whole text, where only they are asked for (16-byte loads, byte
+//                     compares on 32-bit words)
 //   tbl_parse_kernel  one pass over the text. One persistent CTA per SM takes 63 KB tiles in ticket
 //                     order and streams them into shared memory with bulk copies (three stages).
 //                     Workers find the next tile's newlines with word compares and rank them by
 //                     ballots, then parse the current tile's lines, a line a lane, word by word from
-//                     shared memory (parse_fast; any other form goes to the byte-wise parse_line).
+//                     shared memory (parse_fast; any other form goes to the byte-wise parse_line,
+//                     which reads shared memory too unless the line ends beyond the stage).
 //                     A control warp meanwhile sums the newlines before the tile from the counts the
 //                     other CTAs published (decoupled look-back, bounded).
 //
 // What bounds it: instructions, 28 warp instructions a line at half of the issue slots. 6.0 M rows of
 // dbgen text (757 MB, 1.0 GB with the columns, 0.15 ms at the copy bandwidth) take 0.31 ms a call;
 // counting, scanning the counts and parsing byte by byte in three kernels took 1.62 ms (142 warp
-// instructions a line, the text read twice). 10,000 rows: 91 -> 37 us. Measured on the way: tiles of
+// instructions a line, the text read twice). 10,000 rows: 91 -> 37 us. Lines of other forms, 1.0 M rows: a sign
+// before every price 217 us (read again from the text instead of from shared memory 348, three kernels 352),
+// 40 characters in the first two fields 341 (542, 389), all as dbgen writes them 88 (354). Measured on the way: tiles of
 // 30 KB with two CTAs an SM 0.36 to 0.59 ms (twice the tiles to order), a look-back step of 256 tiles
 // 0.1 ms more than one of 64, the newline search with 512 bytes a load across the warp 0.39 ms.
 #include <cuda_runtime.h>
@@ -98,8 +102,11 @@ __device__ __forceinline__ int32_t day_number(int32_t y, int32_t m, int32_t d) {
 // Reads a line through a 16-byte window: one aligned 16-byte load per 16 bytes of the line
 // (lanes of a warp read different lines, so every load touches a different cache line; byte
 // loads would cost one L1 wavefront per byte). Offsets are 32-bit and relative to the line's
-// start (a line whose first eleven fields span more than 2^31 bytes reads as malformed). The
-// last, partial 16-byte block of the buffer is read bytewise so that no load goes past its end.
+// start (a line whose first eleven fields span more than 2^31 bytes reads as malformed).
+// kStaged: the line lies in a tile's stage in shared memory, which may be read to its last block.
+// Else it lies in the text, whose last, partial 16-byte block is read bytewise so that no load goes
+// past its end.
+template <bool kStaged>
 struct Cursor {
     const char* __restrict__ line;   // the line's first byte
     const uint4* __restrict__ blk;   // 16-byte blocks from the one holding line[0]
@@ -108,12 +115,11 @@ struct Cursor {
     uint32_t full;                   // blocks [0, full) lie wholly inside the buffer
     uint32_t wi = 0xFFFFFFFFu;       // block in the window
     uint4 win;
-    __device__ __forceinline__ Cursor(const char* __restrict__ text, uint64_t s, uint64_t bytes) {
-        line = text + s;
+    __device__ __forceinline__ Cursor(const char* __restrict__ first, uint64_t rest) {
+        line = first;
         const uintptr_t a = reinterpret_cast<uintptr_t>(line);
         off = (uint32_t)(a & 15u);
         blk = reinterpret_cast<const uint4*>(a - off);
-        const uint64_t rest = bytes - s;
         end = rest < 0x7FFFFFFFull ? (uint32_t)rest : 0x7FFFFFFFu;
         full = (uint32_t)(((uint64_t)off + end) >> 4);
         p = 0;
@@ -121,9 +127,9 @@ struct Cursor {
     __device__ __forceinline__ int peek() {
         if (p >= end) return -1;
         const uint32_t a = off + p, bi = a >> 4;
-        if (bi >= full) return (int)(unsigned char)line[p];
+        if (!kStaged && bi >= full) return (int)(unsigned char)line[p];
         if (bi != wi) {
-            win = __ldg(blk + bi);
+            win = kStaged ? blk[bi] : __ldg(blk + bi);
             wi = bi;
         }
         const uint32_t o = a & 15u;
@@ -208,9 +214,11 @@ struct Row {
     char rf, ls;
 };
 
-// Parses the line starting at byte s of the text, any form; false (row zeroed) if malformed.
-__device__ __noinline__ bool parse_line(const char* __restrict__ text, uint64_t bytes, uint64_t s, Row& r) {
-    Cursor c(text, s, bytes);
+// Parses the line at `first`, any form, with `rest` bytes up to the end of the text (kStaged: of the line); false (row
+// zeroed) if malformed.
+template <bool kStaged>
+__device__ __noinline__ bool parse_line(const char* __restrict__ first, uint64_t rest, Row& r) {
+    Cursor<kStaged> c(first, rest);
     r = Row{0, 0, 0, 0, 0, 0, 0};
     bool ok = c.skip_field() && c.skip_field() && c.skip_field() && c.skip_field();
     ok = ok && c.decimal(r.qty) && c.sep() && c.decimal(r.price) && c.sep() && c.decimal(r.disc) && c.sep() &&
@@ -531,10 +539,11 @@ __global__ void __launch_bounds__(tbl::kThreads, 1) tbl_parse_kernel(const char*
         }
     };
     // The line at byte `at` of the text, of any form, into row i (newlines before it); counted when
-    // malformed or past the capacity.
-    auto put_any = [&](uint64_t i, uint64_t at) {
+    // malformed or past the capacity. staged, size: the line in shared memory, if it lies there whole.
+    auto put_any = [&](uint64_t i, uint64_t at, const uint8_t* staged = nullptr, uint32_t size = 0) {
         Row row;
-        const bool good = parse_line(text, bytes, at, row);
+        const bool good = staged ? parse_line<true>(reinterpret_cast<const char*>(staged), size, row)
+                                 : parse_line<false>(text + at, bytes - at, row);
         if (i < capacity) {
             o.ship[i] = row.ship;
             o.qty[i] = row.qty;
@@ -656,7 +665,8 @@ __global__ void __launch_bounds__(tbl::kThreads, 1) tbl_parse_kernel(const char*
                         o.ls[i] = (char)(row.flags >> 8);
                     } else if (j < lines) {
                         const uint64_t at = k * kTile + starts[j];
-                        if (at < end) put_any(i, at - off);
+                        const uint32_t next = starts[j + 1];
+                        if (at < end) put_any(i, at - off, next <= kTile + kAhead ? buf + starts[j] : nullptr, next - starts[j]);
                     }
                 }
             }
