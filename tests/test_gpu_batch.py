@@ -439,3 +439,15 @@ def test_cells_of_spaced_keys_take_no_longer(cuda):
         torch.cuda.synchronize()
         q.lib().q1_batch_destroy(b)
     assert spaced < 1.5 * spread, (spread, spaced)
+
+
+@pytest.mark.parametrize("chunk", [1, 7, 1000, 100_000])
+def test_describe_reports_the_chunk_asked_for(cuda, chunk):
+    """Also one larger than any instance, or than a work item may be; without one, the largest piece."""
+    inst = [x for x in make_instances(seed=5, n=30) if len(x[1])]
+    arr, outs, keep = to_device(inst)
+    stream = torch.cuda.current_stream().cuda_stream
+    desc, _ = run_batch(arr, len(inst), _lib.BatchOpts(1, 0, chunk, 0, None), stream, runs=1)
+    assert desc.chunk_tiles == chunk
+    desc, _ = run_batch(arr, len(inst), _lib.BatchOpts(1, 0, 0, 0, None), stream, runs=1)
+    assert 1 <= desc.chunk_tiles <= max(-(-len(k) // 2048) for _, k, _, _ in inst)

@@ -500,7 +500,10 @@ q1_status q1_batch_describe(q1_batch* b, q1_batch_desc* d) {
     memset(d, 0, sizeof(*d));
     d->instances = b->n;
     d->items = (uint32_t)b->items.size();
-    for (const BatchItem& it : b->items) d->chunk_tiles = std::max(d->chunk_tiles, it.num_tiles);
+    // the size asked for (or tuned), else the largest piece
+    d->chunk_tiles = b->chunk;
+    if (!b->chunk)
+        for (const BatchItem& it : b->items) d->chunk_tiles = std::max(d->chunk_tiles, it.num_tiles);
     d->tile_rows = kBatchTileRows;
     d->grid = b->launch_grid;
     d->total_rows = b->total_rows;
