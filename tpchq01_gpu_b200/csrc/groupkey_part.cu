@@ -499,21 +499,6 @@ __global__ void __launch_bounds__(256) q1_gk_lists_kernel(const __grid_constant_
 // Pass 2: per-partition cells
 // ---------------------------------------------------------------------------------------------
 
-// The stage sequence of one CTA: [lo, hi) of the concatenated lists in runs of at most
-// kStageChunks chunks that never cross a partition boundary.
-struct StageWalk {
-    const uint32_t* off;            // [kParts + 1] list offsets of the partitions (shared)
-    uint32_t pos, hi, part;
-    __device__ __forceinline__ void init(const uint32_t* off_s) {
-        using namespace gp;
-        off = off_s;
-        const uint64_t T = off[kParts];
-        pos = (uint32_t)(T * blockIdx.x / gridDim.x);
-        hi = (uint32_t)(T * (blockIdx.x + 1) / gridDim.x);
-        part = 0;
-    }
-};
-
 // 16 bytes of a chunk the first pass wrote (read once).
 __device__ __forceinline__ uint4 ldg_nc_v4(const void* p) {
     uint4 v;
@@ -541,13 +526,16 @@ __global__ void __launch_bounds__(gp::kP2Threads, gp::kP2Ctas) q1_gk_partagg_ker
     cells.zero(tid, T);
     __syncthreads();
 
-    StageWalk walk;
-    walk.init(off_s);
+    // The CTA's share [pos, hi) of the concatenated lists, in stages of at most kStageChunks chunks that
+    // never cross a partition boundary.
+    const uint64_t entries = off_s[kParts];
+    uint32_t pos = (uint32_t)(entries * blockIdx.x / gridDim.x), part = 0;
+    const uint32_t hi = (uint32_t)(entries * (blockIdx.x + 1) / gridDim.x);
     auto next = [&]() -> P2Stage {
-        if (walk.pos >= walk.hi) return P2Stage{kNone, 0, 0};
-        while (walk.part + 1 < kParts && off_s[walk.part + 1] <= walk.pos) ++walk.part;
-        P2Stage st{walk.part, walk.pos, min(kStageChunks, min(walk.hi, off_s[walk.part + 1]) - walk.pos)};
-        walk.pos += st.n;
+        if (pos >= hi) return P2Stage{kNone, 0, 0};
+        while (part + 1 < kParts && off_s[part + 1] <= pos) ++part;
+        P2Stage st{part, pos, min(kStageChunks, min(hi, off_s[part + 1]) - pos)};
+        pos += st.n;
         return st;
     };
     // The thread's list entries in stage st (kNone: none), and its records of those chunks: two pairs of

@@ -7,7 +7,8 @@
 // Engines (one per placement):
 //   PlaneRegs<NG>  num_groups <= NG (4 or 8): per-thread byte-plane dot products (dp4a), four
 //                  rows per instruction, as in the scan kernel, over three price byte planes (a
-//                  row with a price >= 2^24 goes to the global path); no atomics until a flush.
+//                  row with a price >= 2^24 goes to the CTA's 128-bit sums); no atomics until a
+//                  flush.
 //   Cube3Table     num_groups <= 64: a shared-memory table per (group, discount, tax) cell; a
 //                  row adds its count, its quantity and its price: three atomics.
 //   FewTable       num_groups <= 4, in the batch kernel: eight of those tables, by lane, and a slot
@@ -18,9 +19,9 @@
 //                  discount of a cell is known there: sum (100-d) p = sum_d (100-d) P_d and
 //                  sum (100-d)(100+t) p = sum_d (100-d) (100 P_d + TP_d).
 //   SlotTable      one shared-memory slot per key below the table's size (2048 in the batch
-//                  kernel, 4096 in the group-key kernel and the partitioned path): count,
-//                  discount, quantity, price, discount x price, charge; disc_price follows at
-//                  the flush as 100 sum p - sum d p.
+//                  kernel, 4096 in the group-key kernel): count, discount, quantity, price,
+//                  discount x price, charge; disc_price follows at the flush as
+//                  100 sum p - sum d p.
 //   global         every row reduces straight into the scratch accumulators.
 // The shared tables use only 32-bit shared atomics (64-bit shared atomics are far slower).
 // Counts and quantities cannot wrap a 32-bit word between two flushes (at most 2^23 rows per
@@ -37,8 +38,8 @@
 // sums in global memory serialised on the L2 when one key holds many rows: Zipf keys over 1024
 // groups at full pass 2.98 ms per 600 M rows, 1.57 ms without those global atomics.) Rows
 // outside the tables' fast domain
-// (discount > 10, tax > 8 or price >= 2^24; TPC-H data has none) take the global path, so every
-// result is exact over the whole compressed domain.
+// (discount > 10, tax > 8 or price >= 2^24; TPC-H data has none) take the global path, the FewTable's
+// its slots, so every result is exact over the whole compressed domain.
 //
 // Scratch per group (8 x u64, zeroed before a launch): count, quantity (whole units), discount,
 // price, disc_price = a4 + 2^32 a5, charge = a6 + 2^32 a7; folded into an int128 table later.
@@ -127,21 +128,6 @@ __device__ __forceinline__ void scratch_row(unsigned long long* acc, uint32_t ke
     const uint32_t a = 100u - d;
     const uint64_t dp = (uint64_t)a * p, ch = (uint64_t)(a * (100u + t)) * p;
     scratch_add(acc, key, 1, q, d, p, dp & 0xFFFFFFFFull, dp >> 32, ch & 0xFFFFFFFFull, ch >> 32);
-}
-
-__device__ __forceinline__ bool fast_domain(uint32_t d, uint32_t t, uint32_t p) {
-    return d < kCubeDisc && t <= 8u && p < (1u << 24);
-}
-
-// 64-bit sum as (lo, hi) 32-bit shared words: lo += v, carry into hi.
-__device__ __forceinline__ void add_carry(uint32_t* lo, uint32_t* hi, uint32_t v) {
-    const uint32_t old = atomicAdd(lo, v);
-    if (old + v < old) atomicAdd(hi, 1u);
-}
-__device__ __forceinline__ void add_wide(uint32_t* lo, uint32_t* hi, uint32_t vlo, uint32_t vhi) {
-    const uint32_t old = atomicAdd(lo, vlo);
-    const uint32_t h = vhi + (old + vlo < old ? 1u : 0u);
-    if (h) atomicAdd(hi, h);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -321,14 +307,14 @@ struct CubeTable {
     // Rows r of a quad with bit r of `m` set (passing, key < num_groups, fast domain). All
     // atomics of the quad are issued before any carry is checked, so their latencies overlap.
     static constexpr bool kPacked = true, kSlots = false;
-    // The quantity, discount and tax bytes of the four rows packed in Q, D, X; acc: the scratch. A
-    // cell's count and a group's quantity cannot wrap between flushes (at most 2^23 rows per CTA:
+    // The quantity, discount and tax bytes of the four rows packed in Q, D, X. A cell's
+    // count and a group's quantity cannot wrap between flushes (at most 2^23 rows per CTA:
     // count < 2^24, quantity <= 255 * 2^23 < 2^32), so their atomics need no result. A wrap of a
     // cell's price or tax * price word (a few rows in a thousand) is worth, with the cell's
     // discount d and a = 100 - d, 2^32 of price, 2^32 a of disc_price and 2^32 100 a of charge,
     // or 2^32 a of charge.
     __device__ __forceinline__ void add_quad_packed(uint32_t m, const uint32_t key[4], uint32_t Q, uint32_t D,
-                                                    uint32_t X, const uint32_t p[4], unsigned long long* acc) {
+                                                    uint32_t X, const uint32_t p[4]) {
         uint32_t c[4], vt[4], op[4], ot[4];
         if (!__any_sync(0xffffffffu, m)) return;
 #pragma unroll
@@ -413,7 +399,7 @@ struct Cube3Table {
     // of the four rows packed in Q, D, X (D and X zero in rows outside the fast domain). There
     // 9 d + t < 99 fits a byte, so one shift-and-add gives the four (discount, tax) cell offsets.
     __device__ __forceinline__ void add_quad_packed(uint32_t m, const uint32_t key[4], uint32_t Q, uint32_t D,
-                                                    uint32_t X, const uint32_t p[4], unsigned long long*) {
+                                                    uint32_t X, const uint32_t p[4]) {
         uint32_t c[4], op[4];
         if (!__any_sync(0xffffffffu, m)) return;
         const uint32_t DT = (D << 3) + D + X;   // bytes r: 9 d + t (garbage outside the fast domain)
@@ -541,8 +527,8 @@ struct FewTable {
     }
     static constexpr bool kPacked = true, kSlots = true;
     __device__ __forceinline__ void add_quad_packed(uint32_t m, const uint32_t key[4], uint32_t Q, uint32_t D, uint32_t X,
-                                                    const uint32_t p[4], unsigned long long* acc) {
-        cells.add_quad_packed(m, key, Q, D, X, p, acc);
+                                                    const uint32_t p[4]) {
+        cells.add_quad_packed(m, key, Q, D, X, p);
     }
     // Rows r of a quad with bit r of m set, of any values, into the lane's slots.
     __device__ __forceinline__ void slot_rows(uint32_t m, const KeyQuad& x) const { few_slot_rows(slot, groups * 32, m, x); }
@@ -728,7 +714,7 @@ __device__ __forceinline__ void table_quad(Table& tab, const KeyQuad& x, uint32_
         // discount and tax bytes of in-domain rows only (d <= 10, t <= 8), so that byte-wise
         // arithmetic on them cannot carry into a neighbouring row's byte
         const uint32_t inb = ((~outside & 0x80808080u) >> 7) * 0xFFu;
-        tab.add_quad_packed(m, x.k, x.Q, x.D & inb, x.X & inb, x.p, acc);
+        tab.add_quad_packed(m, x.k, x.Q, x.D & inb, x.X & inb, x.p);
     } else {
         uint32_t q[4], d[4], t[4];
 #pragma unroll
