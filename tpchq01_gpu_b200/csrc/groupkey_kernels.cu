@@ -12,11 +12,11 @@
 // Placements:
 //   in_registers_per_thread  num_groups <= 8: per-thread dp4a byte planes (PlaneRegs<4|8>)
 //   shared_mem_per_thread    num_groups <= 64: shared (group, discount, tax) cells
-//                            (Cube3Table); <= 1024: shared (group, discount) cells (CubeTable,
-//                            3-stage ring above 768 groups); <= 4096: shared per-group slots
-//                            (SlotTable, 3-stage ring above 2048 groups), or, above 4096, this
-//                            kernel with keys < 4096 in
-//                            slots and larger keys reduced straight into the global
+//                            (Cube3Table); <= 1024: shared (group, discount) cells (CubeTable);
+//                            <= 4096: shared per-group slots (SlotTable), both in three teams over
+//                            1024-row tiles where three stages of 3072 rows do not fit beside the
+//                            table; or, above 4096, this kernel with keys < 4096 in slots and
+//                            larger keys reduced straight into the global
 //                            accumulators, or the two-pass partitioned path of
 //                            groupkey_part.cu; above 4096 groups, and above about 3100 on a large
 //                            table, the path is chosen on the device from a sample of the rows
@@ -138,8 +138,8 @@ struct GroupKeyParams {
     const uint32_t* mode;           // when set, the path chosen on the device (GroupKeyMode)
 };
 
-// P: placement; NG: plane groups of in_registers_per_thread (4 or 8); kWide: 12 consumer warps
-// over 3072-row tiles for four groups' planes; kTab: table engine of shared_mem_per_thread. (Each engine
+// P: placement; NG: plane groups of in_registers_per_thread (4 or 8); kWide: 15 consumer warps
+// over 3840-row tiles for four groups' planes; kTab: table engine of shared_mem_per_thread. (Each engine
 // its own kernel: one kernel with all of them behind a launch parameter ran 64 groups, 100 M rows, in
 // 255 us instead of 240 once the global path was a fourth alternative.)
 template <uint32_t kTab>
@@ -581,8 +581,8 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
         }
         switch (placement) {
             case kPlaceInRegistersPerThread: {
-                // The wide tiles on a table of at least 32 tiles per CTA of the grid (14.5 M rows on
-                // 148 SMs): one such scan is up to 20% faster (50 M rows 136 -> 115 us), but a queue
+                // The wide tiles on a table of at least 32 tiles per CTA of the grid (18.2 M rows on
+                // 148 SMs): one such scan is up to 20% faster (with 12 warps, 50 M rows 136 -> 115 us), but a queue
                 // of launches on tables of a few million rows ran slower with them (256 launches on
                 // 10^4..5*10^7 rows: 10.72 ms with 2048-row tiles throughout, 11.56 ms with the wide
                 // ones from 2 tiles per CTA, 10.78 ms from 32).

@@ -101,7 +101,7 @@ cudaError_t launch_groupkey(int placement, const uint8_t* const cols[6], uint64_
                             uint32_t* status, int sm_count, int max_blocks, cudaStream_t stream);
 uint64_t groupkey_scratch_bytes(uint32_t num_groups);
 // High-cardinality path of the shared_mem_per_thread placement (groupkey_part.cu): a radix
-// partition by key, then per-partition shared-memory slot tables. acc: num_groups x 8 u64
+// partition by key, then per-partition shared-memory cells. acc: num_groups x 8 u64
 // (zeroed by the caller); workspace: groupkey_part_workspace_bytes(), 256-byte aligned. When
 // `mode` is set, every kernel of the path returns at once unless *mode == kModePartitioned.
 enum GroupKeyMode : uint32_t { kModeSinglePass = 1, kModePartitioned = 2, kModeGlobalPath = 3 };
