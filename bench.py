@@ -693,7 +693,7 @@ def bench_tbl(args):
         ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         t0 = time.perf_counter()
         ev0.record(stream)
-        parse()                      # synchronous: count, scan, parse, read back the row count
+        parse()                      # synchronous: one kernel, the row count read back
         ev1.record(stream)
         ev1.synchronize()
         walls.append((time.perf_counter() - t0) * 1e3)
@@ -702,7 +702,7 @@ def bench_tbl(args):
     ms = sorted(times)[len(times) // 2]
     wall_ms = sorted(walls)[len(walls) // 2]
     peak, kind = measured_peaks()
-    moved = nbytes * 2 + rows * 38   # the text is read twice (count, parse), the columns written once
+    moved = nbytes + rows * 38   # the text is read once, the columns written once
     with tempfile.TemporaryDirectory() as td:
         path = os.path.join(td, "lineitem.tbl")
         with open(path, "wb") as f:
