@@ -37,3 +37,32 @@ def test_reference_arm_json_line():
     assert e2e["value"] == line["value"] and e2e["unit"] == line["unit"]
     assert e2e["h2d_bytes_per_step"] == 0 and e2e["d2h_bytes_per_step"] == 0
     assert line["config"]["rows_per_gpu"] == 40_000_000 and "40,000,000 rows per step" in cb["sample"]
+
+
+def bench_module():
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("bench", os.path.join(ROOT, "bench.py"))
+    m = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(m)
+    return m
+
+
+@pytest.mark.skipif(os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libq1ref.so")), reason="oracle/_ref is built")
+def test_reference_arm_says_that_it_is_unavailable():
+    out = subprocess.run([sys.executable, "bench.py", "--impl", "reference", "--rows", "1000", "--steps", "1", "--warmup",
+                          "0"], cwd=ROOT, capture_output=True, text=True, timeout=600)
+    assert out.returncode == 0, out.stderr[-2000:]
+    line = json.loads(out.stdout.strip().splitlines()[-1])
+    assert line["impl"] == "reference" and line["unavailable"]
+
+
+@pytest.mark.parametrize("rows,chunk", [(1, 16), (1000, 300), (100_003, 1 << 24)])
+def test_restatement_stands_in_for_the_reference(rows, chunk):
+    """The parity table of the own arm where the reference is not built: chunks on all threads, one exact sum."""
+    import numpy as np
+    sys.path.insert(0, ROOT)
+    from oracle import py_oracle as O
+    table, rate, threads = bench_module().restatement_table(rows, 20260101, chunk_rows=chunk)
+    want, flag = O.q1_uncompressed(O.generate(20260101, 0, rows), 729999)
+    assert flag == 0 and rate > 0 and threads >= 1
+    assert np.array_equal(table, want)
