@@ -93,7 +93,7 @@ constexpr uint32_t kSlotWords = 9;          // count, discount, quantity, price 
 // cells, then (CubeTable) kCubeGroupWords words per group: quantity and three wrap counters
 constexpr uint32_t kCubeGroupWords = 4;
 // (the groups' words by place: CubeTable::place)
-__host__ __device__ constexpr uint32_t cube_places(uint32_t num_groups) { return (num_groups + 31) & ~31u; }
+__host__ __device__ constexpr uint32_t cube_places(uint32_t num_groups) { return (num_groups + 63) & ~63u; }
 __host__ __device__ constexpr uint32_t cube_bytes(uint32_t num_groups) {
     return (num_groups * kCubeDisc * kCubeWords + cube_places(num_groups) * kCubeGroupWords) * 4;
 }
@@ -292,9 +292,12 @@ struct CubeTable {
                        // sum (100 - d) over those wraps; sum (100 - d) over wraps of tax * price
                        // words
     uint32_t cells, places;
-    // A group's place in gw: consecutive groups lie in consecutive banks, and so do groups 32 apart. (By group
-    // alone, keys that are multiples of 128, 60 M rows of 1024 groups in the batch kernel, took 368 us instead of 214.)
-    static __device__ __forceinline__ uint32_t place(uint32_t group) { return group ^ (group >> 5); }
+    // A group's place in gw, within its 64: consecutive groups lie in consecutive banks, and groups any power of two
+    // apart spread over the banks too. (By group alone, keys that are multiples of 128, 60 M rows of 1024 groups in the
+    // batch kernel, took 368 us instead of 238. group ^ (group >> 5) leaves steps of 31, 33 and 62 in one bank; turning
+    // every 32 groups by 21 banks spreads nearly any step, but its third instruction made 600 groups, 60 M rows in
+    // the group-key kernel, 150 -> 156 us.)
+    static __device__ __forceinline__ uint32_t place(uint32_t group) { return group ^ (group >> 4); }
     __device__ __forceinline__ void bind(uint8_t* base, uint32_t num_groups) {
         w = reinterpret_cast<uint32_t*>(base);
         cells = num_groups * kCubeDisc;
